@@ -191,7 +191,7 @@ def prepare(case, seed):
     if kind == "solve":
         solver = CASCISolver(norb=n, na=na, nb=nb, multiplicity=1, nroot=case["roots"], E=0.0, H=h, V=V,
                              ci_params=CIParams(ci_algorithm="hz"),
-                             davidson_liu_params=DavidsonLiuParams(e_tol=1e-12, r_tol=1e-9, maxiter=1000))
+                             davidson_liu_params=DavidsonLiuParams(e_tol=1e-10, maxiter=1000))
         # a kept solver: its space and buffers exist, the integrals of a pass are new to it
         solver.run()
         h, V = _integrals(n, seed + 1000003)
