@@ -278,7 +278,14 @@ def footprint_bytes(norb: int, na: int, nb: int, nroot: int, basis_per_root: int
     det_vectors = 8 * ndet * (6 + 2 * m)  # C/sigma staging, transposes, closure buffers
     csf = 4 * ndet + 8 * ndet  # permutation + configuration tables (upper bound)
     davidson = 8 * ndet * (3 * m + 2)  # basis, sigma, residual rows (ncsf <= ndet)
-    return int(ss + det_vectors + csf + davidson + (64 << 20))
+    # FP64 tensor-core sigma (csrc/oz.cu): integrals' digits and two work buffers of at most 2 GiB
+    oz = 0
+    if norb <= 16 and min(na, nb) >= 2 and ndet >= 20000:
+        rows = [comb(norb, k - 2) * comb(norb - k + 2, 2) for k in (na, nb)]
+        need = max(rows[0] * n0b, rows[1] * n0a,
+                   comb(norb, na - 1) * comb(norb, nb - 1) * (norb - na + 1) * (norb - nb + 1))
+        oz = 2 * min(8 * m * need, 2 << 30) + sum(r * 1024 for r in rows)
+    return int(oz + ss + det_vectors + csf + davidson + (64 << 20))
 
 
 def solve_batched(instances, precision="fp64", nstreams=16, one_launch=False, stats=None):

@@ -507,10 +507,13 @@ int f2g_sigma_set_variant(void* sb, int which, int value) {
             b->use_dense_ss = value != 0;
             if (b->use_dense_ss && b->precision == kFP32)
                 b->ensure_fp32();
+        } else if (which == 7) {
+            b->set_oz(value != 0);
         } else
             throw Error(2, "variant must be 0 (tensor cores), 1 (narrow same-spin tiles), 2 (persistent opposite "
                            "grid), 3 (tensor-core wait limit), 4 (irrep-aware opposite-spin kernel), 5 "
-                           "(TMA-fed tensor-core B tiles) or 6 (FP32 same-spin terms as dense GEMMs)");
+                           "(TMA-fed tensor-core B tiles), 6 (FP32 same-spin terms as dense GEMMs) or 7 "
+                           "(FP64 sigma by digit splitting on the tensor cores)");
     });
 }
 

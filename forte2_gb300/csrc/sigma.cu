@@ -30,6 +30,7 @@
 
 #include "sigma.cuh"
 #include "opposite_sym.cuh"
+#include "oz.cuh"
 
 namespace f2g {
 
@@ -618,7 +619,31 @@ SigmaBuilder::SigmaBuilder(CIStrings* s_, double E_, const double* H_, const dou
     // FP32 same-spin terms as dense tensor-core GEMMs by default where they were measured faster than
     // the sparse row kernel (CAS(12,12): 0.08 vs 0.13 ms per spin; CAS(14,14): 0.35 vs 1.31 ms)
     use_dense_ss = dense_ss_supported() && std::max(s->a.N0, s->b.N0) >= kDenseSsMinStrings;
+    if (!osym)
+        oz_supported(s, &oz_fast);
     set_hamiltonian(E_, H_, V_);
+}
+
+// The digit operands of the FP64 tensor-core sigma for the current integrals, in stream order
+void SigmaBuilder::build_oz(cudaStream_t st) {
+    if (oz_fast && use_oz)
+        oz_build(s, oz, dH.get(), dV.get(), E, st);
+}
+
+void SigmaBuilder::set_oz(bool on) {
+    if (on && (osym || !oz_supported(s)))
+        throw Error(2, "FP64 digit splitting: not for this space (irreps, more than 16 orbitals, or too few or too "
+                       "many holes)");
+    if (on && *graph_users > 0 && !oz)
+        throw Error(2, "sigma builder: captured graphs use its scratch; select the variant before them");
+    use_oz = on;
+    oz_fast = oz_fast || on;
+    if (on && !oz) {
+        build_oz(0);
+        if (untimed_nvec > 0)
+            oz_reserve(*oz, 1, untimed_nvec);
+        F2G_CUDA(cudaStreamSynchronize(0));
+    }
 }
 
 bool SigmaBuilder::tensor_cores_available() const { return beta_exc.get() != nullptr; }
@@ -859,6 +884,7 @@ void SigmaBuilder::set_hamiltonian(double E_, const double* H_, const double* V_
     build_string_hamiltonian(0, ha, true, 0);
     build_string_hamiltonian(1, hb, false, 0);
     build_local_ss(0);
+    build_oz(0);
     F2G_CUDA(cudaStreamSynchronize(0)); // set-up ran on the legacy stream: wait for it alone
     fp32_ready = false;
     dss_ready = false;
@@ -892,6 +918,7 @@ void SigmaBuilder::set_hamiltonian_async(double E_, const double* H_, const doub
     build_string_hamiltonian(0, ha, true, st);
     build_string_hamiltonian(1, hb, false, st);
     build_local_ss(st);
+    build_oz(st);
     for (StringHamiltonian* sh : {&ha, &hb}) {
         const int s_ = sh == &ha ? 0 : 1;
         const size_t total = (size_t)s->spin(s_).N0 * sh->nnz;
@@ -920,6 +947,8 @@ void SigmaBuilder::prepare_untimed(int nvec) {
     const size_t tot = (size_t)nvec * std::max<int64_t>(1, s->nfull);
     gCt.reserve(tot);
     gTt.reserve(tot);
+    if (oz)
+        oz_reserve(*oz, 1, nvec);
     gfC.reserve(tot);
     gfS.reserve(tot);
     gfCt.reserve(tot);
@@ -1165,6 +1194,25 @@ void SigmaBuilder::run(const T* C, T* sig, cudaStream_t st, int mask, bool timed
     }
     if (timed)
         F2G_CUDA(cudaEventRecord(cur_ev[0], st));
+    if constexpr (sizeof(T) == 8) {
+        if (oz_path() && mask == 7) {
+            const int set = graph ? 1 : 0;
+            if (!graph)
+                oz_reserve(*oz, 0, nvec);
+            oz_diag(*oz, C, sig, nvec, st);
+            launch_transpose<T>(NA, NB, C, Ct_, st, nvec);
+            oz_same_spin(*oz, set, 1, Ct_, sig, nvec, max_ctas, tc_err.get(), st);
+            if (timed)
+                F2G_CUDA(cudaEventRecord(cur_ev[1], st));
+            oz_same_spin(*oz, set, 0, C, sig, nvec, max_ctas, tc_err.get(), st);
+            if (timed)
+                F2G_CUDA(cudaEventRecord(cur_ev[2], st));
+            oz_opposite(*oz, set, C, sig, nvec, max_ctas, tc_err.get(), st);
+            if (timed)
+                F2G_CUDA(cudaEventRecord(cur_ev[3], st));
+            return;
+        }
+    }
     bool dense = false;
     if constexpr (sizeof(T) == 4) {
         if (use_dense_ss && dss_ready && (mask & 3)) {

@@ -83,6 +83,14 @@ struct SigmaBuilder {
     bool dense_ss_supported() const;
     void prepare_dense_ss(cudaStream_t st);
     void prepare_graph_fp32(int nvec);
+    // FP64 sigma of a C1 space (or of a GAS space's embedding) on the tensor cores by exact digit
+    // splitting (oz.cu), where the sizes allow it and the space is large enough to gain
+    bool use_oz = true;
+    bool oz_fast = false;
+    std::shared_ptr<struct OzSigma> oz;
+    bool oz_path() const { return oz && use_oz; }
+    void build_oz(cudaStream_t st);
+    void set_oz(bool on); // on: also for spaces too small to gain (an error where the sizes rule it out)
     DevBuf<uint32_t> beta_exc; // beta single excitations per string for its scatter
     DevBuf<int> tc_err;        // set by the tensor-core kernel if a bounded wait gave up
     DevBuf<unsigned int> tc_cmax; // per-vector largest |C| of a tensor-core launch (its operand scale)

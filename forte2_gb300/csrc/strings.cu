@@ -152,6 +152,20 @@ void SpinStrings::build_up2(const uint64_t* d_binom, cudaStream_t st) {
     F2G_LAUNCH("k_up2");
 }
 
+void strings_up2(const SpinStrings& ss, const uint64_t* d_binom, uint64_t* out, cudaStream_t st) {
+    if (!ss.N2)
+        return;
+    k_up2<<<ceil_div(ss.N2, 256), 256, 0, st>>>(ss.n, ss.k, ss.N2, ss.m2, d_binom, out);
+    F2G_LAUNCH("k_up2");
+}
+
+void strings_masks(int n, int k, int64_t N, const uint64_t* d_binom, uint64_t* out, cudaStream_t st) {
+    if (!N)
+        return;
+    k_unrank<<<ceil_div(N, 256), 256, 0, st>>>(n, k, N, d_binom, out);
+    F2G_LAUNCH("k_unrank");
+}
+
 CIStrings::CIStrings(int na_, int nb_, int norb_) : norb(norb_), na(na_), nb(nb_) {
     build_c1();
     blocks.set_c1(na, nb, a.N0, b.N0);

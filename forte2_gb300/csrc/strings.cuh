@@ -25,6 +25,10 @@ struct SpinStrings {
     void build_up3(const uint64_t* d_binom, cudaStream_t st);
 };
 
+// 2-hole lists in SpinStrings::up2's layout into caller's memory; masks of the N = C(n, k) strings
+void strings_up2(const SpinStrings& ss, const uint64_t* d_binom, uint64_t* out, cudaStream_t st);
+void strings_masks(int n, int k, int64_t N, const uint64_t* d_binom, uint64_t* out, cudaStream_t st);
+
 // The strings of an active space. The coupling lists and the sigma kernels always cover the C1
 // CAS space of all orbitals (a, b: every string of na / nb electrons, nfull determinants). A
 // space with point-group irreps or GAS restrictions is a set of determinant blocks of it
