@@ -280,7 +280,7 @@ def footprint_bytes(norb: int, na: int, nb: int, nroot: int, basis_per_root: int
     davidson = 8 * ndet * (3 * m + 2)  # basis, sigma, residual rows (ncsf <= ndet)
     # FP64 tensor-core sigma (csrc/oz.cu): integrals' digits and two work buffers of at most 2 GiB
     oz = 0
-    if norb <= 16 and min(na, nb) >= 2 and ndet >= 20000:
+    if norb <= 16 and min(na, nb) >= 2 and ndet > 8192:
         rows = [comb(norb, k - 2) * comb(norb - k + 2, 2) for k in (na, nb)]
         need = max(rows[0] * n0b, rows[1] * n0a,
                    comb(norb, na - 1) * comb(norb, nb - 1) * (norb - na + 1) * (norb - nb + 1))

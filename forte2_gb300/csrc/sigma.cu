@@ -54,89 +54,78 @@ __device__ inline int s2neg(uint64_t X, int hi, int lo) {
     return parity_below(X, lo) ^ parity_below(X & ~(uint64_t(1) << lo), hi);
 }
 
-// parts: bit 0 one-electron, bit 1 same-spin two-electron; e0 is added to the diagonal.
+// parts: bit 0 one-electron, bit 1 same-spin two-electron; e0 is added to the diagonal. One block per
+// string, a thread per entry: entry 0 the diagonal, then the singles (p, q), then the doubles (p > r,
+// q > s), all indices ascending, the last fastest. (A thread per string took 285 us for the 70 strings of
+// (8e,8o), a chain of 53 entries each, whatever the number of strings.)
+constexpr int kBuildSsThreads = 128;
 template <typename T>
-__global__ void k_build_ss(int n, int k, int64_t N0, int nnz, const uint64_t* str, const uint64_t* binom,
-                           const double* h, const double* V, double e0, int parts, int32_t* col,
-                           T* val) {
-    const int64_t J = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (J >= N0)
-        return;
-    const uint64_t mJ = str[J];
+__global__ void __launch_bounds__(kBuildSsThreads)
+    k_build_ss(int n, int k, int64_t N0, int nnz, const uint64_t* str, const uint64_t* binom, const double* h,
+               const double* V, double e0, int parts, int32_t* col, T* val) {
+    __shared__ int8_t occ[kMaxOrb], vir[kMaxOrb];
     const bool one = parts & 1, two = parts & 2;
-    int32_t* c = col + J * (int64_t)nnz;
-    T* v = val + J * (int64_t)nnz;
-    int e = 0;
-    // diagonal
-    double d = e0;
-    for (int t = 0; t < n; ++t) {
-        if (!(mJ >> t & 1))
-            continue;
-        if (one)
-            d += h[t * n + t];
-        if (two)
-            for (int u = 0; u < t; ++u)
-                if (mJ >> u & 1)
-                    d += vanti(V, n, t, u, t, u);
-    }
-    c[e] = (int32_t)J;
-    v[e] = (T)d;
-    ++e;
-    // single replacements Ja <- Ia: p in J, q not in J
-    for (int p = 0; p < n; ++p) {
-        if (!(mJ >> p & 1))
-            continue;
-        for (int q = 0; q < n; ++q) {
-            if (mJ >> q & 1)
-                continue;
-            const uint64_t mI = (mJ & ~(uint64_t(1) << p)) | (uint64_t(1) << q);
-            double x = 0.0;
-            if (one) {
-                const int neg = parity_below(mJ, p) ^ parity_below(mI, q);
-                x = neg ? -h[p * n + q] : h[p * n + q];
-            }
-            if (two) {
-                for (int t = 0; t < n; ++t) {
-                    if (t == p || !(mJ >> t & 1))
-                        continue;
-                    const int ph = p > t ? p : t, pl = p > t ? t : p;
-                    const int qh = q > t ? q : t, ql = q > t ? t : q;
-                    const int neg = s2neg(mJ, ph, pl) ^ s2neg(mI, qh, ql);
-                    const double a = vanti(V, n, ph, pl, qh, ql);
-                    x += neg ? -a : a;
-                }
-            }
-            c[e] = (int32_t)string_rank(mI, n, k, binom);
-            v[e] = (T)x;
-            ++e;
+    const int nv = n - k, nq = nv * (nv - 1) / 2;
+    // i-th pair a > b in the order (1,0), (2,0), (2,1), ...
+    auto pair = [](int i, int& a, int& b) {
+        a = 1;
+        while (a * (a + 1) / 2 <= i)
+            ++a;
+        b = i - a * (a - 1) / 2;
+    };
+    for (int64_t J = blockIdx.x; J < N0; J += gridDim.x) {
+        const uint64_t mJ = str[J];
+        __syncthreads();
+        for (int p = threadIdx.x; p < n; p += blockDim.x) {
+            const int below = popc64(mJ & ((uint64_t(1) << p) - 1));
+            if (mJ >> p & 1)
+                occ[below] = (int8_t)p;
+            else
+                vir[p - below] = (int8_t)p;
         }
-    }
-    // double replacements: p > r in J, q > s not in J
-    for (int p = 0; p < n; ++p) {
-        if (!(mJ >> p & 1))
-            continue;
-        for (int r = 0; r < p; ++r) {
-            if (!(mJ >> r & 1))
-                continue;
-            for (int q = 0; q < n; ++q) {
-                if (mJ >> q & 1)
-                    continue;
-                for (int s = 0; s < q; ++s) {
-                    if (mJ >> s & 1)
-                        continue;
-                    const uint64_t mI =
-                        (mJ & ~((uint64_t(1) << p) | (uint64_t(1) << r))) | (uint64_t(1) << q) | (uint64_t(1) << s);
-                    double x = 0.0;
-                    if (two) {
-                        const int neg = s2neg(mJ, p, r) ^ s2neg(mI, q, s);
-                        const double a = vanti(V, n, p, r, q, s);
-                        x = neg ? -a : a;
+        __syncthreads();
+        for (int e = threadIdx.x; e < nnz; e += blockDim.x) {
+            double x = 0.0;
+            uint64_t mI = mJ;
+            if (e == 0) {
+                x = e0;
+                for (int i = 0; i < k; ++i) {
+                    const int t = occ[i];
+                    if (one)
+                        x += h[t * n + t];
+                    if (two)
+                        for (int l = 0; l < i; ++l)
+                            x += vanti(V, n, t, occ[l], t, occ[l]);
+                }
+            } else if (e <= k * nv) {
+                const int p = occ[(e - 1) / nv], q = vir[(e - 1) % nv];
+                mI = (mJ & ~(uint64_t(1) << p)) | (uint64_t(1) << q);
+                if (one)
+                    x = (parity_below(mJ, p) ^ parity_below(mI, q)) ? -h[p * n + q] : h[p * n + q];
+                if (two) {
+                    for (int l = 0; l < k; ++l) {
+                        const int t = occ[l];
+                        if (t == p)
+                            continue;
+                        const int ph = p > t ? p : t, pl = p > t ? t : p;
+                        const int qh = q > t ? q : t, ql = q > t ? t : q;
+                        const double a = vanti(V, n, ph, pl, qh, ql);
+                        x += (s2neg(mJ, ph, pl) ^ s2neg(mI, qh, ql)) ? -a : a;
                     }
-                    c[e] = (int32_t)string_rank(mI, n, k, binom);
-                    v[e] = (T)x;
-                    ++e;
+                }
+            } else {
+                int pi, ri, qi, si;
+                pair((e - 1 - k * nv) / nq, pi, ri);
+                pair((e - 1 - k * nv) % nq, qi, si);
+                const int p = occ[pi], r = occ[ri], q = vir[qi], s = vir[si];
+                mI = (mJ & ~((uint64_t(1) << p) | (uint64_t(1) << r))) | (uint64_t(1) << q) | (uint64_t(1) << s);
+                if (two) {
+                    const double a = vanti(V, n, p, r, q, s);
+                    x = (s2neg(mJ, p, r) ^ s2neg(mI, q, s)) ? -a : a;
                 }
             }
+            col[J * nnz + e] = e == 0 ? (int32_t)J : (int32_t)string_rank(mI, n, k, binom);
+            val[J * nnz + e] = (T)x;
         }
     }
 }
@@ -593,6 +582,11 @@ void launch_opposite_tc(const CIStrings* s, const uint32_t* exc, const float* V,
                         cudaStream_t st, int nvec, const TcBOperands* tb);
 void opposite_tc_build_b(const CIStrings* s, const float* V, const unsigned int* vmax,
                          std::shared_ptr<TcBOperands>& tb, cudaStream_t st);
+bool small_supported(const CIStrings* s);
+void small_lists(const CIStrings* s, DevBuf<uint32_t> (&exc)[2], cudaStream_t st);
+void launch_small_sigma(const CIStrings* s, const StringHamiltonian& ha, const StringHamiltonian& hb,
+                        const DevBuf<uint32_t> (&exc)[2], const double* V, const double* C, double* sig, int nvec,
+                        cudaStream_t st);
 void dense_ss_build(const CIStrings* s, const StringHamiltonian* sh[2], std::shared_ptr<DenseSameSpin>& d,
                     cudaStream_t st);
 void dense_ss_split(const CIStrings* s, DenseSameSpin& d, const float* C, int nvec, int set, cudaStream_t st);
@@ -621,6 +615,10 @@ SigmaBuilder::SigmaBuilder(CIStrings* s_, double E_, const double* H_, const dou
     use_dense_ss = dense_ss_supported() && std::max(s->a.N0, s->b.N0) >= kDenseSsMinStrings;
     if (!osym)
         oz_supported(s, &oz_fast);
+    if (!oz_fast && !s->blocked() && small_supported(s)) {
+        use_small = true;
+        small_lists(s, small_exc, 0); // ordered before set_hamiltonian's wait on the legacy stream
+    }
     set_hamiltonian(E_, H_, V_);
 }
 
@@ -705,7 +703,7 @@ void SigmaBuilder::build_string_hamiltonian(int spin, StringHamiltonian& sh, boo
     if (!s->blocked()) {
         sh.col.reserve(total);
         sh.val.reserve(total);
-        k_build_ss<double><<<ceil_div(ss.N0, 128), 128, 0, st>>>(n, ss.k, ss.N0, nnz_full, ss.str.get(),
+        k_build_ss<double><<<(unsigned)std::min<int64_t>(ss.N0, 1 << 20), kBuildSsThreads, 0, st>>>(n, ss.k, ss.N0, nnz_full, ss.str.get(),
                                                                 s->binom.get(), dH.get(), dV.get(), with_e0 ? E : 0.0,
                                                                 3, sh.col.get(), sh.val.get());
         F2G_LAUNCH("k_build_ss");
@@ -715,7 +713,7 @@ void SigmaBuilder::build_string_hamiltonian(int spin, StringHamiltonian& sh, boo
     // (a symmetric space keeps about 1/nirrep of them); the layout depends on the strings alone
     TmpBuf<int32_t> fc(total, st);
     TmpBuf<double> fv(total, st);
-    k_build_ss<double><<<ceil_div(ss.N0, 128), 128, 0, st>>>(n, ss.k, ss.N0, nnz_full, ss.str.get(), s->binom.get(),
+    k_build_ss<double><<<(unsigned)std::min<int64_t>(ss.N0, 1 << 20), kBuildSsThreads, 0, st>>>(n, ss.k, ss.N0, nnz_full, ss.str.get(), s->binom.get(),
                                                             dH.get(), dV.get(), with_e0 ? E : 0.0, 3, fc.get(),
                                                             fv.get());
     F2G_LAUNCH("k_build_ss");
@@ -767,7 +765,7 @@ void build_ss_values(int n, int k, int64_t N0, int nnz, const uint64_t* str, con
                      const double* V, double e0, int32_t* col, double* val, cudaStream_t st) {
     if (N0 == 0 || nnz == 0)
         return;
-    k_build_ss<double><<<ceil_div(N0, 128), 128, 0, st>>>(n, k, N0, nnz, str, binom, h, V, e0, 3, col, val);
+    k_build_ss<double><<<(unsigned)std::min<int64_t>(N0, 1 << 20), kBuildSsThreads, 0, st>>>(n, k, N0, nnz, str, binom, h, V, e0, 3, col, val);
     F2G_LAUNCH("k_build_ss");
 }
 
@@ -1195,6 +1193,17 @@ void SigmaBuilder::run(const T* C, T* sig, cudaStream_t st, int mask, bool timed
     if (timed)
         F2G_CUDA(cudaEventRecord(cur_ev[0], st));
     if constexpr (sizeof(T) == 8) {
+        if (use_small && !oz_path() && mask == 7) {
+            // one launch; its time counts as the opposite-spin term's
+            if (timed) {
+                F2G_CUDA(cudaEventRecord(cur_ev[1], st));
+                F2G_CUDA(cudaEventRecord(cur_ev[2], st));
+            }
+            launch_small_sigma(s, ha, hb, small_exc, Vt, C, sig, nvec, st);
+            if (timed)
+                F2G_CUDA(cudaEventRecord(cur_ev[3], st));
+            return;
+        }
         if (oz_path() && mask == 7) {
             const int set = graph ? 1 : 0;
             if (!graph)
@@ -1505,7 +1514,7 @@ void SigmaBuilder::term_c1(int which, const double* C, double* sigma, cudaStream
     const size_t total = (size_t)ss.N0 * tmp.nnz;
     tmp.col.reserve(total);
     tmp.val.reserve(total);
-    k_build_ss<double><<<ceil_div(ss.N0, 128), 128, 0, st>>>(n, ss.k, ss.N0, tmp.nnz, ss.str.get(), s->binom.get(),
+    k_build_ss<double><<<(unsigned)std::min<int64_t>(ss.N0, 1 << 20), kBuildSsThreads, 0, st>>>(n, ss.k, ss.N0, tmp.nnz, ss.str.get(), s->binom.get(),
                                                             dH.get(), dV.get(), 0.0, parts, tmp.col.get(),
                                                             tmp.val.get());
     F2G_LAUNCH("k_build_ss term");

@@ -91,6 +91,9 @@ struct SigmaBuilder {
     bool oz_path() const { return oz && use_oz; }
     void build_oz(cudaStream_t st);
     void set_oz(bool on); // on: also for spaces too small to gain (an error where the sizes rule it out)
+    // FP64 sigma of a small C1 space in one launch (small.cu)
+    bool use_small = false;
+    DevBuf<uint32_t> small_exc[2];
     DevBuf<uint32_t> beta_exc; // beta single excitations per string for its scatter
     DevBuf<int> tc_err;        // set by the tensor-core kernel if a bounded wait gave up
     DevBuf<unsigned int> tc_cmax; // per-vector largest |C| of a tensor-core launch (its operand scale)

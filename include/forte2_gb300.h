@@ -113,7 +113,7 @@ int f2g_sigma_set_tensor_cores(void* sigma, int on, int* available);
  * tensor-core GEMMs (split FP16, three products; spaces of at most 4096 strings per spin, else
  * error 2; default 1 from 512 strings per spin). which = 7: FP64 sigma on the tensor cores by exact
  * digit splitting (the FP64 kernels' accuracy; up to 16 orbitals, two electrons or more of each
- * spin and at most 146 pairs of holes per string pair, no irreps, else error 2; default 1 from 20,000
+ * spin and at most 146 pairs of holes per string pair, no irreps, else error 2; default 1 from 8,193
  * determinants). No reference counterpart. */
 int f2g_sigma_set_variant(void* sigma, int which, int value);
 /* 1 if a tensor-core build (FP32, or FP64 by digit splitting) gave up waiting for its matrix operations
