@@ -104,12 +104,12 @@ void dg_gs_multi(DGState* st, const DGParams& P, double* b, int64_t ld, const do
                  double* partial, cudaStream_t s);
 void dg_correct(const DGState* st, const double* X, const double* D, int64_t ldx, const double* Mxd, const double* A,
                 const double* Bd, int k, int R, int64_t n, double* S, cudaStream_t s);
-// One-block iteration after the sigma build, for vectors up to kDGSmallN and bases up to 32.
+// The iteration after the sigma build in one cluster, for vectors up to kDGSmallN and bases up to 32.
 constexpr int64_t kDGSmallN = 4096;
 bool dg_small_ok(const DGParams& P);
 void dg_small_iter(DGState* st, const DGParams& P, const double* stage_s, int R, double* b, double* sigma, int64_t ld,
-                   double* r, int64_t ldr, const double* hdiag, double* G, double* evals, double* V, double* Dp,
-                   double* tmp, int64_t ldt, double* hist, double* norms2, cudaStream_t s);
+                   double* r, int64_t ldr, const double* hdiag, double* G, double* evals, double* V, double* tmp,
+                   int64_t ldt, double* hist, cudaStream_t s);
 void dg_ritz(const DGState* st, const DGParams& P, const double* b, int64_t ld, const double* V, int ldv, double* out,
              int64_t ldo, cudaStream_t s);
 

@@ -187,8 +187,8 @@ struct DavGraph {
             dg_correct(S, X, D, ldx, Mxd, cA.get(), cB.get(), kc, R, n, stage_s.get(), s);
         }
         if (dg_small_ok(P)) {
-            dg_small_iter(S, P, stage_s.get(), R, b, sigma, ld, r, ldr, hdiag, G.get(), evals.get(), V.get(), Dp.get(),
-                          tmp, ldt, hist.get(), norms2.get(), s);
+            dg_small_iter(S, P, stage_s.get(), R, b, sigma, ld, r, ldr, hdiag, G.get(), evals.get(), V.get(), tmp,
+                          ldt, hist.get(), s);
             return;
         }
         dg_unstage(S, stage_s.get(), R, n, sigma, ld, s);
