@@ -301,60 +301,178 @@ __global__ void k_csf_to_det(int64_t nslot, CsfView v, const T* __restrict__ csf
     det[e & 0x7fffffffu] = (e >> 31) ? -acc : acc;
 }
 
-template <bool SQUARE, typename T = double>
-__global__ void k_det_to_csf(int64_t ncsf, CsfView v, const T* __restrict__ det, T* __restrict__ csf,
-                             int64_t ndet_stride, int64_t ncsf_stride) {
+// sum_j c_j^2 E(det_j) of every CSF (the CSF diagonal), one thread per CSF
+__global__ void k_csf_square(int64_t ncsf, CsfView v, const double* __restrict__ det, double* __restrict__ csf) {
     const int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (u >= ncsf)
         return;
-    det += blockIdx.y * ndet_stride;
-    csf += blockIdx.y * ncsf_stride;
     const int64_t c = find_in(v.conf_csf, v.csf_brk[blockIdx.x], v.csf_brk[blockIdx.x + 1], u);
     const int N = popc64(v.conf_s[c]);
     const int nd = v.ndetN[N], nc = v.ncsfN[N];
-    const int64_t i = u - v.conf_csf[c];
-    // transposed table: the threads of a configuration (consecutive i) read consecutive entries
-    const T* O = overlaps_t<T>(v) + v.offN[N] + i;
+    // transposed table: the threads of a configuration (consecutive CSFs) read consecutive entries
+    const double* O = v.OT + v.offN[N] + (u - v.conf_csf[c]);
     const uint32_t* pm = v.perm + v.conf_slot[c];
-    // eight determinants per step: their table entries and addresses, then their values, are
-    // requested together (the value loads depend on the addresses); zero entries skip the load.
-    // The sum runs over j in order, as one determinant per step would.
-    constexpr int U = 8;
-    T acc = 0;
-    int j = 0;
-    for (; j + U <= nd; j += U) {
-        T o[U], x[U];
-        uint32_t e[U];
-#pragma unroll
-        for (int k = 0; k < U; ++k) {
-            o[k] = O[(int64_t)(j + k) * nc];
-            e[k] = pm[j + k];
-        }
-#pragma unroll
-        for (int k = 0; k < U; ++k)
-            x[k] = o[k] != T(0) ? det[e[k] & 0x7fffffffu] : T(0);
-#pragma unroll
-        for (int k = 0; k < U; ++k) {
-            if (o[k] == T(0))
-                continue;
-            if (SQUARE)
-                acc += o[k] * o[k] * x[k];
-            else
-                acc += ((e[k] >> 31) ? -o[k] : o[k]) * x[k];
-        }
-    }
-    for (; j < nd; ++j) {
-        const T o = O[(int64_t)j * nc];
-        if (o == T(0))
-            continue;
-        const uint32_t e = pm[j];
-        const T x = det[e & 0x7fffffffu];
-        if (SQUARE)
-            acc += o * o * x;
-        else
-            acc += ((e >> 31) ? -o : o) * x;
+    double acc = 0;
+#pragma unroll 4
+    for (int j = 0; j < nd; ++j) {
+        const double o = O[(int64_t)j * nc];
+        if (o != 0.0)
+            acc += o * o * det[pm[j] & 0x7fffffffu];
     }
     csf[u] = acc;
+}
+
+// det -> CSF as small matrix products: the configurations of one open-shell count N share one overlap table, so
+// a block takes 32 of them (a lane each) and up to 64 CSFs (R per warp) and gathers their determinants once,
+// 32 per step, into shared memory, the table's piece beside them. A thread per CSF gathered every
+// determinant again and read the table through L1 for every product: 2.13 ms at CAS(14,14), 8 times its
+// FP64 multiply-adds' time. The sum of a CSF runs over its determinants in order, as before (same bits).
+constexpr int kTileConf = 32, kTileK = 32, kTileWarps = 8;
+struct CsfTiles {
+    int n = 0;                  // groups
+    int N[kMaxOrb + 1], R[kMaxOrb + 1], ntile[kMaxOrb + 1];
+    int64_t block0[kMaxOrb + 2]; // first block of every group
+    int64_t conf0[kMaxOrb + 1], nconf[kMaxOrb + 1];
+};
+
+template <typename T, int R>
+__device__ void det_to_csf_tile(const CsfView& v, const uint32_t* __restrict__ conf, int nconf, int N, int i0,
+                                const T* __restrict__ det, T* __restrict__ csf, T* sx, T* so) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nd = v.ndetN[N], nc = v.ncsfN[N];
+    constexpr int W = R * kTileWarps; // CSFs of the tile
+    const T* O = overlaps_t<T>(v) + v.offN[N] + i0;
+    const int wi = min(W, nc - i0);
+    const uint32_t* pm[kTileConf / kTileWarps]; // determinants of this warp's configurations
+#pragma unroll
+    for (int q = 0; q < kTileConf / kTileWarps; ++q) {
+        const int c = warp + kTileWarps * q;
+        pm[q] = c < nconf ? v.perm + v.conf_slot[conf[c]] : nullptr;
+    }
+    T acc[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        acc[r] = T(0);
+    for (int j0 = 0; j0 < nd; j0 += kTileK) {
+        const int w = min(kTileK, nd - j0);
+        T x[kTileConf / kTileWarps];
+#pragma unroll
+        for (int q = 0; q < kTileConf / kTileWarps; ++q) {
+            x[q] = T(0);
+            if (pm[q] && lane < w) {
+                const uint32_t e = __ldg(pm[q] + j0 + lane);
+                const T d = __ldg(det + (e & 0x7fffffffu));
+                x[q] = (e >> 31) ? -d : d;
+            }
+        }
+        __syncthreads(); // the previous step is consumed
+#pragma unroll
+        for (int q = 0; q < kTileConf / kTileWarps; ++q)
+            sx[lane * (kTileConf + 1) + warp + kTileWarps * q] = x[q];
+        for (int t = threadIdx.x; t < kTileK * W; t += 256) {
+            const int j = t / W, i = t % W;
+            so[t] = (j < w && i < wi) ? __ldg(O + (int64_t)(j0 + j) * nc + i) : T(0);
+        }
+        __syncthreads();
+        if (warp * R < wi) {
+#pragma unroll 4
+            for (int j = 0; j < w; ++j) {
+                const T y = sx[j * (kTileConf + 1) + lane];
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    acc[r] += so[j * W + warp * R + r] * y;
+            }
+        }
+    }
+    if (lane < nconf) {
+        T* out = csf + v.conf_csf[conf[lane]] + i0 + warp * R;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (warp * R + r < wi)
+                out[r] = acc[r];
+    }
+}
+
+// FP64, few configurations with a large table (one of 429 CSFs and 3,432 determinants at CAS(14,14)): a block
+// per configuration and 32 CSFs, a lane each, every warp an eighth of the determinants, the warps' sums added
+// in order. In the tiles above their chain of FP64 multiply-adds ran on a few SMs for 1.8 ms.
+__global__ void __launch_bounds__(256) k_det_to_csf_thin(const __grid_constant__ CsfTiles t, CsfView v,
+                                                         const uint32_t* __restrict__ conf_byN,
+                                                         const double* __restrict__ det, double* __restrict__ csf,
+                                                         int64_t ndet_stride, int64_t ncsf_stride) {
+    __shared__ double red[kTileWarps][32];
+    det += blockIdx.y * ndet_stride;
+    csf += blockIdx.y * ncsf_stride;
+    int g = 0;
+    while (g + 1 < t.n && (int64_t)blockIdx.x >= t.block0[g + 1])
+        ++g;
+    const int64_t b = blockIdx.x - t.block0[g], cb = b / t.ntile[g];
+    const uint32_t c = conf_byN[t.conf0[g] + cb];
+    const int N = t.N[g], warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nd = v.ndetN[N], nc = v.ncsfN[N], i = (int)(b - cb * t.ntile[g]) * 32 + lane;
+    const double* O = v.OT + v.offN[N] + min(i, nc - 1);
+    const uint32_t* pm = v.perm + v.conf_slot[c];
+    double acc[2] = {0.0, 0.0};
+#pragma unroll 4
+    for (int j = warp; j < nd; j += 2 * kTileWarps)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int k = j + h * kTileWarps;
+            if (k < nd) {
+                const uint32_t e = __ldg(pm + k);
+                const double d = __ldg(det + (e & 0x7fffffffu));
+                acc[h] += __ldg(O + (int64_t)k * nc) * ((e >> 31) ? -d : d);
+            }
+        }
+    red[warp][lane] = acc[0] + acc[1];
+    __syncthreads();
+    if (warp == 0 && i < nc) {
+        double s = 0.0;
+        for (int w = 0; w < kTileWarps; ++w)
+            s += red[w][lane];
+        csf[v.conf_csf[c] + i] = s;
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_det_to_csf(const __grid_constant__ CsfTiles t, CsfView v,
+                                                    const uint32_t* __restrict__ conf_byN, const T* __restrict__ det,
+                                                    T* __restrict__ csf, int64_t ndet_stride, int64_t ncsf_stride) {
+    __shared__ T sx[kTileK * (kTileConf + 1)], so[kTileK * 8 * kTileWarps];
+    det += blockIdx.y * ndet_stride;
+    csf += blockIdx.y * ncsf_stride;
+    int g = 0;
+    while (g + 1 < t.n && (int64_t)blockIdx.x >= t.block0[g + 1])
+        ++g;
+    const int64_t b = blockIdx.x - t.block0[g], cb = b / t.ntile[g];
+    const int i0 = (int)(b - cb * t.ntile[g]) * t.R[g] * kTileWarps;
+    const uint32_t* conf = conf_byN + t.conf0[g] + cb * kTileConf;
+    const int nconf = (int)min((int64_t)kTileConf, t.nconf[g] - cb * kTileConf);
+    switch (t.R[g]) {
+    case 1:
+        det_to_csf_tile<T, 1>(v, conf, nconf, t.N[g], i0, det, csf, sx, so);
+        break;
+    case 2:
+        det_to_csf_tile<T, 2>(v, conf, nconf, t.N[g], i0, det, csf, sx, so);
+        break;
+    case 4:
+        det_to_csf_tile<T, 4>(v, conf, nconf, t.N[g], i0, det, csf, sx, so);
+        break;
+    case 6:
+        det_to_csf_tile<T, 6>(v, conf, nconf, t.N[g], i0, det, csf, sx, so);
+        break;
+    default:
+        det_to_csf_tile<T, 8>(v, conf, nconf, t.N[g], i0, det, csf, sx, so);
+    }
+}
+
+__global__ void k_conf_key(int64_t nconf, const uint64_t* __restrict__ conf_s, uint8_t* __restrict__ key,
+                           uint32_t* __restrict__ id) {
+    const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (c >= nconf)
+        return;
+    key[c] = (uint8_t)popc64(conf_s[c]);
+    id[c] = (uint32_t)c;
 }
 
 // ---- Slater rules between two determinants (slater_rules.cc:86-201) ---------------------------
@@ -638,7 +756,71 @@ SpinAdapter::SpinAdapter(const CIStrings* s_, int twoS_, int twoMs_)
     ncoupling = 0;
     for (int N = 0; N <= n; ++N)
         ncoupling += (int64_t)h[N] * nnzN[N];
+    // configurations grouped by open-shell count (a stable sort keeps their order)
+    confN.assign(n + 2, 0);
+    for (int N = 0; N <= n; ++N)
+        confN[N + 1] = confN[N] + (int64_t)h[N];
+    conf_byN.reserve(std::max<int64_t>(1, nconf));
+    if (nconf > 0) {
+        TmpBuf<uint8_t> key(nconf, st), key2(nconf, st);
+        TmpBuf<uint32_t> id(nconf, st);
+        k_conf_key<<<ceil_div(nconf, T), T, 0, st>>>(nconf, conf_s.get(), key.get(), id.get());
+        F2G_LAUNCH("k_conf_key");
+        size_t bytes = 0;
+        F2G_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, bytes, key.get(), key2.get(), id.get(), conf_byN.get(), nconf, 0,
+                                                 6, st));
+        TmpBuf<unsigned char> tmp(bytes, st);
+        F2G_CUDA(cub::DeviceRadixSort::SortPairs(tmp.get(), bytes, key.get(), key2.get(), id.get(), conf_byN.get(), nconf,
+                                                 0, 6, st));
+    }
     F2G_CUDA(cudaStreamSynchronize(st));
+}
+
+// Blocks of the det -> CSF products, the largest tables first (their blocks run longest); CSF tiles of 8, 16,
+// 32, 48 or 64, the smallest that gives the fewest tiles. The groups of k_det_to_csf_thin (FP64, a chain of
+// more than 64 determinants and fewer tiles than two per SM) go to `thin`: at CAS(14,14) 2.13 -> 0.76 ms.
+// FP32 sums keep the order of the determinants, and their chain costs little: no thin groups.
+static void tiles_of(const SpinAdapter& a, CsfTiles& t, CsfTiles* thin) {
+    t.block0[0] = 0;
+    if (thin)
+        thin->block0[0] = 0;
+    for (int N = a.norb; N >= 0; --N) {
+        const int64_t nc = a.confN[N + 1] - a.confN[N];
+        if (nc == 0 || a.ncsfN[N] == 0)
+            continue;
+        const int tiles = ceil_div(a.ncsfN[N], 8 * kTileWarps);
+        int R = 8;
+        for (int r : {6, 4, 2, 1})
+            if (r * kTileWarps * tiles >= a.ncsfN[N])
+                R = r;
+        const int64_t rows = (nc + kTileConf - 1) / kTileConf;
+        const bool is_thin = thin && a.ndetN[N] > 64 && rows * tiles < 304;
+        CsfTiles& o = is_thin ? *thin : t;
+        o.N[o.n] = N;
+        o.R[o.n] = R;
+        o.ntile[o.n] = is_thin ? ceil_div(a.ncsfN[N], 32) : tiles;
+        o.conf0[o.n] = a.confN[N];
+        o.nconf[o.n] = nc;
+        o.block0[o.n + 1] = o.block0[o.n] + (int64_t)o.ntile[o.n] * (is_thin ? nc : rows);
+        ++o.n;
+    }
+}
+
+template <typename T>
+static void launch_det_to_csf(const SpinAdapter& a, const CsfView& v, const T* det, T* csf, int nvec, cudaStream_t st) {
+    CsfTiles t, thin;
+    tiles_of(a, t, sizeof(T) == 8 ? &thin : nullptr);
+    if constexpr (sizeof(T) == 8)
+        if (thin.n > 0) {
+            k_det_to_csf_thin<<<dim3((unsigned)thin.block0[thin.n], (unsigned)nvec), 256, 0, st>>>(
+                thin, v, a.conf_byN.get(), det, csf, a.s->ndet, a.ncsf);
+            F2G_LAUNCH("k_det_to_csf_thin");
+        }
+    if (t.n > 0) {
+        k_det_to_csf<T><<<dim3((unsigned)t.block0[t.n], (unsigned)nvec), 256, 0, st>>>(t, v, a.conf_byN.get(), det, csf,
+                                                                                      a.s->ndet, a.ncsf);
+        F2G_LAUNCH("k_det_to_csf");
+    }
 }
 
 static CsfView view_of(const SpinAdapter& a) {
@@ -666,9 +848,7 @@ void SpinAdapter::det_to_csf(const double* det, double* csf, cudaStream_t st, in
         return;
     if (nvec > 65535)
         throw Error(2, "det_to_csf: at most 65535 vectors per call");
-    k_det_to_csf<false><<<dim3((unsigned)ceil_div(ncsf, 256), (unsigned)nvec), 256, 0, st>>>(ncsf, view_of(*this), det,
-                                                                                             csf, s->ndet, ncsf);
-    F2G_LAUNCH("k_det_to_csf");
+    launch_det_to_csf<double>(*this, view_of(*this), det, csf, nvec, st);
 }
 
 // The FP32 transforms (mixed mode): the overlap tables are copied to FP32 once (stream order st).
@@ -705,9 +885,7 @@ void SpinAdapter::det_to_csf(const float* det, float* csf, cudaStream_t st, int 
     if (nvec > 65535)
         throw Error(2, "det_to_csf: at most 65535 vectors per call");
     ensure_fp32_tables(st);
-    k_det_to_csf<false, float><<<dim3((unsigned)ceil_div(ncsf, 256), (unsigned)nvec), 256, 0, st>>>(
-        ncsf, view_of(*this), det, csf, s->ndet, ncsf);
-    F2G_LAUNCH("k_det_to_csf<float>");
+    launch_det_to_csf<float>(*this, view_of(*this), det, csf, nvec, st);
 }
 
 __global__ void k_convert_f2d(int64_t n, const float* __restrict__ in, double* __restrict__ out) {
@@ -772,7 +950,7 @@ void sigma_csf(SigmaBuilder& sb, const SpinAdapter& sa, const double* in, double
 void SpinAdapter::hdiag(const double* det_energy, double* out, cudaStream_t st) const {
     if (ncsf == 0)
         return;
-    k_det_to_csf<true><<<ceil_div(ncsf, 256), 256, 0, st>>>(ncsf, view_of(*this), det_energy, out, 0, 0);
+    k_csf_square<<<ceil_div(ncsf, 256), 256, 0, st>>>(ncsf, view_of(*this), det_energy, out);
     F2G_LAUNCH("k_hdiag");
 }
 

@@ -23,6 +23,8 @@ struct SpinAdapter {
     DevBuf<uint64_t> conf_d, conf_s;       // [nconf] doubly / singly occupied masks (insertion order)
     DevBuf<int64_t> conf_csf, conf_slot;   // [nconf + 1] exclusive offsets
     DevBuf<uint32_t> perm;                 // [nslot] determinant address | negative sign << 31
+    DevBuf<uint32_t> conf_byN;             // [nconf] configurations grouped by open-shell count, in order
+    std::vector<int64_t> confN;            // offsets of the groups in conf_byN
     DevBuf<int64_t> slot_brk, csf_brk;     // configuration of every 256th slot / CSF (and of the last)
 
     SpinAdapter(const CIStrings* s, int twoS, int twoMs);
