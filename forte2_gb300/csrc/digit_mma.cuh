@@ -1,0 +1,118 @@
+// What the kernels that multiply digits on the tensor cores share (oz.cu, rdm_gram.cu): tcgen05, mbarrier and
+// copy instructions, and the conversion of exact 64-bit sums of digit products to FP64.
+#pragma once
+
+#include <cstdint>
+
+namespace f2g {
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
+           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
+}
+__device__ __forceinline__ void mma_commit(uint32_t mbar, uint32_t el) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(mbar),
+                 "r"(el)
+                 : "memory");
+}
+__device__ __forceinline__ uint32_t elect_lane() {
+    uint32_t el;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(el));
+    return el;
+}
+__device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint32_t mbar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
+}
+// bounded wait for phase `parity`; false if it gave up or another thread of the block did
+__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, const volatile int* abort) {
+#pragma unroll 1
+    for (int it = 0; it < (1 << 26); ++it) {
+        uint32_t done;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}\n"
+                     : "=r"(done)
+                     : "r"(mbar), "r"(parity)
+                     : "memory");
+        if (done)
+            return true;
+        if (abort && (it & 63) == 63 && *abort)
+            return false;
+    }
+    return false;
+}
+// the same for a whole warp, which decides together
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t mbar, uint32_t parity, const volatile int* abort) {
+    return __all_sync(0xffffffffu, mbar_wait(mbar, parity, abort));
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t mbar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(mbar)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st4(uint32_t addr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(r0), "r"(r1), "r"(r2),
+                 "r"(r3)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t addr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+// a * b + c on the FMA pipe. The powers of two it is used with come from registers that the compiler cannot see
+// through: as shifts and adds they would go to the integer ALU, which bounds k_oz.
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
+    long long d;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ int opaque(int x) {
+    int y;
+    asm volatile("mov.b32 %0, %1;" : "=r"(y) : "r"(x));
+    return y;
+}
+
+// The FP64 value T 2^(eab - 2100), |T| < 2^63, rounded once to nearest. `base` is (eab - 1016) << 20, and
+// eab - 1014 - 63 >= 1, eab - 1014 <= 2045 (no underflow or overflow whatever T is). The leading bit comes from
+// a conversion of the leading word to FP32: counting leading zeros of 64 bits takes 31 clocks per warp
+// of the slow integer unit, two FP64 additions or the 64-bit conversion instruction more.
+__device__ __forceinline__ double oz_double(long long T, int base, int m20) { // m20: -2^20
+    const uint32_t th = (uint32_t)((unsigned long long)T >> 32);
+    const long long neg = (long long)((int)th >> 31);
+    unsigned long long m = (unsigned long long)((T ^ neg) - neg);
+    const float f = __fmaf_rz(__uint2float_rz((uint32_t)(m >> 32)), 4294967296.0f, __uint2float_rz((uint32_t)m));
+    const uint32_t fe = __float_as_uint(f) >> 23;       // 127 + leading bit's place, 0 for T = 0
+    const int lz1 = 189 - (int)fe;                      // leading zeros of m, less one
+    m = (m << (lz1 & 63)) + 0x200u;                     // leading bit at 62, rounded at bit 10
+    const uint32_t hi = (uint32_t)(m >> 42) + (uint32_t)(lz1 * m20 + base);
+    const uint32_t lo = (uint32_t)(m >> 10);
+    return __hiloint2double((int)(fe == 0 ? 0u : hi | (th & 0x80000000u)), (int)lo);
+}
+// The same for any eab: outside those bounds oz_double at kOzMid, times 2^(eab - kOzMid) in two factors
+constexpr int kOzSafeLo = 1014 + 64, kOzSafeHi = 1014 + 2045, kOzMid = 2000;
+__device__ __forceinline__ double oz_value(long long T, int eab) {
+    const bool safe = eab >= kOzSafeLo && eab <= kOzSafeHi;
+    double d = oz_double(T, ((safe ? eab : kOzMid) - 1016) << 20, -(1 << 20));
+    if (!safe) {
+        const int e = max(-2044, min(2046, eab - kOzMid)), h = e >> 1;
+        d = d * __hiloint2double((h + 1023) << 20, 0) * __hiloint2double((e - h + 1023) << 20, 0);
+    }
+    return d;
+}
+
+} // namespace f2g

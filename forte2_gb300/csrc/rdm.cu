@@ -2,6 +2,10 @@
 // the reference's CISigmaBuilder::compute_{a,b,sf}_1rdm (forte2/ci/ci_sigma_builder_1rdm.cc:9-84),
 // compute_{aa,bb,ab,sf}_2rdm and compute_sf_2cumulant (ci_sigma_builder_2rdm.cc:46-282).
 //
+// The mixed-spin blocks and the larger same-spin blocks are formed on the tensor cores (rdm_gram.cu); the FP64
+// kernels of this file take the small same-spin blocks, and mixed blocks whose strings of one spin outnumber that
+// kernel's operand buffer (a million rows; 20 orbitals with 10 and 3 electrons, say).
+//
 // Hole-list Gram kernel (1-RDMs, same-spin 2-RDMs). With K a string with one (two) fewer
 // electrons and its hole-list entries (I = K + p (+ q), sign), every element is a sum over K of
 // sign * sign' * <bra row I | ket row I'> over pairs of entries of the same K:
@@ -186,33 +190,6 @@ __device__ __forceinline__ double flip(double x, uint32_t neg) {
 }
 
 // ---- hole-list Gram kernel (1-RDMs, same-spin 2-RDMs) ------------------------------------------
-
-// LIST 1: 1-hole lists up1[K][m] (packed 32-bit: address, orbital, sign); output index = orbital.
-// LIST 2: 2-hole lists up2[K][m] (I | p << 32 | q << 40 | negative << 48, p > q); output index
-// p(p-1)/2 + q.
-// LIST 3: 3-hole lists up3[K][m] (I | p << 32 | q << 40 | r << 48 | negative << 56, p > q > r);
-// output index p(p-1)(p-2)/6 + q(q-1)/2 + r.
-template <int LIST>
-__device__ __forceinline__ void hole_entry(const void* list, int64_t at, int64_t& I, int& o, int& neg) {
-    if (LIST == 1) {
-        const uint32_t e = static_cast<const uint32_t*>(list)[at];
-        I = e_addr(e);
-        o = e_orb(e);
-        neg = e_neg(e);
-    } else if (LIST == 2) {
-        const uint64_t e = static_cast<const uint64_t*>(list)[at];
-        I = (int64_t)(e & 0xffffffffull);
-        const int p = (int)((e >> 32) & 0xff), q = (int)((e >> 40) & 0xff);
-        o = p * (p - 1) / 2 + q;
-        neg = (int)((e >> 48) & 1);
-    } else {
-        const uint64_t e = static_cast<const uint64_t*>(list)[at];
-        I = (int64_t)(e & 0xffffffffull);
-        const int p = (int)((e >> 32) & 0xff), q = (int)((e >> 40) & 0xff), r = (int)((e >> 48) & 0xff);
-        o = p * (p - 1) * (p - 2) / 6 + q * (q - 1) / 2 + r;
-        neg = (int)((e >> 56) & 1);
-    }
-}
 
 // Long hole lists are cut into tiles of mt entries; a block takes one (K, tile a, tile b) and
 // forms the mt x mt Gram block of those rows (bra = ket: tile a <= tile b, the upper triangle on
@@ -589,9 +566,16 @@ static void rdm_ab(SigmaBuilder& sb, RdmScratch& R, int which, const double* CL,
     const int ha = which == 1 ? 2 : 1, hb = which == 2 ? 2 : 1;
     if (s.na < ha || s.nb < hb || n < std::max(ha, hb))
         return;
-    MixedLists& M = ensure_pair_lists(sb, R, which, st);
     const bool sym = CL == CR;
     const int64_t NA = s.a.N0, NB = s.b.N0;
+    const int64_t P = (int64_t)n * (n - 1) / 2;
+    // tensor cores: the holes of the outer strings' slots and the other spin's one hole; [p][Q][s][T] for abb
+    const bool done = which == 0   ? rdm_gram(sb, R.gram, 0, 1, true, CL, CR, (int64_t)n * n, n, 1, out, st)
+                      : which == 1 ? rdm_gram(sb, R.gram, 0, 2, true, CL, CR, P * n, n, 1, out, st)
+                                   : rdm_gram(sb, R.gram, 1, 2, true, CL, CR, P * n, 1, P, out, st);
+    if (done)
+        return;
+    MixedLists& M = ensure_pair_lists(sb, R, which, st);
     const size_t slab = (size_t)M.DB * M.DB * sizeof(double);
     const size_t smem_sm = slab + 2 * (size_t)(NB + 1) * sizeof(double);
     const bool use_sm = smem_sm <= smem_optin();
@@ -646,6 +630,8 @@ static void rdm_one(SigmaBuilder& sb, RdmScratch& R, int spin, const double* CL,
     const SpinStrings& ss = sb.s->spin(spin);
     if (ss.k < 1 || ss.N1 == 0 || sb.n < 1)
         return;
+    if (rdm_gram(sb, R.gram, spin, 1, false, CL, CR, sb.n, 1, 0, out, st))
+        return;
     const double *L, *Rr;
     int64_t ncol;
     spin_rows(sb, R, spin, CL, CR, st, L, Rr, ncol);
@@ -657,6 +643,8 @@ static void rdm_same(SigmaBuilder& sb, RdmScratch& R, int spin, const double* CL
                      cudaStream_t st) {
     SpinStrings& ss = sb.s->spin(spin);
     if (ss.k < 2 || ss.N2 == 0 || sb.n < 2)
+        return;
+    if (rdm_gram(sb, R.gram, spin, 2, false, CL, CR, (int64_t)sb.n * (sb.n - 1) / 2, 1, 0, out, st))
         return;
     ss.build_up2(sb.s->binom.get(), st);
     const double *L, *Rr;
@@ -670,6 +658,8 @@ static void rdm_same3(SigmaBuilder& sb, RdmScratch& R, int spin, const double* C
                       cudaStream_t st) {
     SpinStrings& ss = sb.s->spin(spin);
     if (ss.k < 3 || ss.N3 == 0 || sb.n < 3)
+        return;
+    if (rdm_gram(sb, R.gram, spin, 3, false, CL, CR, (int64_t)sb.n * (sb.n - 1) * (sb.n - 2) / 6, 1, 0, out, st))
         return;
     ss.build_up3(sb.s->binom.get(), st);
     const double *L, *Rr;

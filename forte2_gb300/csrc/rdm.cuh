@@ -76,16 +76,60 @@ struct MixedLists {
     DevBuf<uint16_t> pa, pb;   // segment groups
 };
 
+// Device scratch of the tensor-core Gram kernel (rdm_gram.cu)
+struct GramScratch {
+    DevBuf<uint4> zl, zr;         // digits of the bra / ket rows, at most kGramBytes each
+    DevBuf<int> el, er;           // their exponents
+    DevBuf<double> part;          // partial results, at most 2^25 elements
+    DevBuf<uint32_t> tab[2];      // [orbital][K]: the 1-hole lists of a spin by orbital
+};
+
 // Device scratch of the RDM builder, owned by a SigmaBuilder (created on first use).
 struct RdmScratch {
     MixedLists mixed[3];       // ab (2-RDM), aab, abb (3-RDMs)
     DevBuf<double> tl, tr;     // transposed bra / ket (beta-string rows)
     DevBuf<double> t_ab, t_ss, t_g1; // spin-free assembly temporaries
+    GramScratch gram;
     DevBuf<double> t_aaa, t_bbb, t_aab, t_abb, t_g2; // spin-free 3-RDM / 3-cumulant temporaries
 };
+
+// LIST 1: 1-hole lists up1[K][m] (packed 32-bit: address, orbital, sign); output index = orbital.
+// LIST 2: 2-hole lists up2[K][m] (I | p << 32 | q << 40 | negative << 48, p > q); output index
+// p(p-1)/2 + q.
+// LIST 3: 3-hole lists up3[K][m] (I | p << 32 | q << 40 | r << 48 | negative << 56, p > q > r);
+// output index p(p-1)(p-2)/6 + q(q-1)/2 + r.
+template <int LIST>
+__device__ __forceinline__ void hole_entry(const void* list, int64_t at, int64_t& I, int& o, int& neg) {
+    if (LIST == 1) {
+        const uint32_t e = static_cast<const uint32_t*>(list)[at];
+        I = e_addr(e);
+        o = e_orb(e);
+        neg = e_neg(e);
+    } else if (LIST == 2) {
+        const uint64_t e = static_cast<const uint64_t*>(list)[at];
+        I = (int64_t)(e & 0xffffffffull);
+        const int p = (int)((e >> 32) & 0xff), q = (int)((e >> 40) & 0xff);
+        o = p * (p - 1) / 2 + q;
+        neg = (int)((e >> 48) & 1);
+    } else {
+        const uint64_t e = static_cast<const uint64_t*>(list)[at];
+        I = (int64_t)(e & 0xffffffffull);
+        const int p = (int)((e >> 32) & 0xff), q = (int)((e >> 40) & 0xff), r = (int)((e >> 48) & 0xff);
+        o = p * (p - 1) * (p - 2) / 6 + q * (q - 1) / 2 + r;
+        neg = (int)((e >> 56) & 1);
+    }
+}
 
 // out (device, rdm_size(n, kind) doubles) <- RDM `kind` between the bra CL and the ket CR
 // (device FP64 determinant vectors), ordered on st.
 void compute_rdm(SigmaBuilder& sb, int kind, const double* CL, const double* CR, double* out, cudaStream_t st);
+
+// out[(o ko + v kv) d + o' ko + v' kv] += sum over K and the rows R of
+//   sign(K, o) sign(K, o') sum_R x(K + o, R + v) x'(K + o', R + v')
+// for the hole lists (`holes` holes) of spin `spin`, on the tensor cores (rdm_gram.cu); R are the other spin's
+// strings (inner false, v = 0) or its 1-hole strings with v the hole (inner true). False if the shape is left to
+// the FP64 kernels.
+bool rdm_gram(SigmaBuilder& sb, GramScratch& g, int spin, int holes, bool inner, const double* CL, const double* CR,
+              int64_t d, int64_t ko, int64_t kv, double* out, cudaStream_t st);
 
 } // namespace f2g
