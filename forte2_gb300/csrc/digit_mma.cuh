@@ -1,6 +1,8 @@
-// What the kernels that multiply digits on the tensor cores share (oz.cu, rdm_gram.cu): tcgen05, mbarrier and
+// What the kernels that multiply digits on the tensor cores share (oz.cu, rdm_gram.cu, sym_digits.cu): tcgen05, mbarrier and
 // copy instructions, and the conversion of exact 64-bit sums of digit products to FP64.
 #pragma once
+
+#include <cuda_fp16.h>
 
 #include <cstdint>
 
@@ -113,6 +115,45 @@ __device__ __forceinline__ double oz_value(long long T, int eab) {
         d = d * __hiloint2double((h + 1023) << 20, 0) * __hiloint2double((e - h + 1023) << 20, 0);
     }
     return d;
+}
+
+// ---- eight digits of 62 bits ---
+// x 2^(1084 - E) as an integer of 62 bits, E >= the biased exponent of x, digit offsets added: byte 7 - i is digit
+// i + 128 (digit 0 in [-64, 64], the others in [-128, 127]); bits below 1 are rounded to nearest, ties away
+__device__ __forceinline__ uint64_t gram_digits(double x, bool neg, int E) {
+    const uint64_t bits = (uint64_t)__double_as_longlong(x);
+    const int ex = (int)((bits >> 52) & 0x7ff);
+    uint64_t m = (bits & 0xfffffffffffffull) | (ex ? 0x10000000000000ull : 0);
+    m <<= 10; // bit 62: 2 times the integer
+    const int sft = min(E - max(ex, 1), 63);
+    m = ((m >> sft) + 1) >> 1;
+    const uint64_t s = (bits >> 63) ^ (uint64_t)neg;
+    return ((m ^ (0 - s)) + s) + 0x8080808080808080ull;
+}
+template <int I> __device__ __forceinline__ uint32_t gram_half2(uint64_t y0, uint64_t y1) {
+    constexpr uint32_t byte = (7 - I) & 3;
+    const uint32_t a = I < 4 ? (uint32_t)(y0 >> 32) : (uint32_t)y0, b = I < 4 ? (uint32_t)(y1 >> 32) : (uint32_t)y1;
+    const uint32_t t = (__byte_perm(a, b, byte | (byte + 4) << 8) & 0x00ff00ffu) | 0x64006400u;
+    const uint32_t off = 0xE480E480u; // -1152
+    const __half2 r = __hadd2(*reinterpret_cast<const __half2*>(&t), *reinterpret_cast<const __half2*>(&off));
+    return *reinterpret_cast<const uint32_t*>(&r);
+}
+
+// D[tmem] (+)= A[smem] B[smem] like mma_ts, M = 128, N = n; major: kMajorA for an A that is contiguous along M
+constexpr uint32_t kMajorA = 1u << 15;
+__device__ __forceinline__ void mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t n, uint32_t accumulate, uint32_t el,
+                                       uint32_t major = 0) {
+    const uint32_t idesc = (1u << 4) | ((n >> 3) << 17) | (8u << 24) | major;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %4, 0;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+                 :
+                 : "r"(d), "l"(a), "l"(b), "r"(idesc), "r"(el), "r"(accumulate)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_ld4(uint32_t addr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
 }
 
 } // namespace f2g

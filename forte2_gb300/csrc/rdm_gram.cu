@@ -101,19 +101,6 @@ __device__ __forceinline__ void gram_slot(const GramArgs& a, int64_t K, int s, i
     off = (int)(o * a.ko + v * a.kv);
 }
 
-__device__ __forceinline__ void mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t n, uint32_t accumulate, uint32_t el) {
-    const uint32_t idesc = (1u << 4) | ((n >> 3) << 17) | ((uint32_t)(kGM >> 4) << 24);
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %4, 0;\n\tsetp.ne.b32 p, %5, 0;\n\t"
-                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-                 :
-                 : "r"(d), "l"(a), "l"(b), "r"(idesc), "r"(el), "r"(accumulate)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_ld4(uint32_t addr, uint32_t* r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr));
-}
 template <int LIST>
 __global__ void __launch_bounds__(kGThreads, 1) k_rg_gram(const __grid_constant__ GramArgs a, int64_t nitems) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -407,27 +394,6 @@ __global__ void k_rg_tab(const uint32_t* __restrict__ up1, int m, int64_t nK, ui
         return;
     const uint32_t e = up1[t];
     tab[e_orb(e) * nK + t / m] = e_addr(e) | (uint32_t)e_neg(e) << 31;
-}
-
-// x 2^(1084 - E) as an integer of 62 bits, E >= the biased exponent of x, digit offsets added: byte 7 - i is digit
-// i + 128 (digit 0 in [-64, 64], the others in [-128, 127]); bits below 1 are rounded to nearest, ties away
-__device__ __forceinline__ uint64_t gram_digits(double x, bool neg, int E) {
-    const uint64_t bits = (uint64_t)__double_as_longlong(x);
-    const int ex = (int)((bits >> 52) & 0x7ff);
-    uint64_t m = (bits & 0xfffffffffffffull) | (ex ? 0x10000000000000ull : 0);
-    m <<= 10; // bit 62: 2 times the integer
-    const int sft = min(E - max(ex, 1), 63);
-    m = ((m >> sft) + 1) >> 1;
-    const uint64_t s = (bits >> 63) ^ (uint64_t)neg;
-    return ((m ^ (0 - s)) + s) + 0x8080808080808080ull;
-}
-template <int I> __device__ __forceinline__ uint32_t gram_half2(uint64_t y0, uint64_t y1) {
-    constexpr uint32_t byte = (7 - I) & 3;
-    const uint32_t a = I < 4 ? (uint32_t)(y0 >> 32) : (uint32_t)y0, b = I < 4 ? (uint32_t)(y1 >> 32) : (uint32_t)y1;
-    const uint32_t t = (__byte_perm(a, b, byte | (byte + 4) << 8) & 0x00ff00ffu) | 0x64006400u;
-    const uint32_t off = 0xE480E480u; // -1152
-    const __half2 r = __hadd2(*reinterpret_cast<const __half2*>(&t), *reinterpret_cast<const __half2*>(&off));
-    return *reinterpret_cast<const uint32_t*>(&r);
 }
 
 // digits of rows (I, v) (element (I, R + v) of the source, v = 0 without a table) for the rows R k0 .. k0 + 8 k8 of

@@ -30,6 +30,7 @@
 
 #include "sigma.cuh"
 #include "opposite_sym.cuh"
+#include "sym_digits.cuh"
 #include "oz.cuh"
 
 namespace f2g {
@@ -604,6 +605,7 @@ SigmaBuilder::SigmaBuilder(CIStrings* s_, double E_, const double* H_, const dou
     if (opposite_sym_supported(s)) {
         osym = std::make_shared<OppositeSym>();
         osym->build(s);
+        symd = sym_digits_build(s, *osym);
     }
     if (opposite_tc_supported(s)) {
         build_beta_exc(s, beta_exc, 0); // ordered before set_hamiltonian's wait on the legacy stream
@@ -947,6 +949,8 @@ void SigmaBuilder::prepare_untimed(int nvec) {
     gTt.reserve(tot);
     if (oz)
         oz_reserve(*oz, 1, nvec);
+    if (symd)
+        sym_digits_reserve(*symd, s, 1);
     gfC.reserve(tot);
     gfS.reserve(tot);
     gfCt.reserve(tot);
@@ -1269,7 +1273,7 @@ void SigmaBuilder::run(const T* C, T* sig, cudaStream_t st, int mask, bool timed
         }
         if constexpr (sizeof(T) == 8) {
             if (!done && use_sym && osym) {
-                launch_opposite_sym(s, *osym, Vt, C, sig, st, nvec, g_opposite_max_ctas);
+                opposite_sym(Vt, C, sig, st, nvec, g_opposite_max_ctas, graph);
                 done = true;
             }
         }
@@ -1292,6 +1296,15 @@ static void spmm_rows_raw(int64_t nrows, int ncols, int nnz, const int32_t* col,
     dim3 grid((unsigned)nrows, (unsigned)ceil_div(ncols, 128 * VEC), (unsigned)nvec);
     k_spmm_rows<double, VEC><<<grid, 128, smem, st>>>(nrows, ncols, nnz, col, val, X, Y, accumulate ? 1 : 0, vstride);
     F2G_LAUNCH("k_spmm_rows block");
+}
+
+// the opposite-spin term of a space blocked by irreps, on the tensor cores or the FP64 pipe
+void SigmaBuilder::opposite_sym(const double* V, const double* C, double* sig, cudaStream_t st, int nvec, int ctas,
+                                bool graph) {
+    if (symd)
+        sym_digits_run(*symd, s, graph ? 1 : 0, V, C, sig, nvec, ctas, tc_err.get(), st);
+    else
+        launch_opposite_sym(s, *osym, V, C, sig, st, nvec, ctas);
 }
 
 // FP64 sigma of a space blocked by irreps alone on its own vectors (ndet elements each): the same-
@@ -1339,7 +1352,7 @@ void SigmaBuilder::run_blocked_sym(const double* C, double* S, cudaStream_t st, 
     const DetEnum de = s->dets();
     blocks_embed<double>(de, nf, C, xc, nvec, st);
     F2G_CUDA(cudaMemsetAsync(xs, 0, (size_t)nvec * nf * sizeof(double), st));
-    launch_opposite_sym(s, *osym, dV.get(), xc, xs, st, nvec, max_ctas > 0 ? max_ctas : 0);
+    opposite_sym(dV.get(), xc, xs, st, nvec, max_ctas > 0 ? max_ctas : 0, graph);
     blocks_extract<double>(de, nf, xs, S, nvec, st, true);
     if (timed)
         F2G_CUDA(cudaEventRecord(cur_ev[3], st));

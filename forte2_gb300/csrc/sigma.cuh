@@ -61,6 +61,8 @@ struct SigmaBuilder {
     // (opposite_sym.cu); off: the C1 kernel on the embedding (same sigma up to rounding)
     bool use_sym = true;
     std::shared_ptr<struct OppositeSym> osym; // set when the space allows it
+    std::shared_ptr<struct SymDigits> symd;   // osym on the tensor cores, set where that is faster
+    void opposite_sym(const double* V, const double* C, double* sig, cudaStream_t st, int nvec, int ctas, bool graph);
     // such a space's same-spin terms on its own vectors: class-local string Hamiltonians (rows in
     // the space's string order, columns as positions inside the class), rebuilt with the integrals
     DevBuf<int32_t> lcol[2];

@@ -1,0 +1,617 @@
+// Opposite-spin sigma (FP64) of a point-group-blocked space on the tensor cores, exact in digits.
+//
+// For an alpha 1-hole string Ka and the beta 1-hole strings Kb of irrep c,
+//   E[Kb][(p, r)] = sum_(q, s) V[p, r, q, s] sgn C(Ka + q, Kb + s)
+// over the orbital pairs of irrep(q) ^ irrep(s) = t = S ^ irrep(Ka) ^ c with q not in Ka; p, r run over the same pairs,
+// 14 of them (16 with padding) for 14 orbitals in 8 irreps. That is a GEMM with K = N = 16 per Ka and c, 128 strings
+// Kb to a tile: nearly free on the tensor cores, while the FP64 pipe (2 multiply-adds per clock and SM; it takes
+// the pairs with s or r occupied in Kb along, 196 products for 64 that count) needs 3.0 ms for the 9 million hole
+// pairs of CAS(14,14) and took 5.8 ms.
+//
+// The vector, scaled by its largest exponent to integers of 62 bits, is cut into eight FP16 digits once (k_sy_expand:
+// rows (Ia, s) over the Kb of the one irrep that Ia and s leave), the integrals likewise (k_sy_integrals, in the
+// order of each Ka's pairs, sgn(Ka, q) included). k_sy_gemm's A operand is contiguous along M = Kb, so a row's digits go from
+// there to core matrices by 16-byte copies. Products of digits i, j with i + j <= 7 are kept (the next are 2^-64 of
+// the two maxima), sums of at most 64 rows of eight products are exact in FP32, and an element of E is their 96-bit sum
+// rounded once. k_sy_sum adds sgn E into sigma, a thread per determinant in a fixed order.
+//
+// Bound: the copies into shared memory (23 wavefronts per instruction, every 16 bytes land elsewhere). CAS(14,14) in
+// 8 irreps (1,472,512 determinants), opposite-spin term: 5.82 -> 1.74 ms (k_sy_gemm 1.24 ms, k_sy_sum 0.34 ms,
+// k_sy_expand 0.10 ms).
+#include <algorithm>
+
+#include "common.cuh"
+#include "digit_mma.cuh"
+#include "sym_digits.cuh"
+
+namespace f2g {
+
+namespace {
+
+constexpr int kYM = 128;
+constexpr int kYProd = 4, kYEpi = 16;
+constexpr int kYThreads = (kYProd + kYEpi + 1) * 32;
+constexpr int kYA = 8 * kYM * 16 * 2;               // digits of a K step's 16 pairs x 128 strings
+constexpr int kYStagesMax = 6;
+constexpr int kYSmem = 216 * 1024;
+constexpr int64_t kYBytes = int64_t(1) << 31;       // digits, and E, at a time
+constexpr int kYBad = 0x7ff;
+
+struct SymShared {
+    alignas(8) uint64_t full[kYStagesMax], empty[kYStagesMax], acc_full[4], acc_empty[4], drain;
+    uint32_t tmem_base;
+    volatile int abort;
+    uint32_t row[kYProd][kSymSlots]; // [copy warp][pair]: its digits in z, in 16 bytes; ~0: none
+};
+
+struct SymArgs {
+    const uint4 *z, *b;
+    double* e;
+    const int* mx;
+    int* err;
+    const uint32_t* up_a;
+    const int8_t* hka;
+    int64_t N1a;
+    int ma, n, slots, ksteps, tiles, chunk, nirrep, nbuf, stages, stage_bytes;
+    OrbSym os;
+};
+
+// largest biased exponents of a (into mx[0]) and b (into mx[1])
+__global__ void __launch_bounds__(256) k_sy_max(int64_t na, const double* __restrict__ a, int64_t nb,
+                                                const double* __restrict__ b, int* __restrict__ mx) {
+    for (int w = 0; w < 2; ++w) {
+        const uint32_t* hi = reinterpret_cast<const uint32_t*>(w ? b : a) + 1;
+        const int64_t n = w ? nb : na, stride = (int64_t)gridDim.x * 256;
+        uint32_t m = 0;
+#pragma unroll 8
+        for (int64_t i = blockIdx.x * (int64_t)256 + threadIdx.x; i < n; i += stride)
+            m = max(m, __ldg(hi + 2 * i) & 0x7fffffffu);
+        m = __reduce_max_sync(0xffffffffu, m);
+        if ((threadIdx.x & 31) == 0 && m)
+            atomicMax(mx + w, (int)(m >> 20));
+    }
+}
+
+__global__ void k_sy_tab(const uint32_t* __restrict__ up_b, int mb, int64_t N1b, int n, int lmax,
+                         const int32_t* __restrict__ kpos, uint32_t* __restrict__ tab) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t >= N1b * mb)
+        return;
+    const int32_t p = kpos[t / mb];
+    const uint32_t e = up_b[t];
+    tab[((int64_t)(p >> 24) * n + e_orb(e)) * lmax + (p & 0xffffff)] = e_addr(e) | (uint32_t)e_neg(e) << 31;
+}
+
+__device__ __forceinline__ void digits8(const uint64_t (&y)[8], uint4* dst, int stride) {
+#define F2G_DIGIT(D)                                                                                               \
+    dst[D * stride] = make_uint4(gram_half2<D>(y[0], y[1]), gram_half2<D>(y[2], y[3]), gram_half2<D>(y[4], y[5]),   \
+                                 gram_half2<D>(y[6], y[7]))
+    F2G_DIGIT(0);
+    F2G_DIGIT(1);
+    F2G_DIGIT(2);
+    F2G_DIGIT(3);
+    F2G_DIGIT(4);
+    F2G_DIGIT(5);
+    F2G_DIGIT(6);
+    F2G_DIGIT(7);
+#undef F2G_DIGIT
+}
+
+// z[(Ia, s)][group of 8 positions][digit][8]: C(Ia, Kb + s) sgn for the Kb of irrep S ^ irrep(Ia) ^ irrep(s), positions
+// pos0 .. pos0 + chunk
+__global__ void __launch_bounds__(256) k_sy_expand(const double* __restrict__ C, int64_t N0a, int64_t N0b, int n, int lmax,
+                                                   int pos0, int chunk, const int8_t* __restrict__ hja, const __grid_constant__ OrbSym os,
+                                                   const uint32_t* __restrict__ tab, const int* __restrict__ mx,
+                                                   uint4* __restrict__ z) {
+    __shared__ uint4 sm[8][256]; // a warp's digits, written from here in whole lines
+    const int E = max(mx[0], 1), g8 = chunk >> 3, lane = threadIdx.x & 31; // g8 and with it the total: multiples of 16
+    uint4* my = sm[threadIdx.x >> 5];
+    const int64_t total = N0a * n * g8;
+    for (int64_t t0 = blockIdx.x * (int64_t)256 + (threadIdx.x & ~31); t0 < total; t0 += (int64_t)gridDim.x * 256) {
+        const int64_t t = min(t0 + lane, total - 1);
+        const int g = (int)(t % g8);
+        const int64_t r = t / g8, Ia = r / n;
+        const int s = (int)(r - Ia * n);
+        const uint4* src = reinterpret_cast<const uint4*>(tab + ((int64_t)(os.S ^ hja[Ia] ^ os.h[s]) * n + s) * lmax + pos0 + g * 8);
+        const uint4 a0 = __ldg(src), a1 = __ldg(src + 1);
+        const uint32_t a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        uint64_t y[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            y[j] = gram_digits(a[j] == ~0u ? 0.0 : __ldg(C + Ia * N0b + (a[j] & 0x7fffffffu)), a[j] >> 31, E);
+        uint4 q[8];
+        digits8(y, q, 1);
+#pragma unroll
+        for (int d = 0; d < 8; ++d)
+            my[lane * 8 + (d ^ (lane & 7))] = q[d];
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int o = i * 4 + (lane >> 3), d = lane & 7;
+            if (t0 + o < total)
+                z[(t0 + o) * 8 + d] = my[o * 8 + (d ^ (o & 7))];
+        }
+        __syncwarp();
+    }
+}
+
+// b[(Ka, t)][K step][group of 8 (q, s)][digit][(p, r)][8]: sgn(Ka, q) V[p, r, q, s]; a block per Ka
+__global__ void __launch_bounds__(256) k_sy_integrals(const double* __restrict__ V, int n, int ma, const uint32_t* __restrict__ up_a,
+                                                      const __grid_constant__ OrbSym os, int slots, const int* __restrict__ mx, uint4* __restrict__ b) {
+    __shared__ uint8_t q_of[8][kSymSlots], s_of[8][kSymSlots], neg_of[8][kSymSlots];
+    __shared__ int cnt[8];
+    const int64_t Ka = blockIdx.x;
+    if (threadIdx.x < os.nirrep) {
+        const int t = threadIdx.x;
+        int c = 0;
+        for (int i = 0; i < ma; ++i) {
+            const uint32_t e = up_a[Ka * ma + i];
+            const int q = e_orb(e), h = t ^ os.h[q];
+            for (int j = 0; j < os.cnt[h]; ++j, ++c) {
+                q_of[t][c] = (uint8_t)q;
+                s_of[t][c] = (uint8_t)os.list[h][j];
+                neg_of[t][c] = (uint8_t)e_neg(e);
+            }
+        }
+        cnt[t] = c;
+    }
+    __syncthreads();
+    const int E = max(mx[1], 1), groups = slots >> 3;
+    for (int i = threadIdx.x; i < os.nirrep * groups * slots; i += 256) {
+        const int o = i % slots, g = i / slots % groups, t = i / (slots * groups);
+        uint64_t y[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int k = g * 8 + j;
+            double x = 0.0;
+            bool neg = false;
+            if (o < cnt[t] && k < cnt[t]) {
+                x = __ldg(V + (((int64_t)q_of[t][o] * n + s_of[t][o]) * n + q_of[t][k]) * n + s_of[t][k]);
+                neg = neg_of[t][k];
+            }
+            y[j] = gram_digits(x, neg, E);
+        }
+        digits8(y, b + ((Ka * os.nirrep + t) * groups + g) * 8 * slots + o, slots);
+    }
+}
+
+// item: Ka, irrep of Kb, tile of 128 positions
+__device__ __forceinline__ void sym_item(const SymArgs& a, int64_t w, int64_t& Ka, int& c, int& tile) {
+    tile = (int)(w % a.tiles);
+    const int64_t r = w / a.tiles;
+    c = (int)(r % a.nirrep);
+    Ka = r / a.nirrep;
+}
+
+__global__ void __launch_bounds__(kYThreads, 1) k_sy_gemm(const __grid_constant__ SymArgs a, int64_t nitems) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    SymShared& sh = *reinterpret_cast<SymShared*>(smem_raw);
+    const uint32_t ring = smem_u32(smem_raw) + ((sizeof(SymShared) + 1023) / 1024) * 1024;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const volatile int* abort = &sh.abort;
+    if (tid == 0) {
+        for (int i = 0; i < kYStagesMax; ++i) {
+            mbar_init(smem_u32(&sh.full[i]), kYProd * 32);
+            mbar_init(smem_u32(&sh.empty[i]), 1);
+        }
+        for (int i = 0; i < 4; ++i) {
+            mbar_init(smem_u32(&sh.acc_full[i]), 1);
+            mbar_init(smem_u32(&sh.acc_empty[i]), kYEpi);
+        }
+        mbar_init(smem_u32(&sh.drain), 1);
+        sh.abort = 0;
+    }
+    if (warp == kYProd + kYEpi) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem_base)),
+                     "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_before();
+    __syncthreads();
+    fence_after();
+    constexpr uint32_t tmem = 0; // all 512 columns are this block's
+    auto give_up = [&]() {
+        atomicExch(a.err, 1);
+        sh.abort = 1;
+    };
+    const uint32_t cols = 8u * a.slots; // accumulators of an item: eight groups
+    // neighbouring items, so that a Ka's list is read once per block, not once per item and waited for
+    const int64_t w0 = blockIdx.x * nitems / gridDim.x, w1 = (blockIdx.x + 1) * nitems / gridDim.x;
+
+    if (warp < kYProd) {
+        // ---- copies: a K step (16 pairs) per stage, eight pairs x 64 strings per warp; lanes take 8 pairs x 4 digits
+        uint32_t slot = 0, phase = 1, e = 0;
+        int64_t last = -1;
+        int hk = 0;
+        bool ok = true;
+        for (int64_t w = w0; ok && w < w1; ++w) {
+            int64_t Ka;
+            int c, tile;
+            sym_item(a, w, Ka, c, tile);
+            if (Ka != last) {
+                last = Ka;
+                hk = a.hka[Ka];
+                if (lane < a.ma)
+                    e = __ldg(a.up_a + Ka * a.ma + lane);
+            }
+            const int t = a.os.S ^ hk ^ c;
+            __syncwarp();
+            for (int i = lane; i < kSymSlots; i += 32)
+                sh.row[warp][i] = ~0u;
+            __syncwarp();
+            int at = 0, h = 0, cn = 0;
+            if (lane < a.ma) {
+                h = t ^ a.os.h[e_orb(e)];
+                cn = a.os.cnt[h];
+            }
+            int incl = cn;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o)
+                    incl += y;
+            }
+            at = incl - cn;
+            for (int j = 0; j < cn; ++j)
+                sh.row[warp][at + j] = (uint32_t)((e_addr(e) * (uint32_t)a.n + a.os.list[h][j]) * (uint32_t)a.chunk);
+            __syncwarp();
+            const uint4* zt = a.z + tile * kYM + (warp >> 1) * (kYM / 2) + (lane >> 3);
+            const uint4* bt = a.b + (Ka * a.nirrep + t) * (int64_t)(a.slots * a.slots) + tid;
+            for (int ks = 0; ks < a.ksteps; ++ks) {
+                if (!mbar_wait_warp(smem_u32(&sh.empty[slot]), phase, abort)) {
+                    give_up();
+                    ok = false;
+                    break;
+                }
+                const uint32_t dst = ring + slot * a.stage_bytes;
+                const uint32_t r = sh.row[warp][ks * 16 + (warp & 1) * 8 + (lane & 7)];
+                const uint4* src = zt + (r == ~0u ? 0 : r);
+                const uint32_t to = dst + (lane >> 3) * (kYM * 32) + (warp >> 1) * (kYM * 16) + ((warp & 1) * 8 + (lane & 7)) * 16, bytes = r == ~0u ? 0 : 16;
+#pragma unroll 8
+                for (int k = 0; k < kYM / 16; ++k)
+#pragma unroll
+                    for (int d = 0; d < 2; ++d)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + d * 4 * (kYM * 32) + k * 256),
+                                     "l"(src + k * 8 + d * 4), "r"(bytes));
+                for (int i = 0; i < a.slots / 8; ++i) // 16 slots pieces in all, contiguous
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + kYA + (i * 128 + tid) * 16),
+                                 "l"(bt + ks * 16 * a.slots + i * 128));
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&sh.full[slot]))
+                             : "memory");
+                if (++slot == (uint32_t)a.stages) {
+                    slot = 0;
+                    phase ^= 1;
+                }
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else if (warp < kYProd + kYEpi) {
+        // ---- drains: a row's eight groups into one FP64 number, four columns at a time
+        const int quarter = warp & 3, part = (warp - kYProd) >> 2;
+        uint32_t buf = 0, phase = 0;
+        const int ec = max(a.mx[0], 1), ev = max(a.mx[1], 1);
+        const bool bad = ec >= kYBad || ev >= kYBad;
+        const int e0 = 88 - 68 + ec + ev;
+        const bool safe = e0 - 32 >= kOzSafeLo && e0 <= kOzSafeHi;
+        for (int64_t w = w0; w < w1; ++w) {
+            int64_t Ka;
+            int c, tile;
+            sym_item(a, w, Ka, c, tile);
+            if (!mbar_wait_warp(smem_u32(&sh.acc_full[buf]), phase, abort)) {
+                give_up();
+                break;
+            }
+            fence_after();
+            const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + buf * cols;
+            const int64_t pitch = (int64_t)a.nirrep * a.chunk;
+            double* out = a.e + (Ka * a.slots) * pitch + (int64_t)c * a.chunk + tile * kYM + quarter * 32 + lane;
+            for (int b = part; b < a.slots / 4; b += kYEpi / 4) {
+                uint32_t r[32];
+#pragma unroll
+                for (int g = 0; g < 8; ++g)
+                    tmem_ld4(at + g * a.slots + b * 4, r + 4 * g);
+                tmem_wait_ld();
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    int G[8], P[4];
+#pragma unroll
+                    for (int g = 0; g < 8; ++g)
+                        G[g] = __float2int_rn(__uint_as_float(r[4 * g + j]));
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) // at most 64 rows of 6 products of 2^14 in the leading one: below 2^31
+                        P[g] = G[2 * g] * 256 + G[2 * g + 1];
+                    long long hi = mad_wide(P[0], 65536, P[1]), lo = mad_wide(P[2], 65536, P[3]);
+                    // hi 2^32 + lo, |hi| < 2^47: its leading 64 bits, then one rounding
+                    hi += lo >> 32;
+                    uint32_t low = (uint32_t)lo;
+                    const bool neg = hi < 0;
+                    if (neg) {
+                        low = 0u - low;
+                        hi = ~hi + (low == 0);
+                    }
+                    const int sft = min(32, __clz((uint32_t)((unsigned long long)hi >> 16)) + 14);
+                    long long T = (hi << sft) | (long long)((unsigned long long)low >> (32 - sft));
+                    T = neg ? -T : T;
+                    // units of T: 2^(32 - sft) 2^56 2^(ec - 1084) 2^(ev - 1084)
+                    const double x = safe ? oz_double(T, (e0 - sft - 1016) << 20, -(1 << 20)) : oz_value(T, e0 - sft);
+                    out[(b * 4 + j) * pitch] = bad ? __longlong_as_double(0x7ff8000000000000ll) : x;
+                }
+            }
+            fence_before();
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive(smem_u32(&sh.acc_empty[buf]));
+            if (++buf == (uint32_t)a.nbuf) {
+                buf = 0;
+                phase ^= 1;
+            }
+        }
+    } else {
+        // ---- MMAs
+        const uint32_t el = elect_lane();
+        const uint32_t ns = (uint32_t)a.slots, lbo_b = 8 * ns * 16;
+        uint32_t slot = 0, phase = 0, buf = 0, buf_phase = 1;
+        bool ok = true;
+        for (int64_t w = w0; ok && w < w1; ++w) {
+            if (!mbar_wait_warp(smem_u32(&sh.acc_empty[buf]), buf_phase, abort)) {
+                ok = false;
+                break;
+            }
+            const uint32_t acc = tmem + buf * cols;
+            for (int ks = 0; ks < a.ksteps; ++ks) {
+                if (!mbar_wait_warp(smem_u32(&sh.full[slot]), phase, abort)) {
+                    ok = false;
+                    break;
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // generic copies, read by the MMAs
+                fence_after();
+                // A: 8 strings contiguous per core matrix row, next 8 strings 256 bytes on, next 8 pairs 128
+                const uint64_t ad = smem_desc(ring + slot * a.stage_bytes, 128, 256);
+                const uint64_t bd = smem_desc(ring + slot * a.stage_bytes + kYA, lbo_b, 128);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    uint32_t n = (uint32_t)(8 - i) * ns, dcol = acc + i * ns;
+                    uint64_t b = bd;
+                    if (n > 256) {
+                        mma_ss(dcol, ad + i * (kYM * 32 / 16), b, 256, ks > 0 || i > 0, el, kMajorA);
+                        n -= 256, dcol += 256, b += 256;
+                    }
+                    mma_ss(dcol, ad + i * (kYM * 32 / 16), b, n, ks > 0 || i > 0, el, kMajorA);
+                }
+                mma_commit(smem_u32(&sh.empty[slot]), el);
+                if (++slot == (uint32_t)a.stages) {
+                    slot = 0;
+                    phase ^= 1;
+                }
+            }
+            if (ok)
+                mma_commit(smem_u32(&sh.acc_full[buf]), el);
+            if (++buf == (uint32_t)a.nbuf) {
+                buf = 0;
+                buf_phase ^= 1;
+            }
+        }
+        if (!ok)
+            give_up();
+        mma_commit(smem_u32(&sh.drain), el); // the instructions in flight end before the block leaves
+        mbar_wait_warp(smem_u32(&sh.drain), 0, nullptr);
+    }
+    __syncwarp();
+    __syncthreads();
+    if (warp == kYProd + kYEpi) {
+        fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
+// sigma(Ja, Jb) += sum over p in Ja, r in Jb with Jb - r among this chunk's positions; a block per Ja and 256 strings Jb
+__global__ void __launch_bounds__(256) k_sy_sum(int64_t N0b, int n, int na, int nb, int ma, int slots, int pos0, int chunk,
+                                                const __grid_constant__ OrbSym os, const uint32_t* __restrict__ down_a,
+                                                const uint32_t* __restrict__ up_a, const uint32_t* __restrict__ down_b,
+                                                const int32_t* __restrict__ kpos, const int8_t* __restrict__ hja,
+                                                const int32_t* __restrict__ jb, const int32_t* __restrict__ njb_of, int64_t njb,
+                                                const double* __restrict__ E, double* __restrict__ sig) {
+    __shared__ int off[32][8]; // [p of Ja][t]: the first pair of p
+    const int64_t Ja = blockIdx.x;
+    const int h = os.S ^ hja[Ja], cnt = njb_of[h];
+    if ((int64_t)blockIdx.y * 256 >= cnt)
+        return;
+    for (int i = threadIdx.x; i < na * os.nirrep; i += 256) {
+        const int pi = i / os.nirrep, t = i % os.nirrep;
+        const uint32_t ep = down_a[Ja * na + pi];
+        int o = 0;
+        for (int q = 0; q < ma; ++q) { // pairs in the order of Ka's list
+            const int oq = e_orb(up_a[(int64_t)e_addr(ep) * ma + q]);
+            if (oq == e_orb(ep))
+                break;
+            o += os.cnt[t ^ os.h[oq]];
+        }
+        off[pi][t] = o;
+    }
+    __syncthreads();
+    const int64_t at = (int64_t)blockIdx.y * 256 + threadIdx.x;
+    if (at >= cnt)
+        return;
+    const int64_t Jb = jb[h * njb + at], pitch = (int64_t)os.nirrep * chunk;
+    double* out = sig + Ja * N0b + Jb;
+    double acc = *out;
+    for (int pi = 0; pi < na; ++pi) {
+        const uint32_t ep = __ldg(down_a + Ja * na + pi);
+        const int hp = os.h[e_orb(ep)];
+        const double* e0 = E + (int64_t)e_addr(ep) * slots * pitch;
+#pragma unroll 8
+        for (int j = 0; j < nb; ++j) {
+            const uint32_t er = __ldg(down_b + Jb * nb + j);
+            const int r = e_orb(er), kp = __ldg(kpos + e_addr(er)), pos = (kp & 0xffffff) - pos0;
+            if (pos >= 0 && pos < chunk) {
+                const double x = __ldg(e0 + (off[pi][hp ^ os.h[r]] + os.pos[r]) * pitch + (int64_t)(kp >> 24) * chunk + pos);
+                acc += (e_neg(ep) ^ e_neg(er)) ? -x : x;
+            }
+        }
+    }
+    *out = acc;
+}
+
+int sm_total() {
+    int dev = 0, sms = 0;
+    F2G_CUDA(cudaGetDevice(&dev));
+    F2G_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    return sms;
+}
+
+} // namespace
+
+std::shared_ptr<SymDigits> sym_digits_build(const CIStrings* s, const OppositeSym& t) {
+    const int n = s->norb;
+    int nir = 1; // closed under products, whatever irreps occur
+    while (nir < t.os.nirrep || nir <= t.os.S)
+        nir *= 2;
+    const int64_t N1a = s->a.N1, N1b = s->b.N1, N0a = s->a.N0, N0b = s->b.N0;
+    if (N1a == 0 || N1b == 0 || s->a.m1 > 32 || s->na > 32 || nir > 8)
+        return nullptr;
+    auto d = std::make_shared<SymDigits>();
+    d->os = t.os;
+    d->os.nirrep = nir;
+    std::vector<uint64_t> bt(kBinomLd * kBinomLd);
+    for (int a = 0; a < kBinomLd; ++a)
+        for (int b = 0; b < kBinomLd; ++b)
+            bt[a * kBinomLd + b] = host_binom(a, b);
+    auto irrep = [&](uint64_t m) {
+        int h = 0;
+        for (; m; m &= m - 1)
+            h ^= t.os.h[__builtin_ctzll(m)];
+        return h;
+    };
+    // pairs per (Ka, t)
+    std::vector<int8_t> hka(N1a), hja(N0a);
+    int most = 0;
+    for (int64_t K = 0; K < N1a; ++K) {
+        const uint64_t m = string_unrank((uint64_t)K, n, s->na - 1, bt.data());
+        hka[K] = (int8_t)irrep(m);
+        for (int u = 0; u < nir; ++u) {
+            int c = 0;
+            for (int q = 0; q < n; ++q)
+                if (!(m >> q & 1))
+                    c += t.os.cnt[u ^ t.os.h[q]];
+            most = std::max(most, c);
+        }
+    }
+    // Below some 2e7 products the FP64 kernel's one launch is the faster one: (10 orbitals, 5, 5) in 8, 4 and 2 irreps
+    // (5e6, 1.4e7 and 4e7) sigma 292, 246, 295 us, here 327, 259, 212 us; (12, 6, 6) in 8 (1.2e8) 829 and 546 us
+    if (most > kSymSlots || (double)N1a * (double)N1b * most * most < 2e7)
+        return nullptr;
+    d->slots = (most + 15) / 16 * 16;
+    for (int64_t I = 0; I < N0a; ++I)
+        hja[I] = (int8_t)irrep(string_unrank((uint64_t)I, n, s->na, bt.data()));
+    std::vector<int32_t> kpos(N1b), count(8, 0);
+    for (int64_t K = 0; K < N1b; ++K) {
+        const int h = irrep(string_unrank((uint64_t)K, n, s->nb - 1, bt.data()));
+        kpos[K] = h << 24 | count[h]++;
+    }
+    d->lmax = (*std::max_element(count.begin(), count.end()) + 127) / 128 * 128;
+    std::vector<std::vector<int32_t>> jb(8);
+    for (int64_t J = 0; J < N0b; ++J)
+        jb[irrep(string_unrank((uint64_t)J, n, s->nb, bt.data()))].push_back((int32_t)J);
+    for (const auto& x : jb)
+        d->njb = std::max<int64_t>(d->njb, (int64_t)x.size());
+    std::vector<int32_t> flat((size_t)(8 * d->njb), 0), nj(8);
+    for (int h = 0; h < 8; ++h) {
+        nj[h] = (int32_t)jb[h].size();
+        std::copy(jb[h].begin(), jb[h].end(), flat.begin() + h * d->njb);
+    }
+    // positions at a time: the vector's digits and E within kYBytes each
+    const int64_t z1 = N0a * n * 16 * 128, e1 = N1a * d->slots * nir * 8 * 128;
+    const int64_t most128 = kYBytes / std::max(z1, e1), all128 = d->lmax / 128;
+    if (most128 < 1 || N1a * nir * (int64_t)d->slots * d->slots * 16 > kYBytes)
+        return nullptr;
+    const int64_t parts = (all128 + most128 - 1) / most128;
+    d->chunk = (int)((all128 + parts - 1) / parts * 128);
+    auto put = [](auto& buf, const auto& v) {
+        buf.reserve(v.size());
+        F2G_CUDA(cudaMemcpy(buf.get(), v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice));
+    };
+    put(d->hka, hka);
+    put(d->hja, hja);
+    put(d->kpos, kpos);
+    put(d->jb, flat);
+    put(d->njb_of, nj);
+    const size_t nt = (size_t)8 * n * d->lmax;
+    d->tab.reserve(nt);
+    F2G_CUDA(cudaMemset(d->tab.get(), 0xff, nt * sizeof(uint32_t)));
+    k_sy_tab<<<(unsigned)ceil_div(N1b * s->b.m1, 256), 256>>>(s->b.up1.get(), s->b.m1, N1b, n, d->lmax, d->kpos.get(),
+                                                              d->tab.get());
+    F2G_LAUNCH("k_sy_tab");
+    F2G_CUDA(cudaStreamSynchronize(0));
+    return d;
+}
+
+void sym_digits_reserve(SymDigits& d, const CIStrings* s, int set) {
+    SymDigits::Scratch& w = d.set[set];
+    const int nir = d.os.nirrep;
+    w.z.reserve((size_t)(s->a.N0 * s->norb * d.chunk));
+    w.b.reserve((size_t)(s->a.N1 * nir * d.slots * d.slots));
+    w.e.reserve((size_t)(s->a.N1 * d.slots * nir * d.chunk));
+    w.mx.reserve(2);
+}
+
+void sym_digits_run(SymDigits& d, const CIStrings* s, int set, const double* V, const double* C, double* sig, int nvec,
+                    int max_ctas, int* err, cudaStream_t st) {
+    if (set == 0)
+        sym_digits_reserve(d, s, 0);
+    SymDigits::Scratch& w = d.set[set];
+    const int n = s->norb, nir = d.os.nirrep;
+    const int64_t N0a = s->a.N0, N0b = s->b.N0, n4 = (int64_t)n * n * n * n;
+    const int sms = sm_total(), ctas = max_ctas > 0 ? std::min(max_ctas, sms) : sms;
+    SymArgs a{};
+    a.z = w.z.get();
+    a.b = w.b.get();
+    a.e = w.e.get();
+    a.mx = w.mx.get();
+    a.err = err;
+    a.up_a = s->a.up1.get();
+    a.hka = d.hka.get();
+    a.N1a = s->a.N1;
+    a.ma = s->a.m1;
+    a.n = n;
+    a.slots = d.slots;
+    a.ksteps = d.slots / 16;
+    a.nirrep = nir;
+    a.chunk = d.chunk;
+    a.nbuf = std::min(4, 512 / (8 * d.slots));
+    a.stage_bytes = kYA + d.slots * 256;
+    a.stages = std::min<int>(kYStagesMax, (kYSmem - (int)((sizeof(SymShared) + 1023) / 1024 * 1024)) / a.stage_bytes);
+    a.os = d.os;
+    F2G_CUDA(cudaFuncSetAttribute(k_sy_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, kYSmem));
+    for (int v = 0; v < nvec; ++v) {
+        const double* x = C + v * N0a * N0b;
+        F2G_CUDA(cudaMemsetAsync(w.mx.get(), 0, 2 * sizeof(int), st));
+        k_sy_max<<<(unsigned)std::min<int64_t>(ceil_div(N0a * N0b, 2048), (int64_t)sms * 8), 256, 0, st>>>(N0a * N0b, x, n4, V,
+                                                                                                         w.mx.get());
+        F2G_LAUNCH("k_sy_max");
+        if (v == 0) {
+            k_sy_integrals<<<(unsigned)s->a.N1, 256, 0, st>>>(V, n, s->a.m1, s->a.up1.get(), d.os, d.slots, w.mx.get(),
+                                                              w.b.get());
+            F2G_LAUNCH("k_sy_integrals");
+        }
+        for (int pos0 = 0; pos0 < d.lmax; pos0 += d.chunk) {
+            // the last part may be shorter than the others: positions past lmax do not exist
+            const int now = std::min(d.chunk, d.lmax - pos0);
+            a.chunk = now;
+            a.tiles = now / kYM;
+            const int64_t work = N0a * n * (now / 8), items = s->a.N1 * nir * a.tiles;
+            k_sy_expand<<<(unsigned)std::min<int64_t>(ceil_div(work, 256), (int64_t)sms * 32), 256, 0, st>>>(
+                x, N0a, N0b, n, d.lmax, pos0, now, d.hja.get(), d.os, d.tab.get(), w.mx.get(), w.z.get());
+            F2G_LAUNCH("k_sy_expand");
+            k_sy_gemm<<<(unsigned)std::min<int64_t>(items, ctas), kYThreads, kYSmem, st>>>(a, items);
+            F2G_LAUNCH("k_sy_gemm");
+            k_sy_sum<<<dim3((unsigned)N0a, (unsigned)ceil_div(d.njb, 256)), 256, 0, st>>>(
+                N0b, n, s->na, s->nb, s->a.m1, d.slots, pos0, now, d.os, s->a.down1.get(), s->a.up1.get(), s->b.down1.get(),
+                d.kpos.get(), d.hja.get(), d.jb.get(), d.njb_of.get(), d.njb, w.e.get(), sig + v * N0a * N0b);
+            F2G_LAUNCH("k_sy_sum");
+        }
+    }
+}
+
+} // namespace f2g
