@@ -34,7 +34,8 @@ constexpr int kYThreads = (kYProd + kYEpi + 1) * 32;
 constexpr int kYA = 8 * kYM * 16 * 2;               // digits of a K step's 16 pairs x 128 strings
 constexpr int kYStagesMax = 6;
 constexpr int kYSmem = 216 * 1024;
-constexpr int64_t kYBytes = int64_t(1) << 31;       // digits, and E, at a time
+constexpr int64_t kYBytes = int64_t(1) << 31;       // digits at a time
+constexpr int64_t kYBytesE = int64_t(1) << 32;      // E at a time
 constexpr int kYBad = 0x7ff;
 
 struct SymShared {
@@ -51,8 +52,8 @@ struct SymArgs {
     int* err;
     const uint32_t* up_a;
     const int8_t* hka;
-    int64_t N1a;
-    int ma, n, slots, ksteps, tiles, chunk, nirrep, nbuf, stages, stage_bytes;
+    int64_t ka0; // first Ka
+    int ma, n, most, slots, ksteps, tiles, chunk, nirrep, nbuf, stages, stage_bytes;
     OrbSym os;
 };
 
@@ -180,7 +181,7 @@ __device__ __forceinline__ void sym_item(const SymArgs& a, int64_t w, int64_t& K
     tile = (int)(w % a.tiles);
     const int64_t r = w / a.tiles;
     c = (int)(r % a.nirrep);
-    Ka = r / a.nirrep;
+    Ka = a.ka0 + r / a.nirrep;
 }
 
 __global__ void __launch_bounds__(kYThreads, 1) k_sy_gemm(const __grid_constant__ SymArgs a, int64_t nitems) {
@@ -306,8 +307,8 @@ __global__ void __launch_bounds__(kYThreads, 1) k_sy_gemm(const __grid_constant_
             fence_after();
             const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + buf * cols;
             const int64_t pitch = (int64_t)a.nirrep * a.chunk;
-            double* out = a.e + (Ka * a.slots) * pitch + (int64_t)c * a.chunk + tile * kYM + quarter * 32 + lane;
-            for (int b = part; b < a.slots / 4; b += kYEpi / 4) {
+            double* out = a.e + (Ka - a.ka0) * a.most * pitch + (int64_t)c * a.chunk + tile * kYM + quarter * 32 + lane;
+            for (int b = part; b * 4 < a.most; b += kYEpi / 4) {
                 uint32_t r[32];
 #pragma unroll
                 for (int g = 0; g < 8; ++g)
@@ -406,8 +407,8 @@ __global__ void __launch_bounds__(kYThreads, 1) k_sy_gemm(const __grid_constant_
     }
 }
 
-// sigma(Ja, Jb) += sum over p in Ja, r in Jb with Jb - r among this chunk's positions; a block per Ja and 256 strings Jb
-__global__ void __launch_bounds__(256) k_sy_sum(int64_t N0b, int n, int na, int nb, int ma, int slots, int pos0, int chunk,
+// sigma(Ja, Jb) += sum over p in Ja, r in Jb with Ja - p and Jb - r in this chunk; a block per Ja and 256 strings Jb
+__global__ void __launch_bounds__(256) k_sy_sum(int64_t N0b, int n, int na, int nb, int ma, int most, int64_t ka0, int64_t ka1, int pos0, int chunk,
                                                 const __grid_constant__ OrbSym os, const uint32_t* __restrict__ down_a,
                                                 const uint32_t* __restrict__ up_a, const uint32_t* __restrict__ down_b,
                                                 const int32_t* __restrict__ kpos, const int8_t* __restrict__ hja,
@@ -430,6 +431,13 @@ __global__ void __launch_bounds__(256) k_sy_sum(int64_t N0b, int n, int na, int 
         }
         off[pi][t] = o;
     }
+    bool any = false;
+    for (int pi = 0; pi < na; ++pi) {
+        const int64_t Ka = e_addr(down_a[Ja * na + pi]);
+        any |= Ka >= ka0 && Ka < ka1;
+    }
+    if (!any)
+        return;
     __syncthreads();
     const int64_t at = (int64_t)blockIdx.y * 256 + threadIdx.x;
     if (at >= cnt)
@@ -440,7 +448,10 @@ __global__ void __launch_bounds__(256) k_sy_sum(int64_t N0b, int n, int na, int 
     for (int pi = 0; pi < na; ++pi) {
         const uint32_t ep = __ldg(down_a + Ja * na + pi);
         const int hp = os.h[e_orb(ep)];
-        const double* e0 = E + (int64_t)e_addr(ep) * slots * pitch;
+        const int64_t Ka = e_addr(ep);
+        if (Ka < ka0 || Ka >= ka1)
+            continue;
+        const double* e0 = E + (Ka - ka0) * most * pitch;
 #pragma unroll 8
         for (int j = 0; j < nb; ++j) {
             const uint32_t er = __ldg(down_b + Jb * nb + j);
@@ -521,13 +532,15 @@ std::shared_ptr<SymDigits> sym_digits_build(const CIStrings* s, const OppositeSy
         nj[h] = (int32_t)jb[h].size();
         std::copy(jb[h].begin(), jb[h].end(), flat.begin() + h * d->njb);
     }
-    // positions at a time: the vector's digits and E within kYBytes each
-    const int64_t z1 = N0a * n * 16 * 128, e1 = N1a * d->slots * nir * 8 * 128;
-    const int64_t most128 = kYBytes / std::max(z1, e1), all128 = d->lmax / 128;
+    // positions at a time: the vector's digits within kYBytes; then hole strings Ka at a time: E within kYBytesE
+    d->most = (most + 3) / 4 * 4; // stored four at a time
+    const int64_t most128 = kYBytes / (N0a * n * 16 * 128), all128 = d->lmax / 128;
     if (most128 < 1 || N1a * nir * (int64_t)d->slots * d->slots * 16 > kYBytes)
         return nullptr;
     const int64_t parts = (all128 + most128 - 1) / most128;
     d->chunk = (int)((all128 + parts - 1) / parts * 128);
+    const int64_t mostka = std::max<int64_t>(1, kYBytesE / ((int64_t)d->most * nir * d->chunk * 8)), kparts = (N1a + mostka - 1) / mostka;
+    d->ka = (N1a + kparts - 1) / kparts;
     auto put = [](auto& buf, const auto& v) {
         buf.reserve(v.size());
         F2G_CUDA(cudaMemcpy(buf.get(), v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice));
@@ -552,7 +565,7 @@ void sym_digits_reserve(SymDigits& d, const CIStrings* s, int set) {
     const int nir = d.os.nirrep;
     w.z.reserve((size_t)(s->a.N0 * s->norb * d.chunk));
     w.b.reserve((size_t)(s->a.N1 * nir * d.slots * d.slots));
-    w.e.reserve((size_t)(s->a.N1 * d.slots * nir * d.chunk));
+    w.e.reserve((size_t)(d.ka * d.most * nir * d.chunk));
     w.mx.reserve(2);
 }
 
@@ -572,9 +585,9 @@ void sym_digits_run(SymDigits& d, const CIStrings* s, int set, const double* V, 
     a.err = err;
     a.up_a = s->a.up1.get();
     a.hka = d.hka.get();
-    a.N1a = s->a.N1;
     a.ma = s->a.m1;
     a.n = n;
+    a.most = d.most;
     a.slots = d.slots;
     a.ksteps = d.slots / 16;
     a.nirrep = nir;
@@ -600,16 +613,21 @@ void sym_digits_run(SymDigits& d, const CIStrings* s, int set, const double* V, 
             const int now = std::min(d.chunk, d.lmax - pos0);
             a.chunk = now;
             a.tiles = now / kYM;
-            const int64_t work = N0a * n * (now / 8), items = s->a.N1 * nir * a.tiles;
+            const int64_t work = N0a * n * (now / 8);
             k_sy_expand<<<(unsigned)std::min<int64_t>(ceil_div(work, 256), (int64_t)sms * 32), 256, 0, st>>>(
                 x, N0a, N0b, n, d.lmax, pos0, now, d.hja.get(), d.os, d.tab.get(), w.mx.get(), w.z.get());
             F2G_LAUNCH("k_sy_expand");
-            k_sy_gemm<<<(unsigned)std::min<int64_t>(items, ctas), kYThreads, kYSmem, st>>>(a, items);
-            F2G_LAUNCH("k_sy_gemm");
-            k_sy_sum<<<dim3((unsigned)N0a, (unsigned)ceil_div(d.njb, 256)), 256, 0, st>>>(
-                N0b, n, s->na, s->nb, s->a.m1, d.slots, pos0, now, d.os, s->a.down1.get(), s->a.up1.get(), s->b.down1.get(),
-                d.kpos.get(), d.hja.get(), d.jb.get(), d.njb_of.get(), d.njb, w.e.get(), sig + v * N0a * N0b);
-            F2G_LAUNCH("k_sy_sum");
+            for (int64_t ka0 = 0; ka0 < s->a.N1; ka0 += d.ka) {
+                const int64_t ka1 = std::min(ka0 + d.ka, s->a.N1), items = (ka1 - ka0) * nir * a.tiles;
+                a.ka0 = ka0;
+                k_sy_gemm<<<(unsigned)std::min<int64_t>(items, ctas), kYThreads, kYSmem, st>>>(a, items);
+                F2G_LAUNCH("k_sy_gemm");
+                k_sy_sum<<<dim3((unsigned)N0a, (unsigned)ceil_div(d.njb, 256)), 256, 0, st>>>(
+                    N0b, n, s->na, s->nb, s->a.m1, d.most, ka0, ka1, pos0, now, d.os, s->a.down1.get(), s->a.up1.get(),
+                    s->b.down1.get(), d.kpos.get(), d.hja.get(), d.jb.get(), d.njb_of.get(), d.njb, w.e.get(),
+                    sig + v * N0a * N0b);
+                F2G_LAUNCH("k_sy_sum");
+            }
         }
     }
 }

@@ -11,9 +11,11 @@ constexpr int kSymSlots = 64; // orbital pairs (q, s) of one irrep per hole pair
 
 struct SymDigits {
     OrbSym os{};
-    int slots = 0;    // pairs per hole pair at most, padded to 16
+    int most = 0;     // pairs per hole pair at most, padded to 4
+    int slots = 0;    // padded to 16
     int lmax = 0;     // beta 1-hole strings of one irrep at most, padded to 128
     int chunk = 0;    // of them at a time, a multiple of 128
+    int64_t ka = 0;   // alpha 1-hole strings at a time
     int64_t njb = 0;  // beta strings of one irrep at most
     DevBuf<int8_t> hka, hja;      // irreps of the alpha 1-hole strings and strings
     DevBuf<int32_t> kpos;         // beta 1-hole string -> irrep << 24 | position among its irrep's
