@@ -727,7 +727,7 @@ void dg_stage(const DGState* st, const double* b, int64_t ld, int R, int64_t n, 
     F2G_LAUNCH("k_dg_stage");
 }
 
-// Bodies shared by the one-kernel-per-step iteration and the fused one-block iteration. Loops are
+// Bodies shared by the one-kernel-per-step iteration and the fused one-cluster iteration. Loops are
 // grid-stride, so a body called from a one-block kernel covers everything with that block.
 
 __device__ void dg_unstage_body(const DGState* st, const double* __restrict__ in, int R, int64_t n,
@@ -1461,9 +1461,12 @@ void dg_gs_multi(DGState* st, const DGParams& P, double* b, int64_t ld, const do
 // (unstage, subspace matrix, Jacobi, residuals, convergence, collapse with its checks, projection, Gram-
 // Schmidt). Every block owns a slice of all vectors and runs the subspace steps redundantly on the same
 // numbers; a dot product is one warp per pair and slice, the slices' parts added in block order through
-// distributed shared memory (one cluster barrier per set of dot products). In one block of 64 to 128 threads
-// an iteration of 1,764 elements and 8 vectors took 673 us: its 0.3 M FP64 multiply-adds are 75 us of
-// one SM's FP64 pipe, the rest barriers and the divide and square-root chains of the rotations.
+// distributed shared memory (one cluster barrier per set of dot products), the slices of the basis kept in
+// shared memory. In one block of 64 to 128 threads an iteration of 1,764 elements and 8 vectors took 673 us:
+// its 0.3 M FP64 multiply-adds are 75 us of one SM's FP64 pipe, the rest barriers and the divide and
+// square-root chains of the rotations. Here 68 us (76 us with the basis read from L2 and the norm and the
+// overlaps of a new row reduced one after the other); at 12 vectors 41 us of 140 are the eigenproblem, the rest
+// FP64 dot products and barriers.
 constexpr int kSmallCtas = 8, kSmallThreads = kEigThreads;
 
 template <int MAXM> struct SmallShared {
@@ -1491,6 +1494,13 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
     const int m = st->m, lo = st->sigma_size, it1 = st->iter + 1, gs = min(st->g_size, m);
     // this block's elements
     const int chunk = (n + kSmallCtas - 1) / kSmallCtas, e0 = min(n, rank * chunk), e1 = min(n, e0 + chunk);
+    // the basis rows of the slice in shared memory (global loads were most of every dot product's time); rows that
+    // change are written to both
+    double* bs = reinterpret_cast<double*>(smem_raw + sizeof(SmallShared<MAXM>));
+    const int ne = e1 - e0;
+    for (int i = 0; i < m; ++i)
+        for (int e = tid; e < ne; e += kSmallThreads)
+            bs[i * chunk + e] = b[(int64_t)i * ld + e0 + e];
     int buf = 0;
     // sh.tot[p] = sum over the blocks, in block order, of sh.part[buf][p], p < np
     auto reduce = [&](int np) {
@@ -1504,10 +1514,10 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
         __syncthreads();
         buf ^= 1; // the other buffer: a block that is ahead waits at the next barrier before reusing this one
     };
-    // part of <x, y> over the slice into sh.part[buf][p], by one warp
+    // part of <x, y> over the slice (from its first element on) into sh.part[buf][p], by one warp
     auto dot = [&](const double* x, const double* y, int p) {
         double acc = 0.0;
-        for (int e = e0 + lane; e < e1; e += 32)
+        for (int e = lane; e < ne; e += 32)
             acc += x[e] * y[e];
         for (int off = 16; off > 0; off >>= 1)
             acc += __shfl_down_sync(0xffffffffu, acc, off);
@@ -1530,7 +1540,7 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
     for (int p = warp; p < m * m; p += nw) {
         const int i = p / m, j = p % m;
         if (i >= gs || j >= gs)
-            dot(b + (int64_t)i * ld, sigma + (int64_t)j * ld, p);
+            dot(bs + i * chunk, sigma + (int64_t)j * ld + e0, p);
     }
     reduce(m * m);
     for (int k = tid; k < m * m; k += kSmallThreads) {
@@ -1557,7 +1567,7 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
             double ba = 0.0, sa = 0.0;
             for (int i = 0; i < m; ++i) {
                 const double v = sh.V[i * MAXM + q];
-                ba += b[i * ld + e] * v;
+                ba += bs[i * chunk + e - e0] * v;
                 sa += sigma[i * ld + e] * v;
             }
             const double res = sa - ba * lam;
@@ -1594,13 +1604,14 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
         const int k = P.collapse_k;
         auto overlaps_bad = [&](int mm) {
             for (int p = warp; p < mm * mm; p += nw)
-                dot(b + (int64_t)(p / mm) * ld, b + (int64_t)(p % mm) * ld, p);
+                if (p / mm <= p % mm) // symmetric to the last bit
+                    dot(bs + p / mm * chunk, bs + p % mm * chunk, p);
             if (tid == 0)
                 sh.bad = 0;
             reduce(mm * mm);
             for (int p = tid; p < mm * mm; p += kSmallThreads) {
                 const double d = p / mm == p % mm ? 1.0 : 0.0;
-                if (!(fabs(sh.tot[p] - d) <= 1e-11 + 1e-5 * d))
+                if (p / mm <= p % mm && !(fabs(sh.tot[p] - d) <= 1e-11 + 1e-5 * d))
                     sh.bad = 1;
             }
             __syncthreads();
@@ -1616,14 +1627,14 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
                     double sb = 0.0, ss = 0.0;
                     for (int i = 0; i < m; ++i) {
                         const double c = sh.V[i * MAXM + j];
-                        sb += c * b[i * ld + e];
+                        sb += c * bs[i * chunk + e - e0];
                         ss += c * sigma[i * ld + e];
                     }
                     tmp[j * ldt + e] = sb;
                     tmp[(k + j) * ldt + e] = ss;
                 }
                 for (int j = 0; j < k; ++j) {
-                    b[j * ld + e] = tmp[j * ldt + e];
+                    b[j * ld + e] = bs[j * chunk + e - e0] = tmp[j * ldt + e];
                     sigma[j * ld + e] = tmp[(k + j) * ldt + e];
                 }
             }
@@ -1646,13 +1657,13 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
     if (!stop) {
         // projection of the new directions out of the basis
         for (int p = warp; p < m2 * nroot; p += nw)
-            dot(b + (int64_t)(p / nroot) * ld, r + (int64_t)(p % nroot) * ldr, p);
+            dot(bs + p / nroot * chunk, r + (int64_t)(p % nroot) * ldr + e0, p);
         reduce(m2 * nroot);
         for (int e = e0 + tid; e < e1; e += kSmallThreads)
             for (int j = 0; j < nroot; ++j) {
                 double s = r[j * ldr + e];
                 for (int i = 0; i < m2; ++i)
-                    s += -sh.tot[i * nroot + j] * b[i * ld + e];
+                    s += -sh.tot[i * nroot + j] * bs[i * chunk + e - e0];
                 r[j * ldr + e] = s;
             }
         __syncthreads();
@@ -1661,45 +1672,45 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
         int nadd = 0, refill = 0;
         for (int c = 0; c < to_add + refill; ++c) {
             const int s = m2 + nadd;
-            double* v = b + (int64_t)s * ld;
-            for (int e = e0 + tid; e < e1; e += kSmallThreads)
-                v[e] = c < to_add ? r[(int64_t)c * ldr + e]
-                                  : gs_uniform(P.seed, (uint64_t)it1 * 64 + (c - to_add), (uint64_t)e);
+            double* v = bs + s * chunk;
+            for (int e = tid; e < ne; e += kSmallThreads)
+                v[e] = c < to_add ? r[(int64_t)c * ldr + e0 + e]
+                                  : gs_uniform(P.seed, (uint64_t)it1 * 64 + (c - to_add), (uint64_t)(e0 + e));
             __syncthreads();
             for (int cycle = 0; cycle < 10; ++cycle) {
                 if (s > 0) {
                     for (int p = warp; p < s; p += nw)
-                        dot(b + (int64_t)p * ld, v, p);
+                        dot(bs + p * chunk, v, p);
                     reduce(s);
-                    for (int e = e0 + tid; e < e1; e += kSmallThreads) {
+                    for (int e = tid; e < ne; e += kSmallThreads) {
                         double x = v[e];
                         for (int i = 0; i < s; ++i)
-                            x -= sh.tot[i] * b[(int64_t)i * ld + e];
+                            x -= sh.tot[i] * bs[i * chunk + e];
                         v[e] = x;
                     }
                     __syncthreads();
                 }
-                if (warp == 0)
-                    dot(v, v, 0);
-                reduce(1);
-                const double nrm = sqrt(fmax(sh.tot[0], 0.0));
-                __syncthreads();
-                if (nrm < P.discard)
-                    break;
-                const double inv = 1.0 / nrm;
-                for (int e = e0 + tid; e < e1; e += kSmallThreads)
-                    v[e] *= inv;
-                __syncthreads();
+                // norm and overlaps in one set of dot products, the overlaps scaled as the row is
                 for (int p = warp; p <= s; p += nw)
-                    dot(b + (int64_t)p * ld, v, p); // p = s: the row itself
+                    dot(bs + p * chunk, v, p); // p = s: the row itself
                 reduce(s + 1);
+                const double nrm = sqrt(fmax(sh.tot[s], 0.0));
+                if (nrm < P.discard) {
+                    __syncthreads();
+                    break;
+                }
+                const double inv = 1.0 / nrm;
                 double mo = 0.0;
                 for (int i = 0; i < s; ++i)
-                    mo = fmax(mo, fabs(sh.tot[i]));
-                const double one = sh.tot[s];
+                    mo = fmax(mo, fabs(sh.tot[i] * inv));
+                const double one = sh.tot[s] * inv * inv;
+                for (int e = tid; e < ne; e += kSmallThreads)
+                    v[e] *= inv;
                 __syncthreads();
                 if (mo < P.ortho && fabs(one - 1.0) < P.ortho) {
                     ++nadd;
+                    for (int e = tid; e < ne; e += kSmallThreads)
+                        b[(int64_t)s * ld + e0 + e] = v[e];
                     break;
                 }
             }
@@ -1724,7 +1735,8 @@ template <int MAXM>
 static void launch_small_iter(DGState* st, const DGParams& P, const double* stage_s, int R, double* b, double* sigma,
                               int64_t ld, double* r, int64_t ldr, const double* hdiag, double* G, double* evals,
                               double* V, double* tmp, int64_t ldt, double* hist, cudaStream_t s) {
-    const size_t smem = sizeof(SmallShared<MAXM>);
+    const size_t smem = sizeof(SmallShared<MAXM>) + (size_t)P.maxm * ((P.n + kSmallCtas - 1) / kSmallCtas) * sizeof(double);
+    static_assert(sizeof(SmallShared<MAXM>) + (size_t)MAXM * (kDGSmallN / kSmallCtas) * sizeof(double) <= 227 * 1024);
     F2G_CUDA(cudaFuncSetAttribute(k_dg_small_iter<MAXM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_dg_small_iter<MAXM><<<kSmallCtas, kSmallThreads, smem, s>>>(st, P, stage_s, R, b, sigma, ld, r, ldr, hdiag, G,
                                                                  evals, V, tmp, ldt, hist);
