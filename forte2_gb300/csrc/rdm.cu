@@ -569,6 +569,12 @@ static void rdm_ab(SigmaBuilder& sb, RdmScratch& R, int which, const double* CL,
     const bool sym = CL == CR;
     const int64_t NA = s.a.N0, NB = s.b.N0;
     const int64_t P = (int64_t)n * (n - 1) / 2;
+    const int64_t DB = hb == 1 ? n : P;
+    if ((ha == 2 || hb == 2) && P > 256)
+        throw Error(1, "RDM pair list: more than 256 hole sets (at most 23 orbitals for two holes)");
+    const size_t slab = (size_t)(DB * DB) * sizeof(double);
+    if (slab > smem_optin())
+        throw Error(1, "RDM: the mixed-spin slab does not fit in shared memory");
     // tensor cores: the holes of the outer strings' slots and the other spin's one hole; [p][Q][s][T] for abb
     const bool done = which == 0   ? rdm_gram(sb, R.gram, 0, 1, true, CL, CR, (int64_t)n * n, n, 1, out, st)
                       : which == 1 ? rdm_gram(sb, R.gram, 0, 2, true, CL, CR, P * n, n, 1, out, st)
@@ -576,12 +582,9 @@ static void rdm_ab(SigmaBuilder& sb, RdmScratch& R, int which, const double* CL,
     if (done)
         return;
     MixedLists& M = ensure_pair_lists(sb, R, which, st);
-    const size_t slab = (size_t)M.DB * M.DB * sizeof(double);
     const size_t smem_sm = slab + 2 * (size_t)(NB + 1) * sizeof(double);
     const bool use_sm = smem_sm <= smem_optin();
     const size_t smem = use_sm ? smem_sm : slab;
-    if (smem > smem_optin())
-        throw Error(1, "RDM: the mixed-spin slab does not fit in shared memory");
     if (M.wideb) {
         if (use_sm)
             launch_ab<uint64_t, true>(M, M.eb64.get(), NA, NB, CL, CR, sym, out, st, smem);
