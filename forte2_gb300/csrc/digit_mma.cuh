@@ -15,6 +15,11 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
     return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
+// K-major with the 64-byte swizzle: rows of 64 bytes, 8 rows to an atom of 512 (sbo apart), 16-byte piece c of row r at
+// place c ^ (r / 2 % 4)
+__device__ __forceinline__ uint64_t smem_desc_64b(uint32_t addr, uint32_t sbo) {
+    return smem_desc(addr, 16, sbo) | (4ull << 61);
+}
 __device__ __forceinline__ void mma_commit(uint32_t mbar, uint32_t el) {
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
                  "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(mbar),

@@ -10,21 +10,23 @@
 // Arithmetic. A source row is scaled by its largest exponent to integers of 62 bits and cut into eight signed digits
 // of base 256, which are exact FP16 numbers. Products of digits i and j belong to group i + j; the groups 0..7 are
 // kept (the next one is 2^-64 of the row maxima, so that rows with one large and many small elements lose nothing
-// that FP64 sums would keep). A group's sum over 144 rows (288 for groups 0..3, which have half the products) is an
+// that FP64 sums would keep). A group's sum over 128 rows (256 for groups 0..3, which have half the products) is an
 // integer below 2^24: exact in the FP32 accumulators. Then it is added into a 64-bit integer in a register, so a
 // K's whole sum is exact; it is rounded once per K and added in FP64.
 //
 // k_rg_expand writes the digits once per vector, 16 bytes per element, K-major. k_rg_gram copies a K's rows from
-// there into core matrices with 16-byte asynchronous copies and no register work. Groups 0..3 need digits 0..3 only:
-// they and groups 4..7 are separate work items, so that a tile of 128 x 128 fits the accumulators (4 x 128 columns)
-// and operands are loaded 1.5 times, not twice as by column halves. Where a tile has at most 64 slots, M = 128 holds
+// there into swizzled core matrices with 16-byte asynchronous copies and no register work. Groups 0..3 need digits
+// 0..3 only: they and groups 4..7 are separate work items, so that a tile of 128 x 128 fits the accumulators (4 x 128
+// columns) and operands are loaded 1.5 times, not twice as by column halves. Where a tile has at most 64 slots, M = 128 holds
 // the slots of q = 128 / nt adjacent digits: digit i's and the next ones' products with a digit of B come from one
 // instruction (the accumulator rows then belong to groups one apart).
 //
-// Bound: for the mixed block of CAS(14,14) the copies (24 GB from L2 at 4.7 TB/s, 5.2 ms), the tensor cores (36
-// digit pairs, 4.0 ms) and the drains (1.7 ms, not overlapped at 112 slots: the accumulators take 448 of 512
-// columns) by turns. One vector, FP64 kernels -> this file: mixed block 56.3 -> 8.3 ms, same spin 8.5 -> 1.8 ms and
-// 1-RDM 1.32 -> 1.11 ms per spin; CAS(10,10) mixed 3-RDM block 1,394 -> 149 us, same-spin 3-RDM 139 -> 29 us.
+// Bound, for the mixed block of CAS(14,14): the tensor cores (36 digit pairs, 4.0 ms) and the drains (1.7 ms, not
+// overlapped at 112 slots, where the accumulators take 448 of 512 columns), then the operands (24 GB from L2). Rows of a
+// digit lie 64 bytes together in shared memory (64-byte swizzle): with unswizzled core matrices, 16 bytes together,
+// every 16-byte copy was a wavefront of its own and the copies bound the kernel (7.75 ms, now 6.6). One vector, FP64
+// kernels -> this file: mixed block 56.3 -> 7.4 ms, same spin 8.5 -> 1.7 ms and 1-RDM 1.32 -> 1.06 ms per spin;
+// CAS(10,10) mixed 3-RDM block 1,394 -> 137 us, same-spin 3-RDM 139 -> 30 us.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -43,10 +45,10 @@ constexpr int kGCols = kGM / 4;                   // columns per drain thread at
 constexpr int kGMaxStages = 8;
 constexpr int kGBad = 0x7ff;                      // exponent of a row that holds an infinity or NaN
 constexpr int64_t kGramBytes = int64_t(1) << 31;  // digits of one vector at a time
-constexpr int kGSmem = 216 * 1024;
+constexpr int kGSmem = 227 * 1024;
 
 struct GramArgs {
-    const uint4 *zl, *zr;   // [row][K step][digits 0..3, 4..7][2 groups of 8 rows R][4 digits]
+    const uint4 *zl, *zr;   // [row][32 rows R][digit][4 groups of 8 rows R]
     const int *el, *er;
     const void* list;
     double* out;
@@ -54,7 +56,7 @@ struct GramArgs {
     int64_t d, ko, kv, nK;
     int64_t pstride;        // elements of one partial result, 0 if there is only the output
     int parts;              // K goes to partial result K % parts
-    uint32_t k8, nsteps;    // groups of 8 rows R per row (even), K steps
+    uint32_t k8, nsteps;    // groups of 8 rows R per row (a multiple of 4), double K steps of 32 rows
     int m, nv, S, nt, ntile, ntp, q, sym, stages, nbuf, colsbuf, stage_bytes, spt, per_lo, per_hi;
 };
 
@@ -135,12 +137,12 @@ __global__ void __launch_bounds__(kGThreads, 1) k_rg_gram(const __grid_constant_
         atomicExch(a.err, 1);
         sh.abort = 1;
     };
-    const uint32_t a_bytes = (uint32_t)a.nt * 256; // one K step of eight digits (16 rows R) of a tile
+    const uint32_t a_bytes = (uint32_t)a.nt * 512; // a double K step of eight digits (32 rows R) of a tile
 
     if (warp < kGProd) {
-        // ---- copies: spt K steps per stage. Lanes take 4 slots x 128 contiguous bytes, the two warps every other
-        // group of 4 slots. What is left of a tile past its last slot keeps any value: those rows and columns are
-        // not used
+        // ---- copies: spt double K steps per stage. Four lanes take a row's 64 bytes of a digit, eight rows to an
+        // instruction (16-byte pieces that land apart take a wavefront each: 16 bytes per clock); the warps take every
+        // other digit. What is left of a tile past its last slot keeps any value: those rows and columns are not used
         uint32_t slot = 0, phase = 1; // of the stage's `empty`: the first round finds every stage free
         bool ok = true;
         const uint32_t row_pitch = a.k8 * 8;
@@ -156,10 +158,10 @@ __global__ void __launch_bounds__(kGThreads, 1) k_rg_gram(const __grid_constant_
                     sh.row[warp][side][t] = (uint32_t)(I * a.nv + v) * row_pitch;
                 }
             __syncwarp();
-            const int halves = it.lo ? 2 : 1, piece = lane >> 2;
+            const int nd = it.lo ? 8 : 4, row = lane >> 2, piece = lane & 3;
             const uint32_t side_bytes = it.lo ? a_bytes : a_bytes / 2, step_bytes = two ? 2 * side_bytes : side_bytes;
-            const uint32_t dst0 = ((uint32_t)((piece >> 2) * 4 * halves + (piece & 3)) * a.nt + warp * 4 + (lane & 3)) * 16;
-            const uint32_t spt = it.lo ? a.spt : 2 * a.spt, dig4 = (uint32_t)a.nt * 64;
+            const uint32_t dst0 = (uint32_t)row * 64 + ((piece ^ (row >> 1)) & 3) * 16;
+            const uint32_t spt = it.lo ? a.spt : 2 * a.spt, digit_bytes = (uint32_t)a.nt * 64;
             for (uint32_t ks = 0; ks < a.nsteps;) {
                 if (!mbar_wait_warp(smem_u32(&sh.empty[slot]), phase, abort)) {
                     give_up();
@@ -169,21 +171,21 @@ __global__ void __launch_bounds__(kGThreads, 1) k_rg_gram(const __grid_constant_
                 const uint32_t k0 = ks, ke = min(ks + spt, a.nsteps), dst = ring + slot * a.stage_bytes + dst0;
                 ks = ke;
                 for (int side = 0; side < (two ? 2 : 1); ++side) {
-                    const int ng = (min(a.nt, a.S - (side ? it.tb : it.ta) * a.nt) + 7 - warp * 4) >> 3; // groups of this warp
+                    const int ng = (min(a.nt, a.S - (side ? it.tb : it.ta) * a.nt) + 7) >> 3;
                     uint32_t r[kGM / 8];
 #pragma unroll
                     for (int g = 0; g < kGM / 8; ++g)
-                        r[g] = sh.row[warp][side][g * 8 + warp * 4 + (lane & 3)];
-                    const uint4* z = (side ? a.zr : a.zl) + k0 * 16 + piece;
+                        r[g] = sh.row[warp][side][g * 8 + row];
+                    const uint4* z = (side ? a.zr : a.zl) + k0 * 32 + piece;
                     uint32_t to = dst + side * side_bytes;
-                    for (uint32_t k = k0; k < ke; ++k, z += 16, to += step_bytes)
-                        for (int h = 0; h < halves; ++h)
+                    for (uint32_t k = k0; k < ke; ++k, z += 32, to += step_bytes)
+                        for (int d = warp; d < nd; d += kGProd)
 #pragma unroll
                             for (int g = 0; g < kGM / 8; ++g) {
                                 if (g >= ng)
                                     break;
-                                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + h * dig4 + g * 128),
-                                             "l"(z + h * 8 + r[g]));
+                                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + d * digit_bytes + g * 512),
+                                             "l"(z + d * 4 + r[g]));
                             }
                 }
                 // this thread's arrival, once its copies have landed
@@ -290,15 +292,15 @@ __global__ void __launch_bounds__(kGThreads, 1) k_rg_gram(const __grid_constant_
     } else {
         // ---- MMAs
         const uint32_t el = elect_lane();
-        const uint32_t sbo = 128, nt = (uint32_t)a.nt;
+        const uint32_t nt = (uint32_t)a.nt;
         uint32_t slot = 0, phase = 0, buf = 0, buf_phase = 1;
         bool ok = true;
         for (int64_t w = blockIdx.x; ok && w < nitems; w += gridDim.x) {
             const GramItem it = gram_item(a, w);
             const bool two = !(a.sym && it.ta == it.tb);
             const int cm = it.lo ? 7 : 3, cl = it.lo ? max(0, 5 - a.q) : 0;
-            const uint32_t spt = it.lo ? a.spt : 2 * a.spt, per = it.lo ? a.per_lo : a.per_hi, lbo = (it.lo ? 8 : 4) * nt * 16;
-            const uint32_t side16 = 2 * lbo >> 4, step16 = two ? 2 * side16 : side16; // descriptors count 16 bytes
+            const uint32_t spt = it.lo ? a.spt : 2 * a.spt, per = it.lo ? a.per_lo : a.per_hi;
+            const uint32_t side16 = (it.lo ? 8 : 4) * nt * 4, step16 = two ? 2 * side16 : side16; // descriptors count 16 bytes
             for (uint32_t k = 0; ok && k < a.nsteps;) {
                 if (!mbar_wait_warp(smem_u32(&sh.acc_empty[buf]), buf_phase, abort)) {
                     ok = false;
@@ -315,20 +317,22 @@ __global__ void __launch_bounds__(kGThreads, 1) k_rg_gram(const __grid_constant_
                     // fence waits for all copies in flight (1,100 clocks per K step)
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     fence_after();
-                    uint64_t ad = smem_desc(ring + slot * a.stage_bytes, lbo, sbo);
+                    uint64_t ad = smem_desc_64b(ring + slot * a.stage_bytes, 512);
                     for (const uint32_t ke = min(k + spt, kend); k < ke; ++k, ad += step16) {
-                        const uint64_t bd = ad + (two ? side16 : 0);
-                        for (int i = 0; i <= cm; i += a.q) {
-                            const int j0 = max(0, cl - i);
-                            uint32_t n = (uint32_t)(cm - i - j0 + 1) * nt, dcol = acc + (uint32_t)(i + j0 - cl) * nt;
-                            uint64_t b = bd + j0 * nt;
-                            const uint64_t ai = ad + i * nt;
-                            if (n > 256) {
-                                mma_ss(dcol, ai, b, 256, first ^ 1, el);
-                                n -= 256, dcol += 256, b += 256;
+                        for (int h = 0; h < 2; ++h) { // 16 of the 32 rows R: 32 bytes on in every row of 64
+                            const uint64_t bd = ad + (two ? side16 : 0) + 2 * h;
+                            for (int i = 0; i <= cm; i += a.q) {
+                                const int j0 = max(0, cl - i);
+                                uint32_t n = (uint32_t)(cm - i - j0 + 1) * nt, dcol = acc + (uint32_t)(i + j0 - cl) * nt;
+                                uint64_t b = bd + j0 * nt * 4;
+                                const uint64_t ai = ad + 2 * h + i * nt * 4;
+                                if (n > 256) {
+                                    mma_ss(dcol, ai, b, 256, first ^ 1, el);
+                                    n -= 256, dcol += 256, b += 1024;
+                                }
+                                mma_ss(dcol, ai, b, n, first ^ 1, el);
+                                first = 0;
                             }
-                            mma_ss(dcol, ai, b, n, first ^ 1, el);
-                            first = 0;
                         }
                     }
                     mma_commit(smem_u32(&sh.empty[slot]), el);
@@ -453,9 +457,9 @@ __global__ void __launch_bounds__(256) k_rg_expand(const double* __restrict__ C,
         for (int i = 0; i < 8; ++i) {
             const int o = i * 4 + (lane >> 3), d = lane & 7;
             const int64_t at = __shfl_sync(0xffffffffu, zi, o);
-            // [K step][digits 0..3, 4..7][group of 8][4 digits]
+            // [32 rows R][digit][group of 8]
             if (t0 + o < total)
-                z[(at >> 1) * 16 + (d >> 2) * 8 + (at & 1) * 4 + (d & 3)] = my[o * 8 + (d ^ (o & 7))];
+                z[(at >> 2) * 32 + d * 4 + (at & 3)] = my[o * 8 + (d ^ (o & 7))];
         }
         __syncwarp();
     }
@@ -510,14 +514,14 @@ bool rdm_gram(SigmaBuilder& sb, GramScratch& g, int spin, int holes, bool inner,
     if (nK == 0 || m == 0 || nR == 0)
         return true;
     // The mixed blocks always: their FP64 kernel runs one pass over the other spin's pair list per pair of rows,
-    // 51 us against 17 us at (6 orbitals, 3, 3), 56.3 ms against 8.3 ms at (14, 7, 7). Same-spin blocks where a K is
+    // 51 us against 22 us at (6 orbitals, 3, 3), 56.3 ms against 7.4 ms at (14, 7, 7). Same-spin blocks where a K is
     // worth a tile: two and three holes from m^2 nR = 1.2e5 (1.1e5: 30 us FP64, 37 us here; 2.0e5: 73 and 23 us;
     // 3.9e5: 74 and 24 us), one hole, where a K has few slots, from 2,048 rows R (924 rows: 113 and 181 us; 3,432
-    // rows: 1,320 and 1,110 us)
+    // rows: 1,320 and 1,060 us)
     if (!inner && (holes == 1 ? nR < 2048 : (double)m * m * (double)nR < 1.2e5))
         return false;
     // rows R at a time: digits within kGramBytes, whole drains of 128
-    const int64_t rows = nI * nv, all8 = (nR + 15) / 16 * 2;
+    const int64_t rows = nI * nv, all8 = (nR + 31) / 32 * 4;
     int64_t k8 = all8;
     if (rows * 128 * all8 > kGramBytes) {
         const int64_t most = kGramBytes / (rows * 128) / 16 * 16;
@@ -576,32 +580,35 @@ bool rdm_gram(SigmaBuilder& sb, GramScratch& g, int spin, int holes, bool inner,
     a.m = m;
     a.nv = nv;
     a.S = m * nv;
-    a.ntile = (a.S + kGM - 1) / kGM;
+    // slots per tile: 128 with one operand, 112 with two (two stages of 2 x 112 x 512 bytes just fit)
+    a.ntile = sym && a.S <= kGM ? 1 : (a.S + 111) / 112;
     a.nt = ((a.S + a.ntile - 1) / a.ntile + 15) / 16 * 16;
     a.ntile = (a.S + a.nt - 1) / a.nt;
     a.sym = sym;
     a.ntp = sym ? a.ntile * (a.ntile + 1) / 2 : a.ntile * a.ntile;
     a.q = std::min(8, kGM / a.nt);
     a.colsbuf = std::max(4, 8 - std::max(0, 5 - a.q)) * a.nt;
-    // K steps per drain: 2^24 / 2^14 products of digits, the i q-th digits of A's side in every accumulator
+    // double K steps per drain: 2^24 / 2^14 products of digits, the i q-th digits of A's side in every accumulator
     // (digit 0 is at most 64, so that q = 1 has 7 times and 3 times 2^14 per row)
-    a.per_lo = a.q == 1 ? 9 : 64 / ((8 + a.q - 1) / a.q);
-    a.per_hi = a.q == 1 ? 18 : 64 / ((4 + a.q - 1) / a.q);
+    a.per_lo = a.q == 1 ? 4 : 32 / ((8 + a.q - 1) / a.q);
+    a.per_hi = a.q == 1 ? 8 : 32 / ((4 + a.q - 1) / a.q);
     a.nbuf = 2 * a.colsbuf <= 512 ? 2 : 1;
-    a.stage_bytes = a.nt * 256 * (sym && a.ntile == 1 ? 1 : 2);
-    const int ring = kGSmem - (int)((sizeof(GramShared) + 1023) / 1024 * 1024) - 2048; // a tile's last digits are read
-                                                                                       // as 128 rows
-    // two stages, as large as they can be (seven small ones: same spin 1.99 -> 1.73 ms without the drains). spt K steps of 8 digits (twice that of 4), a divisor of per_lo
-    a.stages = 2;
-    a.spt = a.q == 1 ? 9 : 16;
-    while (a.spt > 1 && a.spt * a.stage_bytes > ring / 2)
-        a.spt /= a.q == 1 ? 3 : 2;
+    a.stage_bytes = a.nt * 512 * (sym && a.ntile == 1 ? 1 : 2);
+    const int ring = kGSmem - (int)((sizeof(GramShared) + 1023) / 1024 * 1024) -
+                     (sym && a.ntile == 1 ? 8192 : 0); // a tile's last digits are read as 128 rows of 64 bytes; behind the
+                                                       // first of two operands lies the second
+    static_assert(kGSmem - (sizeof(GramShared) + 1023) / 1024 * 1024 >= 2 * 2 * 112 * 512);
+    // stages as large as leave two (seven of one K step: same spin 1.99 against 1.73 ms without drains); spt double K steps of 8 digits (twice that of 4), a divisor of per_lo
+    a.spt = a.per_lo;
+    while (a.spt > 1 && 2 * a.spt * a.stage_bytes > ring)
+        a.spt /= 2;
     a.stage_bytes *= a.spt;
+    a.stages = std::min(kGMaxStages, ring / a.stage_bytes);
     const int64_t items = a.nK * a.ntp * 2;
     for (int64_t at = 0; at < all8; at += k8) {
         const int64_t now = std::min(k8, all8 - at);
         a.k8 = (uint32_t)now;
-        a.nsteps = (uint32_t)(now / 2);
+        a.nsteps = (uint32_t)(now / 4);
         const int64_t work = rows * now;
         const unsigned grid = (unsigned)std::min<int64_t>((work + 255) / 256, (int64_t)sms * 32);
         g.zl.reserve((size_t)(rows * k8 * 8));
