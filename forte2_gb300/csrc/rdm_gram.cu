@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(256) k_rg_expand(const double* __restrict__ C,
         __syncwarp();
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const int o = i * 4 + (lane >> 3), d = lane & 7;
+            const int o = i * 4 + (lane & 3), d = lane >> 2; // 512 bytes in the order of the lanes
             const int64_t at = __shfl_sync(0xffffffffu, zi, o);
             // [32 rows R][digit][group of 8]
             if (t0 + o < total)

@@ -15,9 +15,9 @@
 // the two maxima), sums of at most 64 rows of eight products are exact in FP32, and an element of E is their 96-bit sum
 // rounded once. k_sy_sum adds sgn E into sigma, a thread per determinant in a fixed order.
 //
-// Bound: the copies into shared memory (23 wavefronts per instruction, every 16 bytes land elsewhere). CAS(14,14) in
-// 8 irreps (1,472,512 determinants), opposite-spin term: 5.82 -> 1.74 ms (k_sy_gemm 1.24 ms, k_sy_sum 0.34 ms,
-// k_sy_expand 0.10 ms).
+// Bound: operand copies and drains by turns. CAS(14,14) in 8 irreps (1,472,512 determinants), opposite-spin term: 5.82 ->
+// 1.6 ms (k_sy_gemm 1.09 ms, with unswizzled core matrices, whose 16-byte copies take a wavefront each, 1.24 ms;
+// k_sy_sum 0.34 ms, k_sy_expand 0.10 ms).
 #include <algorithm>
 
 #include "common.cuh"
@@ -98,7 +98,7 @@ __device__ __forceinline__ void digits8(const uint64_t (&y)[8], uint4* dst, int 
 #undef F2G_DIGIT
 }
 
-// z[(Ia, s)][group of 8 positions][digit][8]: C(Ia, Kb + s) sgn for the Kb of irrep S ^ irrep(Ia) ^ irrep(s), positions
+// z[(Ia, s)][64 positions][digit][64]: C(Ia, Kb + s) sgn for the Kb of irrep S ^ irrep(Ia) ^ irrep(s), positions
 // pos0 .. pos0 + chunk
 __global__ void __launch_bounds__(256) k_sy_expand(const double* __restrict__ C, int64_t N0a, int64_t N0b, int n, int lmax,
                                                    int pos0, int chunk, const int8_t* __restrict__ hja, const __grid_constant__ OrbSym os,
@@ -128,9 +128,9 @@ __global__ void __launch_bounds__(256) k_sy_expand(const double* __restrict__ C,
         __syncwarp();
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const int o = i * 4 + (lane >> 3), d = lane & 7;
+            const int o = (i & 3) * 8 + (lane & 7), d = (i >> 2) * 4 + (lane >> 3); // eight lanes: 128 bytes
             if (t0 + o < total)
-                z[(t0 + o) * 8 + d] = my[o * 8 + (d ^ (o & 7))];
+                z[((t0 + o) >> 3) * 64 + d * 8 + ((t0 + o) & 7)] = my[o * 8 + (d ^ (o & 7))];
         }
         __syncwarp();
     }
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kYThreads, 1) k_sy_gemm(const __grid_constant_
     const int64_t w0 = blockIdx.x * nitems / gridDim.x, w1 = (blockIdx.x + 1) * nitems / gridDim.x;
 
     if (warp < kYProd) {
-        // ---- copies: a K step (16 pairs) per stage, eight pairs x 64 strings per warp; lanes take 8 pairs x 4 digits
+        // ---- copies: a K step (16 pairs) per stage, four pairs per warp; eight lanes take 64 strings of a digit
         uint32_t slot = 0, phase = 1, e = 0;
         int64_t last = -1;
         int hk = 0;
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kYThreads, 1) k_sy_gemm(const __grid_constant_
             for (int j = 0; j < cn; ++j)
                 sh.row[warp][at + j] = (uint32_t)((e_addr(e) * (uint32_t)a.n + a.os.list[h][j]) * (uint32_t)a.chunk);
             __syncwarp();
-            const uint4* zt = a.z + tile * kYM + (warp >> 1) * (kYM / 2) + (lane >> 3);
+            const uint4* zt = a.z + tile * kYM + (lane & 7);
             const uint4* bt = a.b + (Ka * a.nirrep + t) * (int64_t)(a.slots * a.slots) + tid;
             for (int ks = 0; ks < a.ksteps; ++ks) {
                 if (!mbar_wait_warp(smem_u32(&sh.empty[slot]), phase, abort)) {
@@ -267,15 +267,16 @@ __global__ void __launch_bounds__(kYThreads, 1) k_sy_gemm(const __grid_constant_
                     break;
                 }
                 const uint32_t dst = ring + slot * a.stage_bytes;
-                const uint32_t r = sh.row[warp][ks * 16 + (warp & 1) * 8 + (lane & 7)];
+                const int pair = warp * 4 + (lane >> 3), piece = lane & 7;
+                const uint32_t r = sh.row[warp][ks * 16 + pair];
                 const uint4* src = zt + (r == ~0u ? 0 : r);
-                const uint32_t to = dst + (lane >> 3) * (kYM * 32) + (warp >> 1) * (kYM * 16) + ((warp & 1) * 8 + (lane & 7)) * 16, bytes = r == ~0u ? 0 : 16;
-#pragma unroll 8
-                for (int k = 0; k < kYM / 16; ++k)
+                const uint32_t to = dst + pair * 128 + ((piece ^ pair) & 7) * 16, bytes = r == ~0u ? 0 : 16;
 #pragma unroll
-                    for (int d = 0; d < 2; ++d)
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + d * 4 * (kYM * 32) + k * 256),
-                                     "l"(src + k * 8 + d * 4), "r"(bytes));
+                for (int d = 0; d < 8; ++d)
+#pragma unroll
+                    for (int mb = 0; mb < 2; ++mb)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + d * (kYM * 32) + mb * 2048),
+                                     "l"(src + (mb * 8 + d) * 8), "r"(bytes));
                 for (int i = 0; i < a.slots / 8; ++i) // 16 slots pieces in all, contiguous
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + kYA + (i * 128 + tid) * 16),
                                  "l"(bt + ks * 16 * a.slots + i * 128));
@@ -368,8 +369,9 @@ __global__ void __launch_bounds__(kYThreads, 1) k_sy_gemm(const __grid_constant_
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // generic copies, read by the MMAs
                 fence_after();
-                // A: 8 strings contiguous per core matrix row, next 8 strings 256 bytes on, next 8 pairs 128
-                const uint64_t ad = smem_desc(ring + slot * a.stage_bytes, 128, 256);
+                // A: atoms of 8 pairs x 64 strings (rows of 128 bytes, swizzled), next 64 strings 2,048 bytes on, next
+                // 8 pairs 1,024
+                const uint64_t ad = smem_desc(ring + slot * a.stage_bytes, 2048, 1024) | (2ull << 61);
                 const uint64_t bd = smem_desc(ring + slot * a.stage_bytes + kYA, lbo_b, 128);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
