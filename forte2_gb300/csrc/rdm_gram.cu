@@ -21,12 +21,13 @@
 // the slots of q = 128 / nt adjacent digits: digit i's and the next ones' products with a digit of B come from one
 // instruction (the accumulator rows then belong to groups one apart).
 //
-// Bound, for the mixed block of CAS(14,14): the tensor cores (36 digit pairs, 4.0 ms) and the drains (1.7 ms, not
-// overlapped at 112 slots, where the accumulators take 448 of 512 columns), then the operands (24 GB from L2). Rows of a
-// digit lie 64 bytes together in shared memory (64-byte swizzle): with unswizzled core matrices, 16 bytes together,
-// every 16-byte copy was a wavefront of its own and the copies bound the kernel (7.75 ms, now 6.6). One vector, FP64
-// kernels -> this file: mixed block 56.3 -> 7.4 ms, same spin 8.5 -> 1.7 ms and 1-RDM 1.32 -> 1.06 ms per spin;
-// CAS(10,10) mixed 3-RDM block 1,394 -> 137 us, same-spin 3-RDM 139 -> 30 us.
+// Bound, for the mixed block of CAS(14,14): the tensor cores (36 digit pairs, 4.0 ms), then the drains and the operands
+// (24 GB from L2). At 112 slots the accumulators take 448 of 512 columns: one buffer, whose two halves are drained and
+// refilled in turn, so that the MMAs of one overlap with the drain of the other (as one piece 6.64 ms, so 5.75 ms).
+// Rows of a digit lie 64 bytes together in shared memory (64-byte swizzle): with unswizzled core matrices, 16 bytes
+// together, every 16-byte copy was a wavefront of its own and the copies bound the kernel (7.75 ms, then 6.64). One
+// vector, FP64 kernels -> this file: mixed block 56.3 -> 6.4 ms, same spin 8.5 -> 1.7 ms and 1-RDM 1.32 -> 1.06 ms per
+// spin; CAS(10,10) mixed 3-RDM block 1,394 -> 129 us, same-spin 3-RDM 139 -> 30 us.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -215,44 +216,48 @@ __global__ void __launch_bounds__(kGThreads, 1) k_rg_gram(const __grid_constant_
 #pragma unroll
             for (int j = 0; j < kGCols; ++j)
                 T[j] = 0;
-            for (uint32_t k = 0; k < a.nsteps; k += per) {
-                if (!mbar_wait_warp(smem_u32(&sh.acc_full[buf]), phase, abort)) {
-                    give_up();
-                    ok = false;
-                    break;
-                }
-                fence_after();
-                const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + buf * a.colsbuf + c0;
-                for (int cc = 0; cc < nc; cc += 4) {
-                    int mul[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int g = cl + cc + u + di - base; // this row's group in column block cc + u
-                        mul[u] = cc + u < nc && g >= 0 && g < 4 ? 1 << (8 * (3 - g)) : 0;
+            for (uint32_t k = 0; ok && k < a.nsteps; k += per) {
+                // one buffer: the first half of its column blocks and the second are handed over by themselves
+                for (int half = 0; half < (a.nbuf == 1 ? 2 : 1); ++half) {
+                    const uint32_t bar = a.nbuf == 1 ? half : buf;
+                    if (!mbar_wait_warp(smem_u32(&sh.acc_full[bar]), phase, abort)) {
+                        give_up();
+                        ok = false;
+                        break;
                     }
+                    fence_after();
+                    const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + (a.nbuf == 1 ? 0 : buf * a.colsbuf) + c0;
+                    const int lo = half ? nc / 2 : 0, hi = a.nbuf == 1 && !half ? nc / 2 : nc;
+                    for (int cc = lo; cc < hi; cc += 2) {
+                        int mul[2];
 #pragma unroll
-                    for (int b = 0; b < kGCols / 4; ++b)
-                        if (b < nb) {
-                            uint32_t r[16];
-#pragma unroll
-                            for (int u = 0; u < 4; ++u)
-                                tmem_ld4(at + min(cc + u, nc - 1) * a.nt + b * 4, r + 4 * u);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                                for (int j = 0; j < 4; ++j)
-                                    T[b * 4 + j] = mad_wide(__float2int_rn(__uint_as_float(r[4 * u + j])), mul[u], T[b * 4 + j]);
+                        for (int u = 0; u < 2; ++u) {
+                            const int g = cl + cc + u + di - base; // this row's group in column block cc + u
+                            mul[u] = cc + u < hi && g >= 0 && g < 4 ? 1 << (8 * (3 - g)) : 0;
                         }
+#pragma unroll
+                        for (int b = 0; b < kGCols / 4; ++b)
+                            if (b < nb) {
+                                uint32_t r[8];
+#pragma unroll
+                                for (int u = 0; u < 2; ++u)
+                                    tmem_ld4(at + min(cc + u, hi - 1) * a.nt + b * 4, r + 4 * u);
+                                tmem_wait_ld();
+#pragma unroll
+                                for (int u = 0; u < 2; ++u)
+#pragma unroll
+                                    for (int j = 0; j < 4; ++j)
+                                        T[b * 4 + j] = mad_wide(__float2int_rn(__uint_as_float(r[4 * u + j])), mul[u],
+                                                                T[b * 4 + j]);
+                            }
+                    }
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0)
+                        mbar_arrive(smem_u32(&sh.acc_empty[bar]));
                 }
-                fence_before();
-                __syncwarp();
-                if (lane == 0)
-                    mbar_arrive(smem_u32(&sh.acc_empty[buf]));
-                if (++buf == (uint32_t)a.nbuf) {
-                    buf = 0;
+                if (a.nbuf == 1 || (buf ^= 1) == 0)
                     phase ^= 1;
-                }
             }
             // lane j: offset in the output, exponent and sign of column c0 + j
             int coff = -1, ce = 0, cneg = 0;
@@ -301,13 +306,13 @@ __global__ void __launch_bounds__(kGThreads, 1) k_rg_gram(const __grid_constant_
             const int cm = it.lo ? 7 : 3, cl = it.lo ? max(0, 5 - a.q) : 0;
             const uint32_t spt = it.lo ? a.spt : 2 * a.spt, per = it.lo ? a.per_lo : a.per_hi;
             const uint32_t side16 = (it.lo ? 8 : 4) * nt * 4, step16 = two ? 2 * side16 : side16; // descriptors count 16 bytes
+            const int split = cl + (cm - cl + 1) / 2; // one buffer: column blocks before it are the first half
             for (uint32_t k = 0; ok && k < a.nsteps;) {
-                if (!mbar_wait_warp(smem_u32(&sh.acc_empty[buf]), buf_phase, abort)) {
+                if (!mbar_wait_warp(smem_u32(&sh.acc_empty[a.nbuf == 1 ? 0 : buf]), buf_phase, abort)) {
                     ok = false;
                     break;
                 }
-                const uint32_t acc = tmem + buf * a.colsbuf, kend = min(k + per, a.nsteps);
-                uint32_t first = 1;
+                const uint32_t acc = tmem + (a.nbuf == 1 ? 0 : buf * a.colsbuf), k0 = k, kend = min(k + per, a.nsteps);
                 while (k < kend) {
                     if (!mbar_wait_warp(smem_u32(&sh.full[slot]), phase, abort)) {
                         ok = false;
@@ -317,24 +322,43 @@ __global__ void __launch_bounds__(kGThreads, 1) k_rg_gram(const __grid_constant_
                     // fence waits for all copies in flight (1,100 clocks per K step)
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     fence_after();
-                    uint64_t ad = smem_desc_64b(ring + slot * a.stage_bytes, 512);
-                    for (const uint32_t ke = min(k + spt, kend); k < ke; ++k, ad += step16) {
-                        for (int h = 0; h < 2; ++h) { // 16 of the 32 rows R: 32 bytes on in every row of 64
-                            const uint64_t bd = ad + (two ? side16 : 0) + 2 * h;
-                            for (int i = 0; i <= cm; i += a.q) {
-                                const int j0 = max(0, cl - i);
-                                uint32_t n = (uint32_t)(cm - i - j0 + 1) * nt, dcol = acc + (uint32_t)(i + j0 - cl) * nt;
-                                uint64_t b = bd + j0 * nt * 4;
-                                const uint64_t ai = ad + 2 * h + i * nt * 4;
-                                if (n > 256) {
-                                    mma_ss(dcol, ai, b, 256, first ^ 1, el);
-                                    n -= 256, dcol += 256, b += 1024;
+                    const uint64_t ad0 = smem_desc_64b(ring + slot * a.stage_bytes, 512);
+                    const uint32_t ks = k, ke = min(k + spt, kend);
+                    // column blocks c0 <= c < c1 of the stage's double K steps
+                    auto issue = [&](int c0, int c1) {
+                        uint64_t ad = ad0;
+                        uint32_t add = ks > k0;
+                        for (uint32_t s = ks; s < ke; ++s, ad += step16)
+                            for (int h = 0; h < 2; ++h) { // 16 of the 32 rows R: 32 bytes on in every row of 64
+                                const uint64_t bd = ad + (two ? side16 : 0) + 2 * h;
+                                for (int i = 0; i < c1; i += a.q) {
+                                    const int c = max(i, c0); // digit i reaches column block i and those after it
+                                    uint32_t n = (uint32_t)(c1 - c) * nt, dcol = acc + (uint32_t)(c - cl) * nt;
+                                    uint64_t b = bd + (c - i) * nt * 4;
+                                    const uint64_t ai = ad + 2 * h + i * nt * 4;
+                                    if (n > 256) {
+                                        mma_ss(dcol, ai, b, 256, add, el);
+                                        n -= 256, dcol += 256, b += 1024;
+                                    }
+                                    mma_ss(dcol, ai, b, n, add, el);
+                                    add = 1;
                                 }
-                                mma_ss(dcol, ai, b, n, first ^ 1, el);
-                                first = 0;
                             }
+                    };
+                    if (a.nbuf == 1) {
+                        issue(cl, split);
+                        if (ke == kend)
+                            mma_commit(smem_u32(&sh.acc_full[0]), el);
+                        if (ks == k0 && !mbar_wait_warp(smem_u32(&sh.acc_empty[1]), buf_phase, abort)) {
+                            ok = false;
+                            break;
                         }
+                        fence_after();
+                        issue(split, cm + 1);
+                    } else {
+                        issue(cl, cm + 1);
                     }
+                    k = ke;
                     mma_commit(smem_u32(&sh.empty[slot]), el);
                     if (++slot == (uint32_t)a.stages) {
                         slot = 0;
@@ -342,11 +366,9 @@ __global__ void __launch_bounds__(kGThreads, 1) k_rg_gram(const __grid_constant_
                     }
                 }
                 if (ok)
-                    mma_commit(smem_u32(&sh.acc_full[buf]), el);
-                if (++buf == (uint32_t)a.nbuf) {
-                    buf = 0;
+                    mma_commit(smem_u32(&sh.acc_full[a.nbuf == 1 ? 1 : buf]), el);
+                if (a.nbuf == 1 || (buf ^= 1) == 0)
                     buf_phase ^= 1;
-                }
             }
         }
         if (!ok)
@@ -514,7 +536,7 @@ bool rdm_gram(SigmaBuilder& sb, GramScratch& g, int spin, int holes, bool inner,
     if (nK == 0 || m == 0 || nR == 0)
         return true;
     // The mixed blocks always: their FP64 kernel runs one pass over the other spin's pair list per pair of rows,
-    // 51 us against 22 us at (6 orbitals, 3, 3), 56.3 ms against 7.4 ms at (14, 7, 7). Same-spin blocks where a K is
+    // 51 us against 22 us at (6 orbitals, 3, 3), 56.3 ms against 6.4 ms at (14, 7, 7). Same-spin blocks where a K is
     // worth a tile: two and three holes from m^2 nR = 1.2e5 (1.1e5: 30 us FP64, 37 us here; 2.0e5: 73 and 23 us;
     // 3.9e5: 74 and 24 us), one hole, where a K has few slots, from 2,048 rows R (924 rows: 113 and 181 us; 3,432
     // rows: 1,320 and 1,060 us)

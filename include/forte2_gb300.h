@@ -116,8 +116,8 @@ int f2g_sigma_set_tensor_cores(void* sigma, int on, int* available);
  * spin and at most 146 pairs of holes per string pair, no irreps, else error 2; default 1 from 8,193
  * determinants). No reference counterpart. */
 int f2g_sigma_set_variant(void* sigma, int which, int value);
-/* 1 if a tensor-core build (FP32, or FP64 by digit splitting) gave up waiting for its matrix operations
- * (results invalid). */
+/* 1 if a tensor-core build (FP32, or FP64 by digit splitting, sigma or RDM) gave up waiting for its matrix
+ * operations (results invalid). */
 int f2g_sigma_tc_error(void* sigma, int* out);
 /* Hamiltonian(basis, sigma) for nvec vectors of length ndet stored back to back
  * (ci_sigma_builder.cc:187-218); sigma is overwritten. */
