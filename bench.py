@@ -10,8 +10,9 @@ value     sigma builds/s of the FP64 path with C and sigma resident in HBM (whol
           run independent replicas, weak scaling).
 e2e       the same through the public host-buffer API: CISigmaBuilder.Hamiltonian(numpy C,
           numpy sigma) from pinned host memory, H2D + build + D2H inside the timed region.
-roofline  the dominant kernel (opposite-spin k_opposite): algorithmic FLOPs per launch
-          2 N1a N1b (ma mb)^2 over its CUDA-event duration, against the measured FP64 peak.
+roofline  the dominant phase (opposite spin): the FP16 products of the digit kernel k_oz over the
+          phase's CUDA-event duration, against the measured dense FP16/BF16 rate; spaces outside
+          that kernel's range: FP64 FLOPs of k_opposite against the FP64 rate.
 --impl reference times the reference algorithm's CPU implementation (the oracle port of the
           Harrison-Zarrabian sigma, all host threads, BLAS from numpy's OpenBLAS) on a bounded
           sample of the same build.
@@ -253,6 +254,39 @@ def opposite_traffic(norb, na, nb):
     return 5.04e9 * gathered(norb, na, nb) / gathered(15, 7, 8)
 
 
+def count_launches(fn):
+    """Kernels of this library that one call launches (torch.profiler, untimed)."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    count = 0
+    for _ in range(2):  # a process's first profile may come back empty
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            fn()
+            torch.cuda.synchronize()
+        count = max(count, sum(e.count for e in prof.key_averages() if "f2g::" in e.key))
+    return count
+
+
+def digit_opposite_roofline(norb, na, nb, seconds, fp64_flops, fp64_peak):
+    """Opposite-spin phase of the FP64 sigma on the tensor cores (csrc/oz.cu): per alpha hole string,
+    128 beta hole strings and K step of one annihilated orbital (16 beta orbitals), 28 digit products
+    of M = 128, N = 48 per three created orbitals. The phase also forms the row exponents and adds
+    the products' 64-bit integers into sigma (each written and read once: the traffic given)."""
+    from math import comb
+
+    ma, mb = norb - na + 1, norb - nb + 1
+    n1a, n1b = comb(norb, na - 1), comb(norb, nb - 1)
+    flop = n1a * ((n1b + 127) // 128) * ma * ((ma + 2) // 3) * 28 * 2 * 128 * 48 * 16
+    peak = _measured_peaks().get("bf16_tflops", 1900.0)
+    return {"bound": "tensor", "kernel": "k_oz (opposite-spin sigma in FP16 digits) and its sums",
+            "achieved": flop / seconds / 1e12, "peak": peak, "unit": "TFLOP/s", "frac": flop / seconds / 1e12 / peak,
+            "peak_source": "MEASURED_PEAKS.json bf16_tflops (dense FP16 runs at the BF16 rate)",
+            "flop_per_launch": flop, "launch_ms": 1e3 * seconds, "traffic": 16 * n1a * n1b * ma * mb,
+            "traffic_source": "algorithmic: 8 B written and read per hole pair and created orbital pair",
+            "fp64_flops": fp64_flops, "fp64_equivalent_tflops": fp64_flops / seconds / 1e12, "fp64_peak": fp64_peak}
+
+
 def run_gb300(a):
     import torch
 
@@ -277,6 +311,7 @@ def run_gb300(a):
     for _ in range(a.warmup):
         sb.Hamiltonian(C, S)
     torch.cuda.synchronize()
+    launches = count_launches(lambda: sb.Hamiltonian(C, S))
     sb.reset_build_times()
     clocks = Clocks(local)
     clocks.start()
@@ -357,6 +392,26 @@ def run_gb300(a):
         v, sample, cores = cpu_baseline(a.norb, a.cpu_seconds, na, nb, ints, c_host)
         cpu = {"value": v, "unit": "sigma-builds/s", "cores": cores, "kind": "port", "sample": sample}
     if rank == 0:
+        digits = a.norb <= 16 and min(na, nb) >= 2 and ndet > 8192
+        roofline = digit_opposite_roofline(a.norb, na, nb, t_ab, f_sp["ab"], peak64) if digits else {"bound": "compute", "pipe": "fp64", "kernel": "k_opposite (opposite-spin sigma)",
+            "achieved": achieved, "peak": peak64, "unit": "TFLOP/s",
+            "frac": achieved / peak64, "traffic": opposite_traffic(a.norb, na, nb),
+            "traffic_source": "dram read+write per gathered C element of the ncu capture at "
+            "CAS(15e,15o) (profiles/k_opposite_fp64_cas15.md: 5.04 GB for "
+            "2.09e10 elements), times this launch's gathered elements",
+            "peak_source": "FP64 rate 4 FLOP/clk/SM x SMs x median SM clock sampled in this run "
+            "(no FP64 entry in MEASURED_PEAKS.json)",
+            "probe_tflops": fp64_peak, "frac_of_probe": achieved / fp64_peak,
+            "probe_source": "the library's DFMA issue-rate probe (k_probe_dfma, 16 chains per thread, "
+            "best of 3 launches, CUDA events), measured in this run",
+            "fp64_dgemm_tflops": FP64_DGEMM_TFLOPS, "frac_of_dgemm": achieved / FP64_DGEMM_TFLOPS,
+            "flops_per_launch": f_sp["ab"], "launch_ms": 1e3 * t_ab,
+            # the reference's dense HZ product counts n^2 x n^2 blocks whose D rows are
+            # mostly zero; the kernel skips exactly those (same sigma to 1e-12)
+            "dense_hz_flops_per_launch": f_hz["ab"],
+            "dense_hz_equivalent_tflops": f_hz["ab"] / t_ab / 1e12,
+            "algorithmic_bytes": 24 * ndet,
+            "traffic_over_algorithmic": opposite_traffic(a.norb, na, nb) / (24 * ndet)}
         line = {
             "metric": METRIC if a.norb == NORB else f"CAS({a.norb},{a.norb}) sigma-builds/s",
             "value": value, "unit": "sigma-builds/s", "n_gpus": world, "steps": a.steps, "warmup": a.warmup,
@@ -367,26 +422,8 @@ def run_gb300(a):
                        "l2": "inputs larger than L2 (1.32 GB vectors), no flush"},
             "e2e": {"value": e2e, "unit": "sigma-builds/s", "h2d_bytes_per_step": 8 * ndet,
                     "d2h_bytes_per_step": 8 * ndet},
-            "gpu_launches": 5 * a.steps,
-            "roofline": {"bound": "compute", "pipe": "fp64", "kernel": "k_opposite (opposite-spin sigma)",
-                         "achieved": achieved, "peak": peak64, "unit": "TFLOP/s",
-                         "frac": achieved / peak64, "traffic": opposite_traffic(a.norb, na, nb),
-                         "traffic_source": "dram read+write per gathered C element of the ncu capture at "
-                                           "CAS(15e,15o) (profiles/k_opposite_fp64_cas15.md: 5.04 GB for "
-                                           "2.09e10 elements), times this launch's gathered elements",
-                         "peak_source": "FP64 rate 4 FLOP/clk/SM x SMs x median SM clock sampled in this run "
-                                        "(no FP64 entry in MEASURED_PEAKS.json)",
-                         "probe_tflops": fp64_peak, "frac_of_probe": achieved / fp64_peak,
-                         "probe_source": "the library's DFMA issue-rate probe (k_probe_dfma, 16 chains per thread, "
-                                         "best of 3 launches, CUDA events), measured in this run",
-                         "fp64_dgemm_tflops": FP64_DGEMM_TFLOPS, "frac_of_dgemm": achieved / FP64_DGEMM_TFLOPS,
-                         "flops_per_launch": f_sp["ab"], "launch_ms": 1e3 * t_ab,
-                         # the reference's dense HZ product counts n^2 x n^2 blocks whose D rows are
-                         # mostly zero; the kernel skips exactly those (same sigma to 1e-12)
-                         "dense_hz_flops_per_launch": f_hz["ab"],
-                         "dense_hz_equivalent_tflops": f_hz["ab"] / t_ab / 1e12,
-                         "algorithmic_bytes": 24 * ndet,
-                         "traffic_over_algorithmic": opposite_traffic(a.norb, na, nb) / (24 * ndet)},
+            "gpu_launches": launches * a.steps,
+            "roofline": roofline,
             "terms_ms": {"total": 1e3 * tot, "aabb": 1e3 * t_ab, "aaaa_h1a_h0": 1e3 * t_aa, "bbbb_h1b": 1e3 * t_bb},
             "same_spin": same_spin_rates(a.norb, na, nb, ndet, t_aa, t_bb),
             "hz_dense_flops": f_hz, "sparse_flops": f_sp,
@@ -544,7 +581,8 @@ def same_spin_rates(norb, na, nb, ndet, t_aa, t_bb):
     from math import comb
 
     peak = _measured_peaks().get("hbm_gbs") or 6801.7
-    out = {"hbm_peak_gbs": peak, "bound": "fp64 pipe (the products), the passes are HBM"}
+    out = {"hbm_peak_gbs": peak, "bound": "digit products and their 64-bit sums (csrc/oz.cu); tflops counts the "
+                                          "FP64 multiply-adds of the string Hamiltonian"}
     for spin, k, t in (("alpha_h1a_h0", na, t_aa), ("beta_h1b", nb, t_bb)):
         nnz = 1 + k * (norb - k) + comb(k, 2) * comb(norb - k, 2)
         flops = 2 * ndet * (nnz - 1)
@@ -679,7 +717,8 @@ def run_rdm(a):
     e1.record(st)
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1) / a.steps
-    # dominant kernel: the mixed-spin 2-RDM (k_rdm_ab + its mirror), timed alone
+    launches = count_launches(step)
+    # dominant part: the mixed-spin 2-RDM (digits, k_rg_gram, sum of the partial results), timed alone
     ab_ms = []
     for _ in range(3):
         x0, x1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -690,13 +729,20 @@ def run_rdm(a):
         ab_ms.append(x0.elapsed_time(x1))
     fp64_peak = fp64_fma_peak()
     clk = clocks.stop()
-    # algorithmic FP64 work of k_rdm_ab with bra = ket: alpha pair entries with u <= x times all
-    # beta pair entries, one multiply-add each
+    # FP64 multiply-adds of the sparse contraction with bra = ket (alpha pair entries with u <= x times
+    # all beta pair entries), and the FP16 products of k_rg_gram: per alpha hole string and tile pair
+    # 36 digit products of M = 128, N = nt per 16 beta hole strings
     from math import comb
 
     alpha_sym = n * comb(n - 1, na - 1) + n * (n - 1) // 2 * comb(n - 2, na - 1)
     beta_all = comb(n, nb - 1) * (n - nb + 1) ** 2
     ab_flop = 2.0 * alpha_sym * beta_all
+    slots = (n - na + 1) * n
+    tiles = (slots + 127) // 128
+    nt = ((slots + tiles - 1) // tiles + 15) // 16 * 16
+    mma_flop = (comb(n, na - 1) * (tiles * (tiles + 1) // 2) * ((comb(n, nb - 1) + 15) // 16)
+                * 36 * 2 * 128 * nt * 16)
+    bf16 = _measured_peaks().get("bf16_tflops", 1900.0)
     ab_s = statistics.median(ab_ms) / 1e3
     # end to end through the host-array API (numpy in, numpy out)
     t = time.perf_counter()
@@ -712,16 +758,16 @@ def run_rdm(a):
                                   f"(bra = ket), {ndet} determinants, vector {ndet * 8 / 2**30:.2f} GiB > L2"},
            "e2e": {"value": 1.0 / e2e_s, "unit": "RDM sets/s", "h2d_bytes_per_step": 2 * ndet * 8,
                    "d2h_bytes_per_step": (n * n + n ** 4) * 8},
-           "roofline": {"bound": "compute", "pipe": "fp64", "kernel": "k_rdm_ab (mixed-spin 2-RDM, with its mirror)",
-                        "achieved": ab_flop / ab_s / 1e12,
-                        "peak": fp64_nominal_peak(clk.get("sm_mhz")), "unit": "TFLOP/s",
-                        "frac": ab_flop / ab_s / 1e12 / fp64_nominal_peak(clk.get("sm_mhz")),
-                        "flop_per_launch": ab_flop, "ms": ab_s * 1e3, "traffic": None,
-                        "peak_source": "FP64 rate 4 FLOP/clk/SM x SMs x median SM clock sampled in this run",
-                        "probe_tflops": fp64_peak, "fp64_dgemm_tflops": FP64_DGEMM_TFLOPS},
+           "roofline": {"bound": "tensor", "kernel": "k_rg_gram (mixed-spin 2-RDM in FP16 digits) and its operands",
+                        "achieved": mma_flop / ab_s / 1e12, "peak": bf16, "unit": "TFLOP/s",
+                        "frac": mma_flop / ab_s / 1e12 / bf16, "flop_per_launch": mma_flop, "ms": ab_s * 1e3,
+                        "traffic": None,
+                        "peak_source": "MEASURED_PEAKS.json bf16_tflops (dense FP16 runs at the BF16 rate)",
+                        "fp64_flops": ab_flop, "fp64_equivalent_tflops": ab_flop / ab_s / 1e12,
+                        "fp64_peak": fp64_nominal_peak(clk.get("sm_mhz")), "probe_tflops": fp64_peak,
+                        "fp64_dgemm_tflops": FP64_DGEMM_TFLOPS},
            "clocks": clk,
-           # per set: k_rdm_hole<1> x2, k_transpose x2, k_rdm_ab, its mirror, k_rdm_hole<2> x2, k_rdm_sf2
-           "gpu_launches": 9 * a.steps}
+           "gpu_launches": launches * a.steps}
     # three-body RDMs (make_sf_3rdm / make_sf_3cumulant) at CAS(14e,14o): one warm call, one timed
     n3 = min(n, 14)
     na3, nb3, _, _, ndet3 = cas_dims(n3, n3, 0)

@@ -482,7 +482,7 @@ std::shared_ptr<SymDigits> sym_digits_build(const CIStrings* s, const OppositeSy
     while (nir < t.os.nirrep || nir <= t.os.S)
         nir *= 2;
     const int64_t N1a = s->a.N1, N1b = s->b.N1, N0a = s->a.N0, N0b = s->b.N0;
-    if (N1a == 0 || N1b == 0 || s->a.m1 > 32 || s->na > 32 || nir > 8)
+    if (N1a == 0 || N1b == 0 || s->a.m1 > 32 || s->na > 32 || nir > 8 || N0a * n * 16 * 128 > kYBytes)
         return nullptr;
     auto d = std::make_shared<SymDigits>();
     d->os = t.os;
@@ -537,7 +537,7 @@ std::shared_ptr<SymDigits> sym_digits_build(const CIStrings* s, const OppositeSy
     // positions at a time: the vector's digits within kYBytes; then hole strings Ka at a time: E within kYBytesE
     d->most = (most + 3) / 4 * 4; // stored four at a time
     const int64_t most128 = kYBytes / (N0a * n * 16 * 128), all128 = d->lmax / 128;
-    if (most128 < 1 || N1a * nir * (int64_t)d->slots * d->slots * 16 > kYBytes)
+    if (N1a * nir * (int64_t)d->slots * d->slots * 16 > kYBytes)
         return nullptr;
     const int64_t parts = (all128 + most128 - 1) / most128;
     d->chunk = (int)((all128 + parts - 1) / parts * 128);
