@@ -393,25 +393,30 @@ def run_gb300(a):
         cpu = {"value": v, "unit": "sigma-builds/s", "cores": cores, "kind": "port", "sample": sample}
     if rank == 0:
         digits = a.norb <= 16 and min(na, nb) >= 2 and ndet > 8192
-        roofline = digit_opposite_roofline(a.norb, na, nb, t_ab, f_sp["ab"], peak64) if digits else {"bound": "compute", "pipe": "fp64", "kernel": "k_opposite (opposite-spin sigma)",
-            "achieved": achieved, "peak": peak64, "unit": "TFLOP/s",
-            "frac": achieved / peak64, "traffic": opposite_traffic(a.norb, na, nb),
-            "traffic_source": "dram read+write per gathered C element of the ncu capture at "
-            "CAS(15e,15o) (profiles/k_opposite_fp64_cas15.md: 5.04 GB for "
-            "2.09e10 elements), times this launch's gathered elements",
-            "peak_source": "FP64 rate 4 FLOP/clk/SM x SMs x median SM clock sampled in this run "
-            "(no FP64 entry in MEASURED_PEAKS.json)",
-            "probe_tflops": fp64_peak, "frac_of_probe": achieved / fp64_peak,
-            "probe_source": "the library's DFMA issue-rate probe (k_probe_dfma, 16 chains per thread, "
-            "best of 3 launches, CUDA events), measured in this run",
-            "fp64_dgemm_tflops": FP64_DGEMM_TFLOPS, "frac_of_dgemm": achieved / FP64_DGEMM_TFLOPS,
-            "flops_per_launch": f_sp["ab"], "launch_ms": 1e3 * t_ab,
-            # the reference's dense HZ product counts n^2 x n^2 blocks whose D rows are
-            # mostly zero; the kernel skips exactly those (same sigma to 1e-12)
-            "dense_hz_flops_per_launch": f_hz["ab"],
-            "dense_hz_equivalent_tflops": f_hz["ab"] / t_ab / 1e12,
-            "algorithmic_bytes": 24 * ndet,
-            "traffic_over_algorithmic": opposite_traffic(a.norb, na, nb) / (24 * ndet)}
+        if digits:
+            roofline = digit_opposite_roofline(a.norb, na, nb, t_ab, f_sp["ab"], peak64)
+        else:
+            roofline = {
+                "bound": "compute", "pipe": "fp64", "kernel": "k_opposite (opposite-spin sigma)",
+                "achieved": achieved, "peak": peak64, "unit": "TFLOP/s",
+                "frac": achieved / peak64, "traffic": opposite_traffic(a.norb, na, nb),
+                "traffic_source": "dram read+write per gathered C element of the ncu capture at "
+                  "CAS(15e,15o) (profiles/k_opposite_fp64_cas15.md: 5.04 GB for "
+                  "2.09e10 elements), times this launch's gathered elements",
+                "peak_source": "FP64 rate 4 FLOP/clk/SM x SMs x median SM clock sampled in this run "
+                  "(no FP64 entry in MEASURED_PEAKS.json)",
+                "probe_tflops": fp64_peak, "frac_of_probe": achieved / fp64_peak,
+                "probe_source": "the library's DFMA issue-rate probe (k_probe_dfma, 16 chains per thread, "
+                  "best of 3 launches, CUDA events), measured in this run",
+                "fp64_dgemm_tflops": FP64_DGEMM_TFLOPS, "frac_of_dgemm": achieved / FP64_DGEMM_TFLOPS,
+                "flops_per_launch": f_sp["ab"], "launch_ms": 1e3 * t_ab,
+                # the reference's dense HZ product counts n^2 x n^2 blocks whose D rows are
+                # mostly zero; the kernel skips exactly those (same sigma to 1e-12)
+                "dense_hz_flops_per_launch": f_hz["ab"],
+                "dense_hz_equivalent_tflops": f_hz["ab"] / t_ab / 1e12,
+                "algorithmic_bytes": 24 * ndet,
+                "traffic_over_algorithmic": opposite_traffic(a.norb, na, nb) / (24 * ndet),
+            }
         line = {
             "metric": METRIC if a.norb == NORB else f"CAS({a.norb},{a.norb}) sigma-builds/s",
             "value": value, "unit": "sigma-builds/s", "n_gpus": world, "steps": a.steps, "warmup": a.warmup,
