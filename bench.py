@@ -397,7 +397,8 @@ def run_gb300(a):
             roofline = digit_opposite_roofline(a.norb, na, nb, t_ab, f_sp["ab"], peak64)
         else:
             roofline = {
-                "bound": "compute", "pipe": "fp64", "kernel": "k_opposite (opposite-spin sigma)",
+                "bound": "compute", "pipe": "fp64",
+                "kernel": "k_opposite (opposite-spin sigma)" if a.norb > 16 or ndet > 8192 else "k_small_sigma (all terms)",
                 "achieved": achieved, "peak": peak64, "unit": "TFLOP/s",
                 "frac": achieved / peak64, "traffic": opposite_traffic(a.norb, na, nb),
                 "traffic_source": "dram read+write per gathered C element of the ncu capture at "
