@@ -352,14 +352,24 @@ __global__ void k_transpose(int64_t rows, int64_t cols, const T* __restrict__ in
     }
 }
 
-// One block of a blocked space's vectors transposed: in (rows x cols, vector z at z * ldv) to
-// out (cols x rows, vector z at z * ldv_out), overwritten
-__global__ void k_transpose_blk(int64_t rows, int64_t cols, const double* __restrict__ in, int64_t ldv,
+// The blocks of a space blocked by irreps, rows[b] x cols[b] at off[b] of in, transposed into out at the same places, in
+// one launch (one per block: 16 launches, 43 us at CAS(14,14) in 8 irreps, two 17 us, and most of the host's time for
+// a small space: (8 orbitals, 4, 4) 222 -> 81 us per sigma together with k_spmm_blocks); vectors ldv, ldv_out apart
+constexpr int kIrrepBlocks = 8; // blocks of a space blocked by irreps alone at most
+struct TransposeBlocks {
+    int n;
+    int64_t tile0[kIrrepBlocks + 1], off[kIrrepBlocks], rows[kIrrepBlocks], cols[kIrrepBlocks];
+};
+__global__ void k_transpose_blk(const __grid_constant__ TransposeBlocks B, const double* __restrict__ in, int64_t ldv,
                                 double* __restrict__ out, int64_t ldv_out) {
     __shared__ double tile[32][33];
-    in += blockIdx.z * ldv;
-    out += blockIdx.z * ldv_out;
-    const int64_t bx = (int64_t)blockIdx.x * 32, by = (int64_t)blockIdx.y * 32;
+    int b = 0;
+    while (b + 1 < B.n && (int64_t)blockIdx.x >= B.tile0[b + 1])
+        ++b;
+    const int64_t rows = B.rows[b], cols = B.cols[b], tc = (cols + 31) / 32, t = (int64_t)blockIdx.x - B.tile0[b];
+    in += blockIdx.z * ldv + B.off[b];
+    out += blockIdx.z * ldv_out + B.off[b];
+    const int64_t bx = t % tc * 32, by = t / tc * 32;
     for (int j = threadIdx.y; j < 32; j += blockDim.y) {
         const int64_t r = by + j, c = bx + threadIdx.x;
         if (r < rows && c < cols)
@@ -1284,18 +1294,88 @@ void SigmaBuilder::run(const T* C, T* sig, cudaStream_t st, int mask, bool timed
         F2G_CUDA(cudaEventRecord(cur_ev[3], st));
 }
 
-// Row SpMM on raw operands: Y[J] (+)= sum_k val[J][k] X[col[J][k]] for J < nrows, vectors at z * vstride.
-static void spmm_rows_raw(int64_t nrows, int ncols, int nnz, const int32_t* col, const double* val, const double* X,
-                          double* Y, bool accumulate, int64_t vstride, int nvec, cudaStream_t st) {
-    if (nrows == 0 || ncols == 0 || nnz == 0 || nvec <= 0)
-        return;
+// Row SpMM of the blocks of an irrep-blocked space in one launch: Y_b[J] (+)= sum_k val_b[J][k] X_b[col_b[J][k]] for the
+// rows J of every block b, block vectors at off_b, vectors of a batch vstride apart. Sums in the order of k_spmm_rows.
+// A block's launch alone is 429 thread blocks at CAS(14,14) in 8 irreps, less than three for each SM: 16 launches
+// 818 us, two 721 us (the FP64 pipe's multiply-adds 380 us).
+struct SpmmBlocks {
+    int n;
+    int64_t row0[kIrrepBlocks + 1]; // first row of every block among all rows
+    int64_t off[kIrrepBlocks];
+    int ncols[kIrrepBlocks];
+    const int32_t* col[kIrrepBlocks];
+    const double* val[kIrrepBlocks];
+};
+__global__ void __launch_bounds__(128) k_spmm_blocks(const __grid_constant__ SpmmBlocks B, int nnz, const double* X,
+                                                     double* Y, int accumulate, int64_t vstride) {
     constexpr int VEC = 4;
+    extern __shared__ unsigned char smem_raw[];
+    double* sval = reinterpret_cast<double*>(smem_raw);
+    int32_t* scol = reinterpret_cast<int32_t*>(sval + nnz);
+    int b = 0;
+    while (b + 1 < B.n && (int64_t)blockIdx.x >= B.row0[b + 1])
+        ++b;
+    const int64_t J = (int64_t)blockIdx.x - B.row0[b];
+    const int ncols = B.ncols[b];
+    if ((int)(blockIdx.y * 128 * VEC) >= ncols)
+        return;
+    X += blockIdx.z * vstride + B.off[b];
+    Y += blockIdx.z * vstride + B.off[b] + J * ncols;
+    for (int i = threadIdx.x; i < nnz; i += 128) {
+        sval[i] = B.val[b][J * nnz + i];
+        scol[i] = B.col[b][J * nnz + i];
+    }
+    __syncthreads();
+    const int c0 = blockIdx.y * (128 * VEC) + threadIdx.x;
+    double acc[VEC] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+    for (int i = 0; i < nnz; ++i) {
+        const double v = sval[i];
+        const double* x = X + (int64_t)scol[i] * ncols;
+#pragma unroll
+        for (int j = 0; j < VEC; ++j)
+            if (c0 + j * 128 < ncols)
+                acc[j] += v * __ldg(x + c0 + j * 128);
+    }
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) {
+        const int c = c0 + j * 128;
+        if (c < ncols)
+            Y[c] = accumulate ? Y[c] + acc[j] : acc[j];
+    }
+}
+// spin 0: rows are the blocks' alpha strings, spin 1: their beta strings (operands transposed block by block)
+void SigmaBuilder::spmm_blocks(int spin, const double* X, double* Y, bool accumulate, int nvec, cudaStream_t st) {
+    const DetBlocks& B = s->blocks;
+    const int nnz = spin == 0 ? ha.nnz : hb.nnz;
+    if (nnz == 0 || nvec <= 0)
+        return;
     const size_t smem = (size_t)nnz * (sizeof(double) + sizeof(int32_t));
     if (smem > 48 * 1024)
-        F2G_CUDA(cudaFuncSetAttribute(k_spmm_rows<double, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dim3 grid((unsigned)nrows, (unsigned)ceil_div(ncols, 128 * VEC), (unsigned)nvec);
-    k_spmm_rows<double, VEC><<<grid, 128, smem, st>>>(nrows, ncols, nnz, col, val, X, Y, accumulate ? 1 : 0, vstride);
-    F2G_LAUNCH("k_spmm_rows block");
+        F2G_CUDA(cudaFuncSetAttribute(k_spmm_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    for (int b = 0; b < B.nblk();) {
+        SpmmBlocks a{};
+        int most = 0;
+        for (; b < B.nblk() && a.n < kIrrepBlocks; ++b) {
+            const int64_t* r = B.hblk.data() + 6 * b;
+            const int64_t rows = r[4 + spin], ncols = r[5 - spin];
+            if (r[2] == 0 || rows == 0 || ncols == 0)
+                continue;
+            const int64_t first = B.cls_off[spin][(int)r[spin]] * nnz;
+            a.row0[a.n + 1] = a.row0[a.n] + rows;
+            a.off[a.n] = r[3];
+            a.ncols[a.n] = (int)ncols;
+            a.col[a.n] = lcol[spin].get() + first;
+            a.val[a.n] = lval[spin].get() + first;
+            most = std::max(most, (int)ncols);
+            ++a.n;
+        }
+        if (a.n == 0)
+            continue;
+        k_spmm_blocks<<<dim3((unsigned)a.row0[a.n], (unsigned)ceil_div(most, 512), (unsigned)nvec), 128, smem, st>>>(
+            a, nnz, X, Y, accumulate ? 1 : 0, s->ndet);
+        F2G_LAUNCH("k_spmm_blocks");
+    }
 }
 
 // the opposite-spin term of a space blocked by irreps, on the tensor cores or the FP64 pipe
@@ -1318,34 +1398,33 @@ void SigmaBuilder::run_blocked_sym(const double* C, double* S, cudaStream_t st, 
     double* xs = graph ? gxS.get() : xS.reserve((size_t)nvec * nf);
     if (timed)
         F2G_CUDA(cudaEventRecord(cur_ev[0], st));
-    // beta same spin: per block transpose (Ia x Ib -> Ib x Ia), beta SpMM, transpose back (overwrites S)
-    for (int b = 0; b < B.nblk(); ++b) {
-        const int64_t* r = B.hblk.data() + 6 * b;
-        const int64_t off = r[3], nIa = r[4], nIb = r[5];
-        if (r[2] == 0)
-            continue;
-        const int cb = (int)r[1];
-        k_transpose_blk<<<dim3((unsigned)ceil_div(nIb, 32), (unsigned)ceil_div(nIa, 32), (unsigned)nvec), dim3(32, 8), 0,
-                          st>>>(nIa, nIb, C + off, nd, xc + off, nd);
-        F2G_LAUNCH("k_transpose_blk");
-        spmm_rows_raw(nIb, (int)nIa, hb.nnz, lcol[1].get() + B.cls_off[1][cb] * hb.nnz,
-                      lval[1].get() + B.cls_off[1][cb] * hb.nnz, xc + off, xs + off, false, nd, nvec, st);
-        k_transpose_blk<<<dim3((unsigned)ceil_div(nIa, 32), (unsigned)ceil_div(nIb, 32), (unsigned)nvec), dim3(32, 8), 0,
-                          st>>>(nIb, nIa, xs + off, nd, S + off, nd);
-        F2G_LAUNCH("k_transpose_blk");
-    }
+    // beta same spin: blocks transposed (Ia x Ib -> Ib x Ia), beta SpMM, transposed back (overwrites S)
+    auto transposes = [&](const double* in, double* out, bool back) {
+        for (int b = 0; b < B.nblk();) {
+            TransposeBlocks t{};
+            for (; b < B.nblk() && t.n < kIrrepBlocks; ++b) {
+                const int64_t* r = B.hblk.data() + 6 * b;
+                if (r[2] == 0)
+                    continue;
+                t.off[t.n] = r[3];
+                t.rows[t.n] = back ? r[5] : r[4];
+                t.cols[t.n] = back ? r[4] : r[5];
+                t.tile0[t.n + 1] = t.tile0[t.n] + ((t.rows[t.n] + 31) / 32) * ((t.cols[t.n] + 31) / 32);
+                ++t.n;
+            }
+            if (t.n == 0)
+                continue;
+            k_transpose_blk<<<dim3((unsigned)t.tile0[t.n], 1, (unsigned)nvec), dim3(32, 8), 0, st>>>(t, in, nd, out, nd);
+            F2G_LAUNCH("k_transpose_blk");
+        }
+    };
+    transposes(C, xc, false);
+    spmm_blocks(1, xc, xs, false, nvec, st);
+    transposes(xs, S, true);
     if (timed)
         F2G_CUDA(cudaEventRecord(cur_ev[1], st));
     // alpha same spin + H0, accumulated
-    for (int b = 0; b < B.nblk(); ++b) {
-        const int64_t* r = B.hblk.data() + 6 * b;
-        const int64_t off = r[3], nIa = r[4], nIb = r[5];
-        if (r[2] == 0)
-            continue;
-        const int ca = (int)r[0];
-        spmm_rows_raw(nIa, (int)nIb, ha.nnz, lcol[0].get() + B.cls_off[0][ca] * ha.nnz,
-                      lval[0].get() + B.cls_off[0][ca] * ha.nnz, C + off, S + off, true, nd, nvec, st);
-    }
+    spmm_blocks(0, C, S, true, nvec, st);
     if (timed)
         F2G_CUDA(cudaEventRecord(cur_ev[2], st));
     // opposite spin on the embedding, added into S

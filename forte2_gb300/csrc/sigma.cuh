@@ -62,6 +62,7 @@ struct SigmaBuilder {
     bool use_sym = true;
     std::shared_ptr<struct OppositeSym> osym; // set when the space allows it
     std::shared_ptr<struct SymDigits> symd;   // osym on the tensor cores, set where that is faster
+    void spmm_blocks(int spin, const double* X, double* Y, bool accumulate, int nvec, cudaStream_t st);
     void opposite_sym(const double* V, const double* C, double* sig, cudaStream_t st, int nvec, int ctas, bool graph);
     // such a space's same-spin terms on its own vectors: class-local string Hamiltonians (rows in
     // the space's string order, columns as positions inside the class), rebuilt with the integrals

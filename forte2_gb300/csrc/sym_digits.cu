@@ -512,7 +512,8 @@ std::shared_ptr<SymDigits> sym_digits_build(const CIStrings* s, const OppositeSy
         }
     }
     // Below some 2e7 products the FP64 kernel's one launch is the faster one: (10 orbitals, 5, 5) in 8, 4 and 2 irreps
-    // (5e6, 1.4e7 and 4e7) sigma 292, 246, 295 us, here 327, 259, 212 us; (12, 6, 6) in 8 (1.2e8) 829 and 546 us
+    // (5e6, 1.4e7 and 4e7) sigma 292, 246, 295 us, here 327, 259, 212 us, (12, 6, 6) in 8 (1.2e8) 829 and 546 us, all
+    // with one launch per block of the same-spin terms (now 113, 148, 167 and 331 us by this line)
     if (most > kSymSlots || (double)N1a * (double)N1b * most * most < 2e7)
         return nullptr;
     d->slots = (most + 15) / 16 * 16;
