@@ -634,9 +634,10 @@ SigmaBuilder::SigmaBuilder(CIStrings* s_, double E_, const double* H_, const dou
     set_hamiltonian(E_, H_, V_);
 }
 
-// The digit operands of the FP64 tensor-core sigma for the current integrals, in stream order
+// The digit operands of the FP64 tensor-core sigma for the current integrals, in stream order. Built before: refilled
+// in place also while the variant is off, so that it can be turned on again and captured graphs follow.
 void SigmaBuilder::build_oz(cudaStream_t st) {
-    if (oz_fast && use_oz)
+    if (oz || (oz_fast && use_oz))
         oz_build(s, oz, dH.get(), dV.get(), E, st);
 }
 
