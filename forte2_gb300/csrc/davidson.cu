@@ -364,13 +364,13 @@ __device__ void eig_block(EigShared<MAXM>& z, int m, const double* G, int ldg, d
     if (!(off <= 1.8e-15 * amax))
         jacobi_sweeps<double, MAXM, false>(z, z.S, z.X, m, 1e-16 * amax, 60, t, nt);
     __syncthreads();
-    // ascending order by rank (ties by index), then gather
+    // ascending order by rank (ties by index, NaN last: always a permutation), then gather
     for (int i = t; i < m; i += nt) {
         const double w = z.S[i][i];
         int r = 0;
         for (int j = 0; j < m; ++j) {
             const double x = z.S[j][j];
-            r += (x < w) || (x == w && j < i);
+            r += x < w || (w != w && x == x) || ((x == w || (x != x && w != w)) && j < i);
         }
         z.order[r] = i;
     }
