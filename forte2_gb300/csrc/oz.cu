@@ -80,6 +80,7 @@ struct OzShared {
     uint64_t b_full[kOzMaxRing], b_empty[kOzMaxRing], drain;
     uint32_t tmem_base;
     volatile int abort;
+    volatile uint32_t loaded[3]; // opposite spin: K steps each loading warp has copied
 };
 
 // D[tmem] (+)= A[tmem] B[smem], kind::f16, D F32, A and B F16, K-major, M = 128, issued by the lane with
@@ -677,6 +678,21 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz(const __grid_constant__ Oz
         }
         if (!ok)
             give_up();
+        if (!SS) {
+            // A slot's barrier completes with the copies of all three warps. After an abort one may have stopped
+            // before the others: it arrives in the steps that they have copied and it has not (a step is copied
+            // once its slot's last use is complete, so every arrival counts for its own step), or the waits below
+            // would not end.
+            if (el)
+                sh.loaded[pl] = total;
+            __syncwarp();
+            asm volatile("bar.sync 1, 96;" ::: "memory");
+            const uint32_t most = max(sh.loaded[0], max(sh.loaded[1], sh.loaded[2]));
+            for (; total < most; ++total)
+                if (el)
+                    mbar_arrive(smem_u32(&sh.b_full[total % a.nbuf]));
+            __syncwarp();
+        }
         // the copies in flight end before the block leaves: the last of every slot
 #pragma unroll 1
         for (uint32_t i = 0; i < (uint32_t)a.nbuf && i < total; ++i) {
