@@ -59,6 +59,7 @@ def _declare(L):
         "f2g_sigma_set_variant": (i32, [vp, i32, i32]),
         "f2g_sigma_reset_build_times": (i32, [vp]),
         "f2g_sigma_tc_error": (i32, [vp, P]),
+        "f2g_sigma_check": (i32, [vp]),
         "f2g_sigma_apply": (i32, [vp, P, P, i32, vp]),
         "f2g_sigma_apply_host": (i32, [vp, P, P, i32]),
         "f2g_sigma_term": (i32, [vp, i32, P, P, vp]),

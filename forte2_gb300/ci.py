@@ -244,6 +244,7 @@ class CASCISolver:
             self.evals, evecs = yield from self.eigensolver.solve_steps()
             self.converged = self.eigensolver.converged
             self.phases.append(("fp64", self.eigensolver.iter + 1, self.eigensolver.sigma_builds, list(self.evals)))
+        self.sigma_builder.check()  # no wait of the last iterations gave up
         self.timings["davidson"] = time.perf_counter() - t0
         self.evecs = evecs
         if not self.converged and self.die_if_not_converged:

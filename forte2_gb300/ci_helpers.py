@@ -575,6 +575,13 @@ class CISigmaBuilder:
         check(lib().f2g_sigma_tc_error(self.h, out.ctypes.data))
         return int(out[0])
 
+    def check(self):
+        """RuntimeError if a tensor-core kernel gave up a bounded wait in work that the host has
+        waited for since the last check (no synchronisation). Calls that return host results do it
+        themselves, and so does the next call on this builder; device results of such a call are
+        NaN in FP64. No counterpart in the reference."""
+        check(lib().f2g_sigma_check(self.h))
+
     def set_max_blocks(self, n):
         """Cap the opposite-spin kernel at n thread blocks (one per SM; 0 = no cap), leaving the
         other SMs to concurrent solves. Same sigma. No counterpart in the reference."""
@@ -658,7 +665,11 @@ class CISigmaBuilder:
         out = torch.empty(max(size, 1), dtype=torch.float64, device="cuda")
         check(lib().f2g_sigma_rdm(self.h, k, L.data_ptr(), R.data_ptr(), out.data_ptr(), stream_handle()))
         res = out[:size].view(shape)
-        return res if device else res.cpu().numpy()
+        if device:
+            return res
+        res = res.cpu().numpy()
+        self.check()
+        return res
 
     def a_1rdm(self, C_left, C_right):
         """gamma[p][q] = <L| a+_p a_q |R>, alpha (ci_sigma_builder_1rdm.cc:9-65)."""

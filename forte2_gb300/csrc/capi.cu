@@ -487,12 +487,12 @@ int f2g_sigma_set_variant(void* sb, int which, int value) {
         else if (which == 2)
             b->opposite_persistent = value != 0;
         else if (which == 3) {
-            // polls per bounded wait of the tensor-core kernel (0 = the default limit); also clears
-            // its error flag. A small limit makes the waits give up: the error path, for tests.
+            // polls per bounded wait of the tensor-core kernels (0 = the default limit); also clears
+            // their error flag. A small limit makes the waits give up: the error path, for tests.
             if (value < 0)
                 throw Error(2, "tensor-core wait limit must be >= 0");
             b->tc_poll_limit = value;
-            F2G_CUDA(cudaMemset(b->tc_err.get(), 0, sizeof(int)));
+            b->clear_waits();
         } else if (which == 4)
             b->use_sym = value != 0;
         else if (which == 5) {
@@ -591,7 +591,15 @@ int f2g_sigma_apply_host(void* sb, const double* C, double* sigma, int nvec) {
             F2G_CUDA(cudaMemcpy(dc, C + v * nd, nd * 8, cudaMemcpyHostToDevice));
             b->hamiltonian(dc, ds, 0);
             F2G_CUDA(cudaMemcpy(sigma + v * nd, ds, nd * 8, cudaMemcpyDeviceToHost));
+            b->check_waits();
         }
+    });
+}
+
+int f2g_sigma_check(void* sb) {
+    return guard([&] {
+        need(sb, "sigma");
+        static_cast<SigmaBuilder*>(sb)->check_waits();
     });
 }
 
@@ -635,6 +643,7 @@ int64_t f2g_rdm_size(int norb, int kind) {
 int f2g_sigma_rdm(void* sb, int kind, const double* CL, const double* CR, double* out, void* stream) {
     return guard([&] {
         need(sb, "sigma");
+        static_cast<SigmaBuilder*>(sb)->check_waits();
         compute_rdm(*static_cast<SigmaBuilder*>(sb), kind, CL, CR, out, S(stream));
     });
 }
@@ -694,6 +703,7 @@ int f2g_sigma_apply_csf(void* sb, void* sa, const double* csf_in, double* csf_ou
             need(csf_in, "csf_in");
             need(csf_out, "csf_out");
         }
+        static_cast<SigmaBuilder*>(sb)->check_waits();
         if (!a->host_scratch)
             a->host_scratch = std::make_unique<CsfSigmaScratch>();
         sigma_csf(*static_cast<SigmaBuilder*>(sb), *a, csf_in, csf_out, nvec, S(stream), *a->host_scratch, false);
@@ -971,6 +981,7 @@ int f2g_dgraph_state(void* g, int32_t* host_ints, double* host_dbl) {
         need(g, "dgraph");
         need(host_ints, "ints");
         need(host_dbl, "doubles");
+        static_cast<DavGraph*>(g)->sb->check_waits();
         const DGState& s = *static_cast<DavGraph*>(g)->host_state;
         const int32_t iv[8] = {s.m, s.sigma_size, s.iter, s.status, s.collapse, s.added, s.m_eig, 0};
         std::memcpy(host_ints, iv, sizeof(iv));

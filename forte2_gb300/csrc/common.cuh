@@ -121,6 +121,31 @@ inline uint64_t host_binom(int n, int k) {
 
 inline int ceil_div(long long a, long long b) { return int((a + b - 1) / b); }
 
+// Bounded waits of the tensor-core kernels. One that gives up sets `err` on the device. The kernels that sum what was
+// left incomplete then write NaN and set `host`, a word of page-locked host memory, so that the host knows after its
+// next synchronisation without a copy. polls: tries per wait, 0 for the default limit; the kernels of digit_mma.cuh
+// take any other limit as "the first wait for operands gives up", so that a test can run what follows (counting tries
+// in every wait cost them 2 to 3 % in k_oz).
+struct WaitCtl {
+    int* err = nullptr;
+    int* host = nullptr;
+    int polls = 0;
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ void tell_host(const WaitCtl& w) {
+    *reinterpret_cast<volatile int*>(w.host) = 1;
+    __threadfence_system();
+}
+// a result of the kernels that follow: x, or NaN once a wait has given up
+__device__ __forceinline__ double waited(double x, const WaitCtl& w) {
+    if (*w.err) {
+        tell_host(w);
+        x = __longlong_as_double(0x7ff8000000000000ll);
+    }
+    return x;
+}
+#endif
+
 } // namespace f2g
 
 namespace f2g {

@@ -6,6 +6,8 @@
 
 #include <cstdint>
 
+#include "common.cuh"
+
 namespace f2g {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {

@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                   const uint32_t* __restrict__ up_a, const uint64_t* __restrict__ str_b,
                   const uint32_t* __restrict__ exc_b, const float* __restrict__ V,
                   const unsigned int* __restrict__ vmax, const unsigned int* __restrict__ cmax,
-                  const float* __restrict__ C, float* __restrict__ sig, int* __restrict__ err,
+                  const float* __restrict__ C, float* __restrict__ sig, const WaitCtl wait,
                   long long poll_limit, const __grid_constant__ CUtensorMap bmap, int tma_b) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     TcShared& sh = *reinterpret_cast<TcShared*>(smem_raw);
@@ -364,7 +364,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const uint32_t tmem = sh.tmem_base;
 
     auto give_up = [&]() {
-        atomicExch(err, 1);
+        atomicExch(wait.err, 1);
+        tell_host(wait);
         sh.abort = 1;
     };
 
@@ -667,7 +668,7 @@ void opposite_tc_vmax(const float* V, int64_t count, unsigned int* vmax, cudaStr
 // per-vector largest |C|, written here before the kernel runs.
 // tb: the prebuilt B operands (TMA-fed B tiles), or nullptr (each CTA builds B itself; same sigma).
 void launch_opposite_tc(const CIStrings* s, const uint32_t* exc, const float* V, const unsigned int* vmax,
-                        const float* C, float* sig, unsigned int* cmax, int* err, long long poll_limit, int max_ctas,
+                        const float* C, float* sig, unsigned int* cmax, const WaitCtl& wait, int max_ctas,
                         cudaStream_t st, int nvec, const TcBOperands* tb) {
     const int64_t nd = s->a.N0 * s->b.N0;
     F2G_CUDA(cudaMemsetAsync(cmax, 0, (size_t)nvec * sizeof(unsigned int), st));
@@ -683,7 +684,7 @@ void launch_opposite_tc(const CIStrings* s, const uint32_t* exc, const float* V,
         gx = std::min<int64_t>(gx, max_ctas);
     k_opposite_tc<<<dim3((unsigned)gx, (unsigned)nvec), kTcThreads, smem, st>>>(
         s->norb, s->na, s->nb, s->a.m1, s->a.N0, (int)s->b.N0, s->a.down1.get(), s->a.up1.get(), s->b.str.get(), exc,
-        V, vmax, cmax, C, sig, err, poll_limit > 0 ? poll_limit : (1ll << 26), tb ? tb->map : CUtensorMap{},
+        V, vmax, cmax, C, sig, wait, wait.polls > 0 ? wait.polls : (1ll << 26), tb ? tb->map : CUtensorMap{},
         tb ? 1 : 0);
     F2G_LAUNCH("k_opposite_tc");
 }

@@ -174,7 +174,7 @@ struct OzArgs {
     int tsplit;           // tile ranges per hole string
     int reuse;            // the digits' integers of a tile stay in shared memory for all chunks
     int nbuf;             // B ring: K steps held
-    int* err;
+    WaitCtl wait;
 };
 
 // Work item: a hole string, a range of tiles and (without reuse) one chunk
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz(const __grid_constant__ Oz
     constexpr uint32_t tmem = 0;
     constexpr uint32_t acc0 = tmem, stage0 = tmem + kOzS * kOzN;
     auto give_up = [&]() {
-        atomicExch(a.err, 1);
+        atomicExch(a.wait.err, 1);
         sh.abort = 1;
     };
 
@@ -576,7 +576,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz(const __grid_constant__ Oz
         const uint32_t el = elect_lane();
         const uint32_t lbo = 128, sbo = 256;
         uint32_t slot = 0, suse = 0, ntile = 0, bslot = 0, buse = 0;
-        bool ok = true;
+        bool ok = a.wait.polls == 0; // with a limit on the tries (for tests) the first wait counts as given up
 #pragma unroll 1
         for (uint32_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
             const OzItem it = oz_item<SS>(a, w);
@@ -808,12 +808,13 @@ __global__ void __launch_bounds__(256) k_oz_sum_a(const long long* __restrict__ 
                                                   int64_t nx, int m2, const uint32_t* __restrict__ down,
                                                   const uint16_t* __restrict__ dpair, const int* __restrict__ bexp,
                                                   int np, int tpv, int64_t ncol, int64_t t0, int64_t nd,
-                                                  double* __restrict__ S) {
+                                                  double* __restrict__ S, const WaitCtl wait) {
     const int64_t x = blockIdx.y * (int64_t)blockDim.x + threadIdx.x, J = blockIdx.x;
     const int64_t tg = t0 + x / kOzM, v = tg / tpv, c = (tg - v * tpv) * kOzM + x % kOzM;
     if (x >= nx || c >= ncol)
         return;
-    S[v * nd + J * ncol + c] += oz_pairs_sum(E, rexp, nx, m2, down, dpair, bexp, np, J, x);
+    const double sum = oz_pairs_sum(E, rexp, nx, m2, down, dpair, bexp, np, J, x);
+    S[v * nd + J * ncol + c] += waited(sum, wait);
 }
 
 // beta: the chunk's columns are alpha strings; 32 x 32 tiles turned in shared memory
@@ -821,7 +822,7 @@ __global__ void __launch_bounds__(256) k_oz_sum_b(const long long* __restrict__ 
                                                   int64_t nx, int m2, const uint32_t* __restrict__ down,
                                                   const uint16_t* __restrict__ dpair, const int* __restrict__ bexp,
                                                   int np, int64_t N0b, int tpv, int64_t ncol, int64_t t0, int64_t nd,
-                                                  double* __restrict__ S) {
+                                                  double* __restrict__ S, const WaitCtl wait) {
     __shared__ double tile[32][33];
     const int64_t x0 = blockIdx.y * 32, j0 = blockIdx.x * (int64_t)32;
     const int64_t tg = t0 + x0 / kOzM, v = tg / tpv, c0 = (tg - v * tpv) * kOzM + x0 % kOzM;
@@ -836,7 +837,7 @@ __global__ void __launch_bounds__(256) k_oz_sum_b(const long long* __restrict__ 
     __syncthreads();
     for (int j = ty; j < 32; j += 8)
         if (c0 + j < ncol && j0 + tx < N0b)
-            S[v * nd + (c0 + j) * N0b + j0 + tx] += tile[tx][j];
+            S[v * nd + (c0 + j) * N0b + j0 + tx] += waited(tile[tx][j], wait);
 }
 
 // opposite spin: sigma(Ja, Jb) += sum over the p of Ja with Ja - p in the range, r of Jb
@@ -847,7 +848,8 @@ __global__ void __launch_bounds__(256) k_oz_sum_ab(const long long* __restrict__
                                                    int64_t v0, int64_t N0a, int64_t N0b, int64_t N1a, int64_t x0,
                                                    int64_t x1, const uint32_t* __restrict__ down_a,
                                                    const uint32_t* __restrict__ down_b,
-                                                   const uint64_t* __restrict__ stra, double* __restrict__ S) {
+                                                   const uint64_t* __restrict__ stra, double* __restrict__ S,
+                                                   const WaitCtl wait) {
     __shared__ int ve[16 * 16];
     for (int i = threadIdx.x; i < n * 16; i += blockDim.x)
         ve[i] = vexp[i];
@@ -905,7 +907,7 @@ __global__ void __launch_bounds__(256) k_oz_sum_ab(const long long* __restrict__
             acc += oz_sum<M>(T, e, s >> h);
         }
     }
-    *out = acc;
+    *out = waited(acc, wait);
 }
 
 // ---- set-up ----------------------------------------------------------------------------------------
@@ -1245,7 +1247,7 @@ static void oz_launch(OzArgs& a, int64_t nk, int64_t tiles, int max_ctas, cudaSt
     F2G_LAUNCH("k_oz");
 }
 
-void oz_same_spin(OzSigma& o, int set, int spin, const double* C, double* S, int nvec, int max_ctas, int* err,
+void oz_same_spin(OzSigma& o, int set, int spin, const double* C, double* S, int nvec, int max_ctas, const WaitCtl& wait,
                   cudaStream_t st) {
     const CIStrings* s = o.s;
     const SpinStrings& ss = s->spin(spin);
@@ -1275,16 +1277,17 @@ void oz_same_spin(OzSigma& o, int set, int spin, const double* C, double* S, int
         a.n = s->norb;
         a.nchunk = t.nchunk;
         a.ksteps = t.ksteps;
-        a.err = err;
+        a.wait = wait;
         oz_launch<true, 8>(a, ss.N2, nt, max_ctas, st);
         if (spin == 0) {
             k_oz_sum_a<<<dim3((unsigned)ss.N0, (unsigned)ceil_div(nx, 256)), 256, 0, st>>>(
-                w.E.get(), w.rexp.get(), nx, t.m2, t.down.get(), t.dpair.get(), t.bexp.get(), np, (int)tpv, ncol, t0, nd, S);
+                w.E.get(), w.rexp.get(), nx, t.m2, t.down.get(), t.dpair.get(), t.bexp.get(), np, (int)tpv, ncol, t0, nd, S,
+                wait);
             F2G_LAUNCH("k_oz_sum_a");
         } else {
             k_oz_sum_b<<<dim3((unsigned)ceil_div(ss.N0, 32), (unsigned)(nx / 32)), 256, 0, st>>>(
                 w.E.get(), w.rexp.get(), nx, t.m2, t.down.get(), t.dpair.get(), t.bexp.get(), np, ss.N0, (int)tpv, ncol, t0,
-                nd, S);
+                nd, S, wait);
             F2G_LAUNCH("k_oz_sum_b");
         }
     }
@@ -1292,15 +1295,15 @@ void oz_same_spin(OzSigma& o, int set, int spin, const double* C, double* S, int
 
 template <int NB>
 static void oz_sum_ab(const OzSigma& o, const OzScratch& w, const uint32_t* rows, int64_t nrows, int64_t v0, int64_t x0,
-                      int64_t x1, double* S, cudaStream_t st) {
+                      int64_t x1, double* S, const WaitCtl& wait, cudaStream_t st) {
     const CIStrings* s = o.s;
     k_oz_sum_ab<NB><<<dim3((unsigned)nrows, (unsigned)ceil_div(s->b.N0, 256)), 256, 0, st>>>(
         w.E.get(), w.rexp.get(), o.ldE, s->a.m1, s->b.m1, s->na, s->nb, s->norb, o.vexp.get(), rows, v0, s->a.N0, s->b.N0, s->a.N1, x0, x1,
-        s->a.down1.get(), s->b.down1.get(), s->a.str.get(), S);
+        s->a.down1.get(), s->b.down1.get(), s->a.str.get(), S, wait);
     F2G_LAUNCH("k_oz_sum_ab");
 }
 
-void oz_opposite(OzSigma& o, int set, const double* C, double* S, int nvec, int max_ctas, int* err, cudaStream_t st) {
+void oz_opposite(OzSigma& o, int set, const double* C, double* S, int nvec, int max_ctas, const WaitCtl& wait, cudaStream_t st) {
     const CIStrings* s = o.s;
     OzScratch& w = o.scr[set];
     const int64_t N1a = s->a.N1, N1b = s->b.N1, N0b = s->b.N0;
@@ -1331,7 +1334,7 @@ void oz_opposite(OzSigma& o, int set, const double* C, double* S, int nvec, int 
         a.n = s->norb;
         a.nchunk = (s->a.m1 + 2) / 3;
         a.ksteps = s->a.m1;
-        a.err = err;
+        a.wait = wait;
         const int tiles = ceil_div(N1b, kOzM);
         if (a.mb <= 8)
             oz_launch<false, 8>(a, x1 - x0, tiles, max_ctas, st);
@@ -1340,11 +1343,11 @@ void oz_opposite(OzSigma& o, int set, const double* C, double* S, int nvec, int 
         else
             oz_launch<false, 16>(a, x1 - x0, tiles, max_ctas, st);
         if (s->nb <= 4)
-            oz_sum_ab<4>(o, w, rows, nrows, v0, x0, x1, S, st);
+            oz_sum_ab<4>(o, w, rows, nrows, v0, x0, x1, S, wait, st);
         else if (s->nb <= 8)
-            oz_sum_ab<8>(o, w, rows, nrows, v0, x0, x1, S, st);
+            oz_sum_ab<8>(o, w, rows, nrows, v0, x0, x1, S, wait, st);
         else
-            oz_sum_ab<16>(o, w, rows, nrows, v0, x0, x1, S, st);
+            oz_sum_ab<16>(o, w, rows, nrows, v0, x0, x1, S, wait, st);
     };
     if (o.ranges.empty()) { // whole vectors per range
         const int64_t vs = std::max<int64_t>(1, o.range_strings / N1a);

@@ -61,8 +61,8 @@ void oz_build(const CIStrings* s, std::shared_ptr<OzSigma>& oz, const double* H,
 void oz_reserve(OzSigma& oz, int set, int nvec);
 // sigma = diagonal of H times C (overwrites), then the same-spin terms and the opposite-spin term, added
 void oz_diag(const OzSigma& oz, const double* C, double* S, int nvec, cudaStream_t st);
-void oz_same_spin(OzSigma& oz, int set, int spin, const double* C, double* S, int nvec, int max_ctas, int* err,
+void oz_same_spin(OzSigma& oz, int set, int spin, const double* C, double* S, int nvec, int max_ctas, const WaitCtl& wait,
                   cudaStream_t st);
-void oz_opposite(OzSigma& oz, int set, const double* C, double* S, int nvec, int max_ctas, int* err, cudaStream_t st);
+void oz_opposite(OzSigma& oz, int set, const double* C, double* S, int nvec, int max_ctas, const WaitCtl& wait, cudaStream_t st);
 
 } // namespace f2g

@@ -53,9 +53,9 @@ struct GramArgs {
     const int *el, *er;
     const void* list;
     double* out;
-    int* err;
+    WaitCtl wait;
     int64_t d, ko, kv, nK;
-    int64_t pstride;        // elements of one partial result, 0 if there is only the output
+    int64_t pstride;        // elements of one partial result
     int parts;              // K goes to partial result K % parts
     uint32_t k8, nsteps;    // groups of 8 rows R per row (a multiple of 4), double K steps of 32 rows
     int m, nv, S, nt, ntile, ntp, q, sym, stages, nbuf, colsbuf, stage_bytes, spt, per_lo, per_hi;
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_rg_gram(const __grid_constant_
     fence_after();
     constexpr uint32_t tmem = 0; // all 512 columns are this block's
     auto give_up = [&]() {
-        atomicExch(a.err, 1);
+        atomicExch(a.wait.err, 1);
         sh.abort = 1;
     };
     const uint32_t a_bytes = (uint32_t)a.nt * 512; // a double K step of eight digits (32 rows R) of a tile
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_rg_gram(const __grid_constant_
                 ce = max(a.er[I], 1);
             }
             const int s = it.ta * a.nt + rs;
-            double* out = a.out + (a.pstride ? (it.K % a.parts) * a.pstride : 0);
+            double* out = a.out + (it.K % a.parts) * a.pstride;
             const bool mine = ok && di < a.q && s < a.S, mirror = a.sym && it.ta != it.tb;
             int64_t I;
             int v, off = 0, neg = 0, ea = 1;
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_rg_gram(const __grid_constant_
         const uint32_t el = elect_lane();
         const uint32_t nt = (uint32_t)a.nt;
         uint32_t slot = 0, phase = 0, buf = 0, buf_phase = 1;
-        bool ok = true;
+        bool ok = a.wait.polls == 0; // with a limit on the tries (for tests) the first wait counts as given up
         for (int64_t w = blockIdx.x; ok && w < nitems; w += gridDim.x) {
             const GramItem it = gram_item(a, w);
             const bool two = !(a.sym && it.ta == it.tb);
@@ -487,8 +487,9 @@ __global__ void __launch_bounds__(256) k_rg_expand(const double* __restrict__ C,
     }
 }
 
-// out += the partial results, added as a tree over eight of them at a time
-__global__ void k_rg_reduce(int64_t size, int parts, const double* __restrict__ part, double* __restrict__ out) {
+// out += the partial results, added as a tree over eight of them at a time; NaN once a wait has given up
+__global__ void k_rg_reduce(int64_t size, int parts, const double* __restrict__ part, double* __restrict__ out,
+                            const WaitCtl wait) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < size; i += (int64_t)gridDim.x * blockDim.x) {
         double sum = 0.0;
         for (int p = 0; p < parts; p += 8) {
@@ -498,7 +499,7 @@ __global__ void k_rg_reduce(int64_t size, int parts, const double* __restrict__ 
                 x[j] = p + j < parts ? part[(p + j) * size + i] : 0.0;
             sum += ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
         }
-        out[i] += sum;
+        out[i] += waited(sum, wait);
     }
 }
 
@@ -588,13 +589,10 @@ bool rdm_gram(SigmaBuilder& sb, GramScratch& g, int spin, int holes, bool inner,
     const int64_t size = d * d;
     const bool many = nK >= 768;
     a.parts = (int)std::min<int64_t>({nK, many ? 128 : 16, std::max<int64_t>(4, (int64_t(1) << (many ? 25 : 20)) / size)});
-    a.pstride = a.parts > 1 ? size : 0;
-    a.out = out;
-    if (a.parts > 1) {
-        a.out = g.part.reserve((size_t)(a.parts * size));
-        F2G_CUDA(cudaMemsetAsync(a.out, 0, (size_t)(a.parts * size) * sizeof(double), st));
-    }
-    a.err = sb.tc_err.get();
+    a.pstride = size;
+    a.out = g.part.reserve((size_t)(a.parts * size));
+    F2G_CUDA(cudaMemsetAsync(a.out, 0, (size_t)(a.parts * size) * sizeof(double), st));
+    a.wait = sb.wait_ctl();
     a.d = d;
     a.ko = ko;
     a.kv = kv;
@@ -650,10 +648,9 @@ bool rdm_gram(SigmaBuilder& sb, GramScratch& g, int spin, int holes, bool inner,
         else
             gram_launch<3>(a, items, sms, st);
     }
-    if (a.parts > 1) {
-        k_rg_reduce<<<(unsigned)std::min<int64_t>((size + 255) / 256, 4096), 256, 0, st>>>(size, a.parts, a.out, out);
-        F2G_LAUNCH("k_rg_reduce");
-    }
+    k_rg_reduce<<<(unsigned)std::min<int64_t>((size + 255) / 256, 4096), 256, 0, st>>>(size, a.parts, a.out, out,
+                                                                                       a.wait);
+    F2G_LAUNCH("k_rg_reduce");
     return true;
 }
 

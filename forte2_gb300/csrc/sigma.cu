@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 
 #include "sigma.cuh"
 #include "opposite_sym.cuh"
@@ -589,7 +590,7 @@ bool opposite_tc_supported(const CIStrings* s);
 void build_beta_exc(const CIStrings* s, DevBuf<uint32_t>& exc, cudaStream_t st);
 void opposite_tc_vmax(const float* V, int64_t count, unsigned int* vmax, cudaStream_t st);
 void launch_opposite_tc(const CIStrings* s, const uint32_t* exc, const float* V, const unsigned int* vmax,
-                        const float* C, float* sig, unsigned int* cmax, int* err, long long poll_limit, int max_ctas,
+                        const float* C, float* sig, unsigned int* cmax, const WaitCtl& wait, int max_ctas,
                         cudaStream_t st, int nvec, const TcBOperands* tb);
 void opposite_tc_build_b(const CIStrings* s, const float* V, const unsigned int* vmax,
                          std::shared_ptr<TcBOperands>& tb, cudaStream_t st);
@@ -605,6 +606,39 @@ void dense_ss_reserve(const CIStrings* s, DenseSameSpin& d, int nvec, int set);
 void dense_ss_term(const CIStrings* s, DenseSameSpin& d, float* sig, int spin, bool accumulate, int nvec, int set,
                    cudaStream_t st);
 
+// Page-locked words, carved from chunks that stay allocated until the process exits: page-locked allocation
+// synchronises the device, so it happens once per 1,024 builders, not per builder.
+class PinnedWords {
+  public:
+    static PinnedWords& get() {
+        static PinnedWords inst;
+        return inst;
+    }
+    int* take() {
+        std::lock_guard<std::mutex> lock(mu_);
+        if (free_.empty()) {
+            int* chunk = nullptr;
+            F2G_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&chunk), 1024 * sizeof(int), cudaHostAllocPortable));
+            for (int i = 1023; i >= 0; --i)
+                free_.push_back(chunk + i);
+        }
+        int* p = free_.back();
+        free_.pop_back();
+        *p = 0;
+        return p;
+    }
+    void give(int* p) {
+        if (!p)
+            return;
+        std::lock_guard<std::mutex> lock(mu_);
+        free_.push_back(p);
+    }
+
+  private:
+    std::mutex mu_;
+    std::vector<int*> free_;
+};
+
 SigmaBuilder::SigmaBuilder(CIStrings* s_, double E_, const double* H_, const double* V_, int ll)
     : s(s_), n(s_->norb), log_level(ll) {
     for (auto& slot : ev)
@@ -612,6 +646,7 @@ SigmaBuilder::SigmaBuilder(CIStrings* s_, double E_, const double* H_, const dou
             F2G_CUDA(cudaEventCreate(&e));
     tc_err.reserve(1);
     F2G_CUDA(cudaMemsetAsync(tc_err.get(), 0, sizeof(int), 0));
+    wait_host = PinnedWords::get().take();
     if (opposite_sym_supported(s)) {
         osym = std::make_shared<OppositeSym>();
         osym->build(s);
@@ -665,7 +700,22 @@ int SigmaBuilder::tc_error() const {
     return h;
 }
 
+void SigmaBuilder::clear_waits() {
+    F2G_CUDA(cudaDeviceSynchronize()); // a kernel in flight may still set the words
+    F2G_CUDA(cudaMemset(tc_err.get(), 0, sizeof(int)));
+    *wait_host = 0;
+}
+
+void SigmaBuilder::check_waits() {
+    if (!*static_cast<volatile int*>(wait_host))
+        return;
+    clear_waits();
+    throw Error(1, "sigma builder: a tensor-core kernel gave up waiting for its operations; the results computed since "
+                   "the last check are not valid");
+}
+
 SigmaBuilder::~SigmaBuilder() {
+    PinnedWords::get().give(wait_host);
     for (auto& slot : ev)
         for (auto& e : slot)
             if (e)
@@ -1225,13 +1275,13 @@ void SigmaBuilder::run(const T* C, T* sig, cudaStream_t st, int mask, bool timed
                 oz_reserve(*oz, 0, nvec);
             oz_diag(*oz, C, sig, nvec, st);
             launch_transpose<T>(NA, NB, C, Ct_, st, nvec);
-            oz_same_spin(*oz, set, 1, Ct_, sig, nvec, max_ctas, tc_err.get(), st);
+            oz_same_spin(*oz, set, 1, Ct_, sig, nvec, max_ctas, wait_ctl(), st);
             if (timed)
                 F2G_CUDA(cudaEventRecord(cur_ev[1], st));
-            oz_same_spin(*oz, set, 0, C, sig, nvec, max_ctas, tc_err.get(), st);
+            oz_same_spin(*oz, set, 0, C, sig, nvec, max_ctas, wait_ctl(), st);
             if (timed)
                 F2G_CUDA(cudaEventRecord(cur_ev[2], st));
-            oz_opposite(*oz, set, C, sig, nvec, max_ctas, tc_err.get(), st);
+            oz_opposite(*oz, set, C, sig, nvec, max_ctas, wait_ctl(), st);
             if (timed)
                 F2G_CUDA(cudaEventRecord(cur_ev[3], st));
             return;
@@ -1277,7 +1327,7 @@ void SigmaBuilder::run(const T* C, T* sig, cudaStream_t st, int mask, bool timed
                 // graph launches use their own half of the scale scratch, so a captured solve and a
                 // direct call on the same builder never share it
                 unsigned int* cmax = tc_cmax.get() + (graph ? 65536 : 0);
-                launch_opposite_tc(s, beta_exc.get(), Vt, tc_vmax.get(), C, sig, cmax, tc_err.get(), tc_poll_limit,
+                launch_opposite_tc(s, beta_exc.get(), Vt, tc_vmax.get(), C, sig, cmax, wait_ctl(),
                                    max_ctas, st, nvec, (use_tma_b && tc_b_ready) ? tc_b.get() : nullptr);
                 done = true;
             }
@@ -1383,7 +1433,7 @@ void SigmaBuilder::spmm_blocks(int spin, const double* X, double* Y, bool accumu
 void SigmaBuilder::opposite_sym(const double* V, const double* C, double* sig, cudaStream_t st, int nvec, int ctas,
                                 bool graph) {
     if (symd)
-        sym_digits_run(*symd, s, graph ? 1 : 0, V, C, sig, nvec, ctas, tc_err.get(), st);
+        sym_digits_run(*symd, s, graph ? 1 : 0, V, C, sig, nvec, ctas, wait_ctl(), st);
     else
         launch_opposite_sym(s, *osym, V, C, sig, st, nvec, ctas);
 }
@@ -1512,6 +1562,7 @@ int SigmaBuilder::batch_size(int nvec) const {
 }
 
 void SigmaBuilder::hamiltonian(const double* C, double* sigma, cudaStream_t st, int nvec) {
+    check_waits();
     check_memory();
     const int64_t nd = s->ndet, nf = s->nfull;
     if (nd == 0 || nvec <= 0)

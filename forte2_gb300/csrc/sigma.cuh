@@ -98,10 +98,14 @@ struct SigmaBuilder {
     bool use_small = false;
     DevBuf<uint32_t> small_exc[2];
     DevBuf<uint32_t> beta_exc; // beta single excitations per string for its scatter
-    DevBuf<int> tc_err;        // set by the tensor-core kernel if a bounded wait gave up
+    DevBuf<int> tc_err;        // set by a tensor-core kernel if a bounded wait gave up
+    int* wait_host = nullptr;  // the same in page-locked host memory
+    WaitCtl wait_ctl() const { return {tc_err.get(), wait_host, (int)std::min<long long>(tc_poll_limit, 1 << 30)}; }
+    void check_waits(); // throws (and clears both) if a wait gave up in work that the host has waited for
+    void clear_waits();
     DevBuf<unsigned int> tc_cmax; // per-vector largest |C| of a tensor-core launch (its operand scale)
     DevBuf<unsigned int> tc_vmax; // largest |V| of the FP32 integrals (the FP16 split's scale)
-    long long tc_poll_limit = 0; // polls per bounded wait in the tensor-core kernel (0: the default)
+    long long tc_poll_limit = 0; // polls per bounded wait in the tensor-core kernels (0: the default)
     bool tensor_cores_available() const;
     int tc_error() const;
     int log_level = 3;

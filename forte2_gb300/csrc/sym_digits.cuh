@@ -33,6 +33,6 @@ std::shared_ptr<SymDigits> sym_digits_build(const CIStrings* s, const OppositeSy
 void sym_digits_reserve(SymDigits& d, const CIStrings* s, int set);
 // sigma += the opposite-spin term for nvec C1-embedded vectors back to back
 void sym_digits_run(SymDigits& d, const CIStrings* s, int set, const double* V, const double* C, double* sig, int nvec,
-                    int max_ctas, int* err, cudaStream_t st);
+                    int max_ctas, const WaitCtl& wait, cudaStream_t st);
 
 } // namespace f2g

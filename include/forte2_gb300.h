@@ -119,6 +119,11 @@ int f2g_sigma_set_variant(void* sigma, int which, int value);
 /* 1 if a tensor-core build (FP32, or FP64 by digit splitting, sigma or RDM) gave up waiting for its matrix
  * operations (results invalid). */
 int f2g_sigma_tc_error(void* sigma, int* out);
+/* Error 1, once, if a tensor-core build gave up waiting in work that the host has waited for since the last check
+ * (no synchronisation). f2g_sigma_apply, _apply_host, _apply_csf, f2g_sigma_rdm and f2g_dgraph_state check by
+ * themselves; a caller that reads a device result of its last call checks with this after its own synchronisation
+ * (the FP64 results of such a call are NaN). */
+int f2g_sigma_check(void* sigma);
 /* Hamiltonian(basis, sigma) for nvec vectors of length ndet stored back to back
  * (ci_sigma_builder.cc:187-218); sigma is overwritten. */
 int f2g_sigma_apply(void* sigma, const double* dev_C, double* dev_sigma, int nvec, void* stream);
