@@ -8,16 +8,23 @@
 // the pairs with s or r occupied in Kb along, 196 products for 64 that count) needs 3.0 ms for the 9 million hole
 // pairs of CAS(14,14) and took 5.8 ms.
 //
-// The vector, scaled by its largest exponent to integers of 62 bits, is cut into eight FP16 digits once (k_sy_expand:
-// rows (Ia, s) over the Kb of the one irrep that Ia and s leave), the integrals likewise (k_sy_integrals, in the
-// order of each Ka's pairs, sgn(Ka, q) included). k_sy_gemm's A operand is contiguous along M = Kb, so a row's digits go from
-// there to core matrices by 16-byte copies. Products of digits i, j with i + j <= 7 are kept (the next are 2^-64 of
-// the two maxima), sums of at most 64 rows of eight products are exact in FP32, and an element of E is their 96-bit sum
-// rounded once. k_sy_sum adds sgn E into sigma, a thread per determinant in a fixed order.
+// The rows of the vector, scaled by their largest exponents e(Ia) to integers of 62 bits, are cut into eight FP16 digits
+// once (k_sy_expand: rows (Ia, s) over the Kb of the one irrep that Ia and s leave). The integrals take the rows' scales
+// along: those of a Ka and an output pair (p, r) are the V[p, r, q, s] 2^e(Ka + q), scaled by the largest of them
+// (k_sy_integrals, in the order of each Ka's pairs, sgn(Ka, q) included). k_sy_gemm's A operand is contiguous along
+// M = Kb, so a row's digits go from there to core matrices by 16-byte copies. Products of digits i, j with i + j <= 7 are
+// kept, sums of at most 64 rows of eight products are exact in FP32, and an element of E is their 96-bit sum rounded
+// once. k_sy_sum adds sgn E into sigma, a thread per determinant in a fixed order.
+//
+// Accuracy. A product of E[Kb][(p, r)] loses less than 2^-58 of the largest |V[p, r, q, s]| max_Ib |C(Ka + q, Ib)| in its
+// sum: 2^-62 each from the element and the integral, at most 2^-59 from the digit products left out. Compared with a
+// sum in FP64 that is less in the norm of the rows that meet in a Ka, and more for an element whose own products are
+// all 2^-6 and less of that largest one. (With one scale for the whole vector that held for its norm alone: rows at 1e-12
+// of the largest were left with 22 bits.)
 //
 // Bound: operand copies and drains by turns. CAS(14,14) in 8 irreps (1,472,512 determinants), opposite-spin term: 5.82 ->
-// 1.6 ms (k_sy_gemm 1.09 ms, with unswizzled core matrices, whose 16-byte copies take a wavefront each, 1.24 ms;
-// k_sy_sum 0.34 ms, k_sy_expand 0.10 ms).
+// 1.7 ms (k_sy_gemm 1.15 ms; 1.09 ms with one scale for all output pairs; 0.15 ms more with unswizzled core matrices,
+// whose 16-byte copies take a wavefront each; k_sy_sum 0.34 ms, k_sy_expand 0.10 ms).
 #include <algorithm>
 
 #include "common.cuh"
@@ -36,7 +43,9 @@ constexpr int kYStagesMax = 6;
 constexpr int kYSmem = 216 * 1024;
 constexpr int64_t kYBytes = int64_t(1) << 31;       // digits at a time
 constexpr int64_t kYBytesE = int64_t(1) << 32;      // E at a time
-constexpr int kYBad = 0x7ff;
+constexpr int kYUnit = 88 - 68;                     // exponent of the digits' sums, see below
+constexpr int kYSlow = 1 << 16;                     // with the first exponent of four: some need the general conversion
+constexpr int kYBad = 1 << 14;                       // exponent of an output pair whose sum holds an infinity or NaN
 
 struct SymShared {
     alignas(8) uint64_t full[kYStagesMax], empty[kYStagesMax], acc_full[4], acc_empty[4], drain;
@@ -48,7 +57,7 @@ struct SymShared {
 struct SymArgs {
     const uint4 *z, *b;
     double* e;
-    const int* mx;
+    const int* ecol;
     WaitCtl wait;
     const uint32_t* up_a;
     const int8_t* hka;
@@ -57,19 +66,22 @@ struct SymArgs {
     OrbSym os;
 };
 
-// largest biased exponents of a (into mx[0]) and b (into mx[1])
-__global__ void __launch_bounds__(256) k_sy_max(int64_t na, const double* __restrict__ a, int64_t nb,
-                                                const double* __restrict__ b, int* __restrict__ mx) {
-    for (int w = 0; w < 2; ++w) {
-        const uint32_t* hi = reinterpret_cast<const uint32_t*>(w ? b : a) + 1;
-        const int64_t n = w ? nb : na, stride = (int64_t)gridDim.x * 256;
-        uint32_t m = 0;
-#pragma unroll 8
-        for (int64_t i = blockIdx.x * (int64_t)256 + threadIdx.x; i < n; i += stride)
-            m = max(m, __ldg(hi + 2 * i) & 0x7fffffffu);
-        m = __reduce_max_sync(0xffffffffu, m);
-        if ((threadIdx.x & 31) == 0 && m)
-            atomicMax(mx + w, (int)(m >> 20));
+// ec[Ia]: largest biased exponent of row Ia of the vector, at least 1; a block per row
+__global__ void __launch_bounds__(256) k_sy_rowexp(int64_t N0b, const double* __restrict__ C, int* __restrict__ ec) {
+    const uint32_t* hi = reinterpret_cast<const uint32_t*>(C + blockIdx.x * N0b) + 1;
+    uint32_t m = 0;
+#pragma unroll 4
+    for (int64_t i = threadIdx.x; i < N0b; i += 256)
+        m = max(m, __ldg(hi + 2 * i) & 0x7fffffffu);
+    m = __reduce_max_sync(0xffffffffu, m);
+    __shared__ uint32_t w[8];
+    if ((threadIdx.x & 31) == 0)
+        w[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < 8; ++i)
+            m = max(m, w[i]);
+        ec[blockIdx.x] = max((int)(m >> 20), 1);
     }
 }
 
@@ -102,17 +114,17 @@ __device__ __forceinline__ void digits8(const uint64_t (&y)[8], uint4* dst, int 
 // pos0 .. pos0 + chunk
 __global__ void __launch_bounds__(256) k_sy_expand(const double* __restrict__ C, int64_t N0a, int64_t N0b, int n, int lmax,
                                                    int pos0, int chunk, const int8_t* __restrict__ hja, const __grid_constant__ OrbSym os,
-                                                   const uint32_t* __restrict__ tab, const int* __restrict__ mx,
+                                                   const uint32_t* __restrict__ tab, const int* __restrict__ ec,
                                                    uint4* __restrict__ z) {
     __shared__ uint4 sm[8][256]; // a warp's digits, written from here in whole lines
-    const int E = max(mx[0], 1), g8 = chunk >> 3, lane = threadIdx.x & 31; // g8 and with it the total: multiples of 16
+    const int g8 = chunk >> 3, lane = threadIdx.x & 31; // g8 and with it the total: multiples of 16
     uint4* my = sm[threadIdx.x >> 5];
     const int64_t total = N0a * n * g8;
     for (int64_t t0 = blockIdx.x * (int64_t)256 + (threadIdx.x & ~31); t0 < total; t0 += (int64_t)gridDim.x * 256) {
         const int64_t t = min(t0 + lane, total - 1);
         const int g = (int)(t % g8);
         const int64_t r = t / g8, Ia = r / n;
-        const int s = (int)(r - Ia * n);
+        const int s = (int)(r - Ia * n), E = __ldg(ec + Ia);
         const uint4* src = reinterpret_cast<const uint4*>(tab + ((int64_t)(os.S ^ hja[Ia] ^ os.h[s]) * n + s) * lmax + pos0 + g * 8);
         const uint4 a0 = __ldg(src), a1 = __ldg(src + 1);
         const uint32_t a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
@@ -136,41 +148,79 @@ __global__ void __launch_bounds__(256) k_sy_expand(const double* __restrict__ C,
     }
 }
 
-// b[(Ka, t)][K step][group of 8 (q, s)][digit][(p, r)][8]: sgn(Ka, q) V[p, r, q, s]; a block per Ka
+// b[(Ka, t)][K step][group of 8 (q, s)][digit][(p, r)][8]: sgn(Ka, q) V[p, r, q, s] 2^ec(Ka + q) below 2^ecol;
+// ecol[(Ka, t)][(p, r)]: the largest exponent of these products, kYBad if one is not finite (and kYSlow); a block per Ka
 __global__ void __launch_bounds__(256) k_sy_integrals(const double* __restrict__ V, int n, int ma, const uint32_t* __restrict__ up_a,
-                                                      const __grid_constant__ OrbSym os, int slots, const int* __restrict__ mx, uint4* __restrict__ b) {
+                                                      const __grid_constant__ OrbSym os, int slots, const int* __restrict__ ec,
+                                                      int* __restrict__ ecol, uint4* __restrict__ b) {
     __shared__ uint8_t q_of[8][kSymSlots], s_of[8][kSymSlots], neg_of[8][kSymSlots];
-    __shared__ int cnt[8];
+    __shared__ int16_t ec_of[8][kSymSlots];
+    __shared__ int cnt[8], col[8 * kSymSlots];
     const int64_t Ka = blockIdx.x;
     if (threadIdx.x < os.nirrep) {
         const int t = threadIdx.x;
         int c = 0;
         for (int i = 0; i < ma; ++i) {
             const uint32_t e = up_a[Ka * ma + i];
-            const int q = e_orb(e), h = t ^ os.h[q];
+            const int q = e_orb(e), h = t ^ os.h[q], x = ec[e_addr(e)];
             for (int j = 0; j < os.cnt[h]; ++j, ++c) {
                 q_of[t][c] = (uint8_t)q;
                 s_of[t][c] = (uint8_t)os.list[h][j];
                 neg_of[t][c] = (uint8_t)e_neg(e);
+                ec_of[t][c] = (int16_t)x;
             }
         }
         cnt[t] = c;
     }
     __syncthreads();
-    const int E = max(mx[1], 1), groups = slots >> 3;
-    for (int i = threadIdx.x; i < os.nirrep * groups * slots; i += 256) {
-        const int o = i % slots, g = i / slots % groups, t = i / (slots * groups);
+    const int groups = slots >> 3, items = os.nirrep * groups * slots, stride = os.nirrep * slots;
+    for (int i = threadIdx.x; i < stride; i += 256)
+        col[i] = 2; // of a zero below the smallest scale
+    __syncthreads();
+    double x[8];
+    auto load = [&](int i, int& o, int& t, int& g) { // eight integrals of one output pair
+        o = i % slots;
+        g = i / slots % groups;
+        t = i / (slots * groups);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int k = g * 8 + j;
+            x[j] = o < cnt[t] && k < cnt[t]
+                       ? __ldg(V + (((int64_t)q_of[t][o] * n + s_of[t][o]) * n + q_of[t][k]) * n + s_of[t][k])
+                       : 0.0;
+        }
+    };
+    int o, t, g;
+    for (int i = threadIdx.x; i < items; i += 256) {
+        load(i, o, t, g);
+        int m = 2;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int k = g * 8 + j, ev = (int)((__double_as_longlong(x[j]) >> 52) & 0x7ff);
+            if (o < cnt[t] && k < cnt[t])
+                m = max(m, ev == 0x7ff || ec_of[t][k] == 0x7ff ? kYBad : max(ev, 1) + ec_of[t][k]);
+        }
+        atomicMax(col + t * slots + o, m);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < stride; i += 256) {
+        int x = col[i];
+        if ((i & 3) == 0) {
+            const int lo = min(min(x, col[i + 1]), min(col[i + 2], col[i + 3]));
+            const int hi = max(max(x, col[i + 1]), max(col[i + 2], col[i + 3]));
+            if (lo + kYUnit - 32 < kOzSafeLo || hi + kYUnit > kOzSafeHi)
+                x |= kYSlow;
+        }
+        ecol[Ka * stride + i] = x;
+    }
+    for (int i = threadIdx.x; i < items; i += 256) {
+        if (items > 256)
+            load(i, o, t, g); // with 16 pairs in 8 irreps every thread still has its own
         uint64_t y[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const int k = g * 8 + j;
-            double x = 0.0;
-            bool neg = false;
-            if (o < cnt[t] && k < cnt[t]) {
-                x = __ldg(V + (((int64_t)q_of[t][o] * n + s_of[t][o]) * n + q_of[t][k]) * n + s_of[t][k]);
-                neg = neg_of[t][k];
-            }
-            y[j] = gram_digits(x, neg, E);
+            y[j] = gram_digits(x[j], neg_of[t][k], o < cnt[t] && k < cnt[t] ? col[t * slots + o] - ec_of[t][k] : 1);
         }
         digits8(y, b + ((Ka * os.nirrep + t) * groups + g) * 8 * slots + o, slots);
     }
@@ -182,6 +232,16 @@ __device__ __forceinline__ void sym_item(const SymArgs& a, int64_t w, int64_t& K
     const int64_t r = w / a.tiles;
     c = (int)(r % a.nirrep);
     Ka = a.ka0 + r / a.nirrep;
+}
+
+__device__ __forceinline__ void sym_next(const SymArgs& a, int64_t& Ka, int& c, int& tile) { // the item after it
+    if (++tile < a.tiles)
+        return;
+    tile = 0;
+    if (++c < a.nirrep)
+        return;
+    c = 0;
+    ++Ka;
 }
 
 __global__ void __launch_bounds__(kYThreads, 1) k_sy_gemm(const __grid_constant__ SymArgs a, int64_t nitems) {
@@ -227,10 +287,10 @@ __global__ void __launch_bounds__(kYThreads, 1) k_sy_gemm(const __grid_constant_
         int64_t last = -1;
         int hk = 0;
         bool ok = true;
-        for (int64_t w = w0; ok && w < w1; ++w) {
-            int64_t Ka;
-            int c, tile;
-            sym_item(a, w, Ka, c, tile);
+        int64_t Ka;
+        int c, tile;
+        sym_item(a, min(w0, nitems - 1), Ka, c, tile);
+        for (int64_t w = w0; ok && w < w1; ++w, sym_next(a, Ka, c, tile)) {
             if (Ka != last) {
                 last = Ka;
                 hk = a.hka[Ka];
@@ -293,14 +353,27 @@ __global__ void __launch_bounds__(kYThreads, 1) k_sy_gemm(const __grid_constant_
         // ---- drains: a row's eight groups into one FP64 number, four columns at a time
         const int quarter = warp & 3, part = (warp - kYProd) >> 2;
         uint32_t buf = 0, phase = 0;
-        const int ec = max(a.mx[0], 1), ev = max(a.mx[1], 1);
-        const bool bad = ec >= kYBad || ev >= kYBad;
-        const int e0 = 88 - 68 + ec + ev;
-        const bool safe = e0 - 32 >= kOzSafeLo && e0 <= kOzSafeHi;
+        auto exponents = [&](int64_t Ka, int c) { // of an item's output pairs, four to a vector
+            return reinterpret_cast<const int4*>(a.ecol + (Ka * a.nirrep + (a.os.S ^ __ldg(a.hka + Ka) ^ c)) * a.slots);
+        };
+        const int last4 = a.slots / 4 - 1;
+        int64_t nKa; // the next item: its exponents are loaded an item ahead, so that nothing waits for them
+        int nc, ntile;
+        sym_item(a, min(w0, nitems - 1), nKa, nc, ntile);
+        const int4* ecol_next = exponents(nKa, nc);
+        int4 ev_next = __ldg(ecol_next + min(part, last4));
         for (int64_t w = w0; w < w1; ++w) {
-            int64_t Ka;
-            int c, tile;
-            sym_item(a, w, Ka, c, tile);
+            const int64_t Ka = nKa;
+            const int c = nc, tile = ntile;
+            const int4* ecol = ecol_next;
+            int4 ev = ev_next;
+            if (w + 1 < w1) {
+                sym_next(a, nKa, nc, ntile);
+                if (nc != c || nKa != Ka) {
+                    ecol_next = exponents(nKa, nc);
+                    ev_next = __ldg(ecol_next + min(part, last4));
+                }
+            }
             if (!mbar_wait_warp(smem_u32(&sh.acc_full[buf]), phase, abort)) {
                 give_up();
                 break;
@@ -314,6 +387,10 @@ __global__ void __launch_bounds__(kYThreads, 1) k_sy_gemm(const __grid_constant_
 #pragma unroll
                 for (int g = 0; g < 8; ++g)
                     tmem_ld4(at + g * a.slots + b * 4, r + 4 * g);
+                const bool safe = !(ev.x & kYSlow);
+                const int col[4] = {ev.x & (kYSlow - 1), ev.y, ev.z, ev.w};
+                if (b + kYEpi / 4 < a.most / 4)
+                    ev = __ldg(ecol + b + kYEpi / 4);
                 tmem_wait_ld();
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -336,9 +413,11 @@ __global__ void __launch_bounds__(kYThreads, 1) k_sy_gemm(const __grid_constant_
                     const int sft = min(32, __clz((uint32_t)((unsigned long long)hi >> 16)) + 14);
                     long long T = (hi << sft) | (long long)((unsigned long long)low >> (32 - sft));
                     T = neg ? -T : T;
-                    // units of T: 2^(32 - sft) 2^56 2^(ec - 1084) 2^(ev - 1084)
-                    const double x = safe ? oz_double(T, (e0 - sft - 1016) << 20, -(1 << 20)) : oz_value(T, e0 - sft);
-                    out[(b * 4 + j) * pitch] = bad ? __longlong_as_double(0x7ff8000000000000ll) : x;
+                    // units of T: 2^(32 - sft) 2^56 2^(col - 2 1084)
+                    const int e = col[j] + kYUnit - sft;
+                    out[(b * 4 + j) * pitch] = safe ? oz_double(T, (e - 1016) << 20, -(1 << 20))
+                                               : col[j] >= kYBad ? __longlong_as_double(0x7ff8000000000000ll)
+                                                                 : oz_value(T, e);
                 }
             }
             fence_before();
@@ -569,7 +648,8 @@ void sym_digits_reserve(SymDigits& d, const CIStrings* s, int set) {
     w.z.reserve((size_t)(s->a.N0 * s->norb * d.chunk));
     w.b.reserve((size_t)(s->a.N1 * nir * d.slots * d.slots));
     w.e.reserve((size_t)(d.ka * d.most * nir * d.chunk));
-    w.mx.reserve(2);
+    w.ec.reserve((size_t)s->a.N0);
+    w.ecol.reserve((size_t)(s->a.N1 * nir * d.slots));
 }
 
 void sym_digits_run(SymDigits& d, const CIStrings* s, int set, const double* V, const double* C, double* sig, int nvec,
@@ -578,13 +658,13 @@ void sym_digits_run(SymDigits& d, const CIStrings* s, int set, const double* V, 
         sym_digits_reserve(d, s, 0);
     SymDigits::Scratch& w = d.set[set];
     const int n = s->norb, nir = d.os.nirrep;
-    const int64_t N0a = s->a.N0, N0b = s->b.N0, n4 = (int64_t)n * n * n * n;
+    const int64_t N0a = s->a.N0, N0b = s->b.N0;
     const int sms = sm_total(), ctas = max_ctas > 0 ? std::min(max_ctas, sms) : sms;
     SymArgs a{};
     a.z = w.z.get();
     a.b = w.b.get();
     a.e = w.e.get();
-    a.mx = w.mx.get();
+    a.ecol = w.ecol.get();
     a.wait = wait;
     a.up_a = s->a.up1.get();
     a.hka = d.hka.get();
@@ -602,15 +682,11 @@ void sym_digits_run(SymDigits& d, const CIStrings* s, int set, const double* V, 
     F2G_CUDA(cudaFuncSetAttribute(k_sy_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, kYSmem));
     for (int v = 0; v < nvec; ++v) {
         const double* x = C + v * N0a * N0b;
-        F2G_CUDA(cudaMemsetAsync(w.mx.get(), 0, 2 * sizeof(int), st));
-        k_sy_max<<<(unsigned)std::min<int64_t>(ceil_div(N0a * N0b, 2048), (int64_t)sms * 8), 256, 0, st>>>(N0a * N0b, x, n4, V,
-                                                                                                         w.mx.get());
-        F2G_LAUNCH("k_sy_max");
-        if (v == 0) {
-            k_sy_integrals<<<(unsigned)s->a.N1, 256, 0, st>>>(V, n, s->a.m1, s->a.up1.get(), d.os, d.slots, w.mx.get(),
-                                                              w.b.get());
-            F2G_LAUNCH("k_sy_integrals");
-        }
+        k_sy_rowexp<<<(unsigned)N0a, 256, 0, st>>>(N0b, x, w.ec.get());
+        F2G_LAUNCH("k_sy_rowexp");
+        k_sy_integrals<<<(unsigned)s->a.N1, 256, 0, st>>>(V, n, s->a.m1, s->a.up1.get(), d.os, d.slots, w.ec.get(),
+                                                          w.ecol.get(), w.b.get());
+        F2G_LAUNCH("k_sy_integrals");
         for (int pos0 = 0; pos0 < d.lmax; pos0 += d.chunk) {
             // the last part may be shorter than the others: positions past lmax do not exist
             const int now = std::min(d.chunk, d.lmax - pos0);
@@ -618,7 +694,7 @@ void sym_digits_run(SymDigits& d, const CIStrings* s, int set, const double* V, 
             a.tiles = now / kYM;
             const int64_t work = N0a * n * (now / 8);
             k_sy_expand<<<(unsigned)std::min<int64_t>(ceil_div(work, 256), (int64_t)sms * 32), 256, 0, st>>>(
-                x, N0a, N0b, n, d.lmax, pos0, now, d.hja.get(), d.os, d.tab.get(), w.mx.get(), w.z.get());
+                x, N0a, N0b, n, d.lmax, pos0, now, d.hja.get(), d.os, d.tab.get(), w.ec.get(), w.z.get());
             F2G_LAUNCH("k_sy_expand");
             for (int64_t ka0 = 0; ka0 < s->a.N1; ka0 += d.ka) {
                 const int64_t ka1 = std::min(ka0 + d.ka, s->a.N1), items = (ka1 - ka0) * nir * a.tiles;
