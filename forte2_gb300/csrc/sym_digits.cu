@@ -44,8 +44,9 @@ constexpr int kYSmem = 216 * 1024;
 constexpr int64_t kYBytes = int64_t(1) << 31;       // digits at a time
 constexpr int64_t kYBytesE = int64_t(1) << 32;      // E at a time
 constexpr int kYUnit = 88 - 68;                     // exponent of the digits' sums, see below
+constexpr int kYBadRow = 1 << 15;                   // with a row's exponent: it holds an infinity or NaN
 constexpr int kYSlow = 1 << 16;                     // with the first exponent of four: some need the general conversion
-constexpr int kYBad = 1 << 14;                       // exponent of an output pair whose sum holds an infinity or NaN
+constexpr int kYBad = 1 << 14;                       // exponent of an output pair with an integral that is not finite
 
 struct SymShared {
     alignas(8) uint64_t full[kYStagesMax], empty[kYStagesMax], acc_full[4], acc_empty[4], drain;
@@ -66,14 +67,20 @@ struct SymArgs {
     OrbSym os;
 };
 
-// ec[Ia]: largest biased exponent of row Ia of the vector, at least 1; a block per row
-__global__ void __launch_bounds__(256) k_sy_rowexp(int64_t N0b, const double* __restrict__ C, int* __restrict__ ec) {
+// ec[Ia]: largest biased exponent of the finite elements of row Ia of the vector, at least 1, with kYBadRow if there are
+// others (then ec[N0a] is set: k_sy_not_finite adds their products); a block per row
+__global__ void __launch_bounds__(256) k_sy_rowexp(int64_t N0a, int64_t N0b, const double* __restrict__ C, int* __restrict__ ec) {
     const uint32_t* hi = reinterpret_cast<const uint32_t*>(C + blockIdx.x * N0b) + 1;
     uint32_t m = 0;
+    bool bad = false;
 #pragma unroll 4
-    for (int64_t i = threadIdx.x; i < N0b; i += 256)
-        m = max(m, __ldg(hi + 2 * i) & 0x7fffffffu);
+    for (int64_t i = threadIdx.x; i < N0b; i += 256) {
+        const uint32_t x = __ldg(hi + 2 * i) & 0x7fffffffu;
+        bad |= x >= 0x7ff00000u;
+        m = max(m, x < 0x7ff00000u ? x : 0u);
+    }
     m = __reduce_max_sync(0xffffffffu, m);
+    bad = __syncthreads_or(bad);
     __shared__ uint32_t w[8];
     if ((threadIdx.x & 31) == 0)
         w[threadIdx.x >> 5] = m;
@@ -81,7 +88,9 @@ __global__ void __launch_bounds__(256) k_sy_rowexp(int64_t N0b, const double* __
     if (threadIdx.x == 0) {
         for (int i = 1; i < 8; ++i)
             m = max(m, w[i]);
-        ec[blockIdx.x] = max((int)(m >> 20), 1);
+        ec[blockIdx.x] = max((int)(m >> 20), 1) | (bad ? kYBadRow : 0);
+        if (bad)
+            atomicExch(ec + N0a, 1);
     }
 }
 
@@ -124,14 +133,18 @@ __global__ void __launch_bounds__(256) k_sy_expand(const double* __restrict__ C,
         const int64_t t = min(t0 + lane, total - 1);
         const int g = (int)(t % g8);
         const int64_t r = t / g8, Ia = r / n;
-        const int s = (int)(r - Ia * n), E = __ldg(ec + Ia);
+        const int s = (int)(r - Ia * n), e = __ldg(ec + Ia), E = e & (kYBadRow - 1);
         const uint4* src = reinterpret_cast<const uint4*>(tab + ((int64_t)(os.S ^ hja[Ia] ^ os.h[s]) * n + s) * lmax + pos0 + g * 8);
         const uint4 a0 = __ldg(src), a1 = __ldg(src + 1);
         const uint32_t a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
         uint64_t y[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-            y[j] = gram_digits(a[j] == ~0u ? 0.0 : __ldg(C + Ia * N0b + (a[j] & 0x7fffffffu)), a[j] >> 31, E);
+        for (int j = 0; j < 8; ++j) {
+            double x = a[j] == ~0u ? 0.0 : __ldg(C + Ia * N0b + (a[j] & 0x7fffffffu));
+            if (e >= kYBadRow && !isfinite(x))
+                x = 0.0;
+            y[j] = gram_digits(x, a[j] >> 31, E);
+        }
         uint4 q[8];
         digits8(y, q, 1);
 #pragma unroll
@@ -162,7 +175,7 @@ __global__ void __launch_bounds__(256) k_sy_integrals(const double* __restrict__
         int c = 0;
         for (int i = 0; i < ma; ++i) {
             const uint32_t e = up_a[Ka * ma + i];
-            const int q = e_orb(e), h = t ^ os.h[q], x = ec[e_addr(e)];
+            const int q = e_orb(e), h = t ^ os.h[q], x = ec[e_addr(e)] & (kYBadRow - 1);
             for (int j = 0; j < os.cnt[h]; ++j, ++c) {
                 q_of[t][c] = (uint8_t)q;
                 s_of[t][c] = (uint8_t)os.list[h][j];
@@ -198,7 +211,7 @@ __global__ void __launch_bounds__(256) k_sy_integrals(const double* __restrict__
         for (int j = 0; j < 8; ++j) {
             const int k = g * 8 + j, ev = (int)((__double_as_longlong(x[j]) >> 52) & 0x7ff);
             if (o < cnt[t] && k < cnt[t])
-                m = max(m, ev == 0x7ff || ec_of[t][k] == 0x7ff ? kYBad : max(ev, 1) + ec_of[t][k]);
+                m = max(m, ev == 0x7ff ? kYBad : max(ev, 1) + ec_of[t][k]);
         }
         atomicMax(col + t * slots + o, m);
     }
@@ -546,6 +559,48 @@ __global__ void __launch_bounds__(256) k_sy_sum(int64_t N0b, int n, int na, int 
     *out = waited(acc, wait);
 }
 
+// Elements of the vector that are not finite count as zero in E. If there are any, their products are added here, as a
+// sum in FP64 would have them.
+__global__ void __launch_bounds__(256) k_sy_not_finite(int64_t N0a, int64_t N0b, int n, int na, int nb, int ma, const __grid_constant__ OrbSym os,
+                                                       const uint32_t* __restrict__ down_a, const uint32_t* __restrict__ up_a,
+                                                       const uint32_t* __restrict__ down_b, const int32_t* __restrict__ kpos,
+                                                       const int8_t* __restrict__ hja, const int32_t* __restrict__ jb,
+                                                       const int32_t* __restrict__ njb_of, int64_t njb, const uint32_t* __restrict__ tab,
+                                                       int lmax, const int* __restrict__ ec, const double* __restrict__ C,
+                                                       const double* __restrict__ V, double* __restrict__ sig) {
+    if (!ec[N0a])
+        return;
+    for (int64_t Ja = blockIdx.x; Ja < N0a; Ja += gridDim.x)
+        for (int i = 0; i < na * ma; ++i) {
+            const uint32_t ep = down_a[Ja * na + i / ma], eq = up_a[(int64_t)e_addr(ep) * ma + i % ma];
+            const int64_t Ia = e_addr(eq);
+            if (ec[Ia] < kYBadRow)
+                continue;
+            const int p = e_orb(ep), q = e_orb(eq), h = os.S ^ hja[Ja], cnt = njb_of[h];
+            for (int at = threadIdx.x; at < cnt; at += 256) {
+                const int64_t Jb = jb[h * njb + at];
+                double acc = 0.0;
+                for (int j = 0; j < nb; ++j) {
+                    const uint32_t er = down_b[Jb * nb + j];
+                    const int kp = kpos[e_addr(er)], hb = kp >> 24, hs = os.S ^ hja[Ia] ^ hb;
+                    for (int l = 0; l < os.cnt[hs]; ++l) {
+                        const int s = os.list[hs][l];
+                        const uint32_t es = tab[((int64_t)hb * n + s) * lmax + (kp & 0xffffff)];
+                        if (es == ~0u)
+                            continue;
+                        const double x = C[Ia * N0b + (es & 0x7fffffffu)];
+                        if (!isfinite(x)) {
+                            const double y = V[(((int64_t)p * n + e_orb(er)) * n + q) * n + s] * x;
+                            acc += (e_neg(ep) ^ e_neg(er) ^ e_neg(eq) ^ (es >> 31)) ? -y : y;
+                        }
+                    }
+                }
+                if (acc != 0.0)
+                    sig[Ja * N0b + Jb] += acc;
+            }
+        }
+}
+
 int sm_total() {
     int dev = 0, sms = 0;
     F2G_CUDA(cudaGetDevice(&dev));
@@ -648,7 +703,7 @@ void sym_digits_reserve(SymDigits& d, const CIStrings* s, int set) {
     w.z.reserve((size_t)(s->a.N0 * s->norb * d.chunk));
     w.b.reserve((size_t)(s->a.N1 * nir * d.slots * d.slots));
     w.e.reserve((size_t)(d.ka * d.most * nir * d.chunk));
-    w.ec.reserve((size_t)s->a.N0);
+    w.ec.reserve((size_t)s->a.N0 + 1);
     w.ecol.reserve((size_t)(s->a.N1 * nir * d.slots));
 }
 
@@ -682,7 +737,8 @@ void sym_digits_run(SymDigits& d, const CIStrings* s, int set, const double* V, 
     F2G_CUDA(cudaFuncSetAttribute(k_sy_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, kYSmem));
     for (int v = 0; v < nvec; ++v) {
         const double* x = C + v * N0a * N0b;
-        k_sy_rowexp<<<(unsigned)N0a, 256, 0, st>>>(N0b, x, w.ec.get());
+        F2G_CUDA(cudaMemsetAsync(w.ec.get() + N0a, 0, sizeof(int), st));
+        k_sy_rowexp<<<(unsigned)N0a, 256, 0, st>>>(N0a, N0b, x, w.ec.get());
         F2G_LAUNCH("k_sy_rowexp");
         k_sy_integrals<<<(unsigned)s->a.N1, 256, 0, st>>>(V, n, s->a.m1, s->a.up1.get(), d.os, d.slots, w.ec.get(),
                                                           w.ecol.get(), w.b.get());
@@ -708,6 +764,10 @@ void sym_digits_run(SymDigits& d, const CIStrings* s, int set, const double* V, 
                 F2G_LAUNCH("k_sy_sum");
             }
         }
+        k_sy_not_finite<<<(unsigned)std::min<int64_t>(N0a, sms), 256, 0, st>>>(
+            N0a, N0b, n, s->na, s->nb, s->a.m1, d.os, s->a.down1.get(), s->a.up1.get(), s->b.down1.get(), d.kpos.get(),
+            d.hja.get(), d.jb.get(), d.njb_of.get(), d.njb, d.tab.get(), d.lmax, w.ec.get(), x, V, sig + v * N0a * N0b);
+        F2G_LAUNCH("k_sy_not_finite");
     }
 }
 

@@ -24,7 +24,7 @@ struct SymDigits {
     struct Scratch {
         DevBuf<uint4> z, b;       // digits of the vector and of the integrals
         DevBuf<double> e;
-        DevBuf<int> ec, ecol;     // exponents of the vector's rows; of every output pair of (Ka, t)
+        DevBuf<int> ec, ecol;     // exponents of the vector's rows and a mark behind them; of every output pair of (Ka, t)
     } set[2];                     // direct calls, captured graphs
 };
 
