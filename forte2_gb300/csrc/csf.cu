@@ -335,6 +335,21 @@ struct CsfTiles {
     int64_t conf0[kMaxOrb + 1], nconf[kMaxOrb + 1];
 };
 
+// One CSF's sum over the determinants j0, j0 + step, ... without those it does not contain. The kernels below multiply
+// these by zero, which is not zero for an infinity or NaN: they take a sum that is not finite from here.
+template <typename T>
+__device__ __noinline__ T det_to_csf_skip(const T* O, int nc, const uint32_t* pm, int nd, const T* det, int j0, int step) {
+    T acc = T(0);
+    for (int j = j0; j < nd; j += step) {
+        const T o = O[(int64_t)j * nc];
+        if (o == T(0))
+            continue;
+        const uint32_t e = pm[j];
+        acc += ((e >> 31) ? -o : o) * det[e & 0x7fffffffu];
+    }
+    return acc;
+}
+
 template <typename T, int R>
 __device__ void det_to_csf_tile(const CsfView& v, const uint32_t* __restrict__ conf, int nconf, int N, int i0,
                                 const T* __restrict__ det, T* __restrict__ csf, T* sx, T* so) {
@@ -388,8 +403,11 @@ __device__ void det_to_csf_tile(const CsfView& v, const uint32_t* __restrict__ c
         T* out = csf + v.conf_csf[conf[lane]] + i0 + warp * R;
 #pragma unroll
         for (int r = 0; r < R; ++r)
-            if (warp * R + r < wi)
+            if (warp * R + r < wi) {
+                if (!isfinite(acc[r]))
+                    acc[r] = det_to_csf_skip(O + warp * R + r, nc, v.perm + v.conf_slot[conf[lane]], nd, det, 0, 1);
                 out[r] = acc[r];
+            }
     }
 }
 
@@ -430,6 +448,12 @@ __global__ void __launch_bounds__(256) k_det_to_csf_thin(const __grid_constant__
         double s = 0.0;
         for (int w = 0; w < kTileWarps; ++w)
             s += red[w][lane];
+        if (!isfinite(s)) {
+            s = 0.0;
+            for (int w = 0; w < kTileWarps; ++w) // in the order of the sum above
+                s += det_to_csf_skip(O, nc, pm, nd, det, w, 2 * kTileWarps) +
+                     det_to_csf_skip(O, nc, pm, nd, det, w + kTileWarps, 2 * kTileWarps);
+        }
         csf[v.conf_csf[c] + i] = s;
     }
 }
