@@ -567,8 +567,14 @@ class CISigmaBuilder:
                  "irrep_blocks": 4, "tma_b": 5, "dense_same_spin": 6, "digit_fp64": 7}
 
     def set_variant(self, name, value):
-        """Select a kernel variant with identical results (see forte2_gb300.autotune)."""
+        """Select a kernel variant (see forte2_gb300.autotune); results are the same up to rounding in the
+        norm. digit_fp64 also decides how small elements are carried: the digit kernels (FP64 sigma of C1
+        and of blocked spaces, density matrices) keep 56 to 62 bits below the largest element of a row of
+        the vector. 0 takes the FP64 multiply-add kernels everywhere, 2 returns to the space's default, 1
+        also takes the digits for C1 spaces too small to gain (an error where the sizes rule them out)."""
         check(lib().f2g_sigma_set_variant(self.h, self._VARIANTS[name], int(value)))
+        if name == "digit_fp64":
+            self._digits = bool(value)
 
     def tensor_core_error(self):
         out = np.zeros(1, dtype=np.int32)

@@ -508,7 +508,10 @@ int f2g_sigma_set_variant(void* sb, int which, int value) {
             if (b->use_dense_ss && b->precision == kFP32)
                 b->ensure_fp32();
         } else if (which == 7) {
-            b->set_oz(value != 0);
+            if (value == 2)
+                b->use_oz = true;
+            else
+                b->set_oz(value != 0);
         } else
             throw Error(2, "variant must be 0 (tensor cores), 1 (narrow same-spin tiles), 2 (persistent opposite "
                            "grid), 3 (tensor-core wait limit), 4 (irrep-aware opposite-spin kernel), 5 "

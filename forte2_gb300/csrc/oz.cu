@@ -23,7 +23,10 @@
 // most 2^24, so the FP32 sums are exact (see oz_lead for the bound). Digits and accumulators of neighbouring
 // groups lie next to each other along N, so 11 MMAs do the 28 products of a K step. The epilogue combines
 // the seven sums in a 64-bit integer T (unit: 2^-56 of the largest |a| times the largest |b|). What is
-// dropped (i + j > 6) is a few units: less than the roundings of an FP64 chain of the same length.
+// dropped (i + j > 6) is at most six products of 2^14 in the next group: with the digits' cut, below 2^-53 of the largest
+// |a| times the largest |b| per product (2^-51 with slack in both, see oz_lead). In the norm of a row that is less than
+// the roundings of an FP64 chain (figures below). It is more for an output whose own products are all far below that
+// largest one: a tail of 1e-8 beside a 1 whose integral is zero is left with about half its digits.
 //
 // T goes to memory and a second kernel sums the terms of each sigma element, eight at a time in 64-bit
 // integers aligned at their largest exponent, one conversion to FP64 per eight. One thread per element, list

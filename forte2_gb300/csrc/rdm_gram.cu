@@ -525,6 +525,8 @@ template <int LIST> void gram_launch(const GramArgs& a, int64_t items, int sms, 
 
 bool rdm_gram(SigmaBuilder& sb, GramScratch& g, int spin, int holes, bool inner, const double* CL, const double* CR,
               int64_t d, int64_t ko, int64_t kv, double* out, cudaStream_t st) {
+    if (!sb.use_oz)
+        return false;
     const CIStrings& s = *sb.s;
     SpinStrings& so = sb.s->spin(spin);
     SpinStrings& si = sb.s->spin(1 - spin);

@@ -1432,7 +1432,7 @@ void SigmaBuilder::spmm_blocks(int spin, const double* X, double* Y, bool accumu
 // the opposite-spin term of a space blocked by irreps, on the tensor cores or the FP64 pipe
 void SigmaBuilder::opposite_sym(const double* V, const double* C, double* sig, cudaStream_t st, int nvec, int ctas,
                                 bool graph) {
-    if (symd)
+    if (symd && use_oz)
         sym_digits_run(*symd, s, graph ? 1 : 0, V, C, sig, nvec, ctas, wait_ctl(), st);
     else
         launch_opposite_sym(s, *osym, V, C, sig, st, nvec, ctas);

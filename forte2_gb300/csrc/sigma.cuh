@@ -87,7 +87,8 @@ struct SigmaBuilder {
     void prepare_dense_ss(cudaStream_t st);
     void prepare_graph_fp32(int nvec);
     // FP64 sigma of a C1 space (or of a GAS space's embedding) on the tensor cores by exact digit
-    // splitting (oz.cu), where the sizes allow it and the space is large enough to gain
+    // splitting (oz.cu), where the sizes allow it and the space is large enough to gain. Off: no digit
+    // kernel at all, neither this nor those of blocked spaces (sym_digits.cu) and of the RDMs (rdm_gram.cu)
     bool use_oz = true;
     bool oz_fast = false;
     std::shared_ptr<struct OzSigma> oz;

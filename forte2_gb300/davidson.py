@@ -383,7 +383,8 @@ class DavidsonLiuSolver:
 
         torch = _torch()
         sb, sa, corr = spec
-        key = (sb.h.value, sa.h.value, sb.get_precision(),
+        # (the variants that only choose between equal results stay those of the capture)
+        key = (sb.h.value, sa.h.value, sb.get_precision(), getattr(sb, "_digits", True),
                None if corr is None else tuple(t.data_ptr() for t in corr[:3]) + (corr[3],))
         g = self._graphs.get(key)
         if g is not None and g[1] >= self.maxiter:

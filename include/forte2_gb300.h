@@ -112,9 +112,11 @@ int f2g_sigma_set_tensor_cores(void* sigma, int on, int* available);
  * them in each thread block (the same sigma bits). which = 6: the FP32 same-spin terms as dense
  * tensor-core GEMMs (split FP16, three products; spaces of at most 4096 strings per spin, else
  * error 2; default 1 from 512 strings per spin). which = 7: FP64 sigma on the tensor cores by exact
- * digit splitting (the FP64 kernels' accuracy; up to 16 orbitals, two electrons or more of each
- * spin and at most 146 pairs of holes per string pair, no irreps, else error 2; default 1 from 8,193
- * determinants). No reference counterpart. */
+ * digit splitting (up to 16 orbitals, two electrons or more of each spin and at most 146 pairs of holes
+ * per string pair, no irreps, else error 2; default 1 from 8,193 determinants). 0 turns every digit kernel
+ * off, those of blocked spaces and of the RDMs too; 2 is the default of the space. Their errors are those of
+ * FP64 sums in the norm; elements far below the largest of their row of the vector are carried in fewer than
+ * 53 bits. No reference counterpart. */
 int f2g_sigma_set_variant(void* sigma, int which, int value);
 /* 1 if a tensor-core build (FP32, or FP64 by digit splitting, sigma or RDM) gave up waiting for its matrix
  * operations (results invalid). */
