@@ -512,11 +512,13 @@ int f2g_sigma_set_variant(void* sb, int which, int value) {
                 b->use_oz = true;
             else
                 b->set_oz(value != 0);
+        } else if (which == 8) {
+            b->set_digit_bytes(value);
         } else
             throw Error(2, "variant must be 0 (tensor cores), 1 (narrow same-spin tiles), 2 (persistent opposite "
                            "grid), 3 (tensor-core wait limit), 4 (irrep-aware opposite-spin kernel), 5 "
-                           "(TMA-fed tensor-core B tiles), 6 (FP32 same-spin terms as dense GEMMs) or 7 "
-                           "(FP64 sigma by digit splitting on the tensor cores)");
+                           "(TMA-fed tensor-core B tiles), 6 (FP32 same-spin terms as dense GEMMs), 7 "
+                           "(FP64 sigma by digit splitting on the tensor cores) or 8 (bytes of a digit buffer)");
     });
 }
 

@@ -75,7 +75,6 @@ constexpr int kOzMaxRing = 8;                            // K steps of B in shar
 constexpr uint32_t kOzNone = 0x40000000u;                // list padding: no determinant
 constexpr int kOzMinExp = 64;                            // smallest row/column exponent (denormals count as 0)
 constexpr int kOzBad = 4095;                             // exponent of a row or column that holds an infinity or NaN
-constexpr int64_t kOzElems = int64_t(1) << 28;           // elements of the E buffer (2 GiB)
 
 struct OzShared {
     alignas(8) uint64_t a_full[kOzStages], a_empty[kOzStages];
@@ -1114,12 +1113,13 @@ bool oz_supported(const CIStrings* s, bool* fast) {
 }
 
 void oz_build(const CIStrings* s, std::shared_ptr<OzSigma>& ozp, const double* H, const double* V, double E,
-              cudaStream_t st) {
+              int64_t bytes, cudaStream_t st) {
     const int n = s->norb, P = n * (n - 1) / 2;
     if (!ozp) {
         ozp = std::make_shared<OzSigma>();
         OzSigma& o = *ozp;
         o.s = s;
+        o.max_elems = bytes / (int64_t)sizeof(long long);
         o.lead = oz_lead(std::max({s->a.m1 * s->b.m1, s->a.m2, s->b.m2}));
         for (int sp = 0; sp < 2; ++sp) {
             const SpinStrings& ss = s->spin(sp);
@@ -1176,7 +1176,7 @@ void OzSigma::plan(cudaStream_t st) {
     const int64_t N1a = s->a.N1, N1b = s->b.N1;
     ldE = (N1b + 15) / 16 * 16;
     const int64_t per = (int64_t)s->a.m1 * s->b.m1 * ldE;
-    range_strings = std::max<int64_t>(1, kOzElems / per);
+    range_strings = std::max<int64_t>(1, max_elems / per);
     ranges.clear();
     if (range_strings >= N1a)
         return;
@@ -1201,6 +1201,13 @@ void OzSigma::plan(cudaStream_t st) {
     F2G_CUDA(cudaStreamSynchronize(st));
 }
 
+void oz_limit(OzSigma& o, int64_t bytes, cudaStream_t st) {
+    o.max_elems = bytes / (int64_t)sizeof(long long);
+    for (OzScratch& w : o.scr)
+        w.nvec = 0; // reserved again by the new plan
+    o.plan(st);
+}
+
 void oz_reserve(OzSigma& o, int set, int nvec) {
     OzScratch& w = o.scr[set];
     nvec = std::max(1, nvec);
@@ -1211,7 +1218,7 @@ void oz_reserve(OzSigma& o, int set, int nvec) {
         const SpinStrings& ss = o.s->spin(sp);
         const int64_t ncol = o.s->spin(1 - sp).N0, tiles = (ncol + kOzM - 1) / kOzM * nvec;
         const int64_t per = ss.N2 * ss.m2 * kOzM;
-        const int64_t nt = std::min(tiles, std::max<int64_t>(1, kOzElems / per));
+        const int64_t nt = std::min(tiles, std::max<int64_t>(1, o.max_elems / per));
         e = std::max<size_t>(e, (size_t)(nt * per));
         r = std::max<size_t>(r, (size_t)(nt * kOzM * ss.N2));
     }
@@ -1257,7 +1264,7 @@ void oz_same_spin(OzSigma& o, int set, int spin, const double* C, double* S, int
     OzSpin& t = o.spin[spin];
     OzScratch& w = o.scr[set];
     const int64_t ncol = s->spin(1 - spin).N0, nd = s->nfull, tpv = (ncol + kOzM - 1) / kOzM, tiles = tpv * nvec;
-    const int64_t per = ss.N2 * ss.m2 * kOzM, step = std::min(tiles, std::max<int64_t>(1, kOzElems / per));
+    const int64_t per = ss.N2 * ss.m2 * kOzM, step = std::min(tiles, std::max<int64_t>(1, o.max_elems / per));
     const int np = ss.k * (ss.k - 1) / 2;
     for (int64_t t0 = 0; t0 < tiles; t0 += step) {
         const int64_t nt = std::min(step, tiles - t0), nx = nt * kOzM;

@@ -42,6 +42,7 @@ struct OzSigma {
     DevBuf<int> vexp;         // [n][16] exponent of V[p][r][..][..]
     DevBuf<double> coul;      // [N0a][n] Coulomb energy of beta orbital q with the alpha string
     int64_t ldE = 0;          // opposite spin: elements per E row
+    int64_t max_elems = 0;     // elements of the E buffer
     int64_t range_strings = 0; // alpha one-hole strings whose E fits the buffer
     std::vector<OzRange> ranges; // empty: whole vectors fit
     DevBuf<uint32_t> rows;
@@ -53,9 +54,12 @@ struct OzSigma {
 // The space's sizes fit the digit sums and the tile shapes; `fast` (optional) tells whether it is large
 // enough to gain from it
 bool oz_supported(const CIStrings* s, bool* fast = nullptr);
-// lists of the strings (once), then the digits of the integrals (stream order)
+// lists of the strings (once, with at most `bytes` of E at a time where one tile or one alpha hole string allows it),
+// then the digits of the integrals (stream order)
 void oz_build(const CIStrings* s, std::shared_ptr<OzSigma>& oz, const double* H, const double* V, double E,
-              cudaStream_t st);
+              int64_t bytes, cudaStream_t st);
+// another limit for the E buffers of later calls
+void oz_limit(OzSigma& oz, int64_t bytes, cudaStream_t st);
 // buffers of set 0 (direct calls) or 1 (captured graphs) for calls with up to nvec vectors
 // (never smaller than before)
 void oz_reserve(OzSigma& oz, int set, int nvec);

@@ -78,9 +78,9 @@ struct MixedLists {
 
 // Device scratch of the tensor-core Gram kernel (rdm_gram.cu)
 struct GramScratch {
-    DevBuf<uint4> zl, zr;         // digits of the bra / ket rows, at most kGramBytes each
+    DevBuf<uint4> zl, zr;         // digits of the bra / ket rows, SigmaBuilder::digit_limit() bytes each
     DevBuf<int> el, er;           // their exponents
-    DevBuf<double> part;          // partial results, at most 2^25 elements
+    DevBuf<double> part;          // partial results, 2^25 elements or four results, the larger
     DevBuf<uint32_t> tab[2];      // [orbital][K]: the 1-hole lists of a spin by orbital
 };
 

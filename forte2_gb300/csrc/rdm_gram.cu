@@ -45,7 +45,6 @@ constexpr int kGThreads = (kGProd + kGEpi + 1) * 32;
 constexpr int kGCols = kGM / 4;                   // columns per drain thread at most
 constexpr int kGMaxStages = 8;
 constexpr int kGBad = 0x7ff;                      // exponent of a row that holds an infinity or NaN
-constexpr int64_t kGramBytes = int64_t(1) << 31;  // digits of one vector at a time
 constexpr int kGSmem = 227 * 1024;
 
 struct GramArgs {
@@ -545,13 +544,13 @@ bool rdm_gram(SigmaBuilder& sb, GramScratch& g, int spin, int holes, bool inner,
     // rows: 1,320 and 1,060 us)
     if (!inner && (holes == 1 ? nR < 2048 : (double)m * m * (double)nR < 1.2e5))
         return false;
-    // rows R at a time: digits within kGramBytes, whole drains of 128
+    // rows R at a time: digits of a vector within the limit, whole drains of 128
     const int64_t rows = nI * nv, all8 = (nR + 31) / 32 * 4;
     int64_t k8 = all8;
-    if (rows * 128 * all8 > kGramBytes) {
-        const int64_t most = kGramBytes / (rows * 128) / 16 * 16;
-        if (most < 16)
-            return false;
+    if (rows * 128 * std::min<int64_t>(all8, 16) > int64_t(1) << 31)
+        return false;
+    if (rows * 128 * all8 > sb.digit_limit()) {
+        const int64_t most = std::max<int64_t>(1, sb.digit_limit() / (rows * 128 * 16)) * 16;
         const int64_t parts = (all8 + most - 1) / most;
         k8 = std::min(most, ((all8 + parts - 1) / parts + 15) / 16 * 16);
     }

@@ -606,6 +606,27 @@ void dense_ss_reserve(const CIStrings* s, DenseSameSpin& d, int nvec, int set);
 void dense_ss_term(const CIStrings* s, DenseSameSpin& d, float* sig, int spin, bool accumulate, int nvec, int set,
                    cudaStream_t st);
 
+void SigmaBuilder::set_digit_bytes(int64_t bytes) {
+    if (bytes < 0)
+        throw Error(2, "digit buffer limit must be >= 0");
+    if (bytes == digit_bytes)
+        return;
+    if (*graph_users > 0)
+        throw Error(2, "sigma builder: captured graphs use its scratch; set the digit buffer limit before them");
+    digit_bytes = bytes;
+    if (oz)
+        oz_limit(*oz, digit_limit(), 0);
+    if (symd)
+        sym_digits_plan(*symd, s, digit_limit());
+    if (untimed_nvec > 0) {
+        if (oz)
+            oz_reserve(*oz, 1, untimed_nvec);
+        if (symd)
+            sym_digits_reserve(*symd, s, 1);
+    }
+    F2G_CUDA(cudaStreamSynchronize(0));
+}
+
 // Page-locked words, carved from chunks that stay allocated until the process exits: page-locked allocation
 // synchronises the device, so it happens once per 1,024 builders, not per builder.
 class PinnedWords {
@@ -673,7 +694,7 @@ SigmaBuilder::SigmaBuilder(CIStrings* s_, double E_, const double* H_, const dou
 // in place also while the variant is off, so that it can be turned on again and captured graphs follow.
 void SigmaBuilder::build_oz(cudaStream_t st) {
     if (oz || (oz_fast && use_oz))
-        oz_build(s, oz, dH.get(), dV.get(), E, st);
+        oz_build(s, oz, dH.get(), dV.get(), E, digit_limit(), st);
 }
 
 void SigmaBuilder::set_oz(bool on) {

@@ -95,6 +95,11 @@ struct SigmaBuilder {
     bool oz_path() const { return oz && use_oz; }
     void build_oz(cudaStream_t st);
     void set_oz(bool on); // on: also for spaces too small to gain (an error where the sizes rule it out)
+    // Bytes of a work buffer of the digit kernels: E of oz.cu, digits of a vector and half of E in sym_digits.cu,
+    // digits of a vector in rdm_gram.cu (0: 2 GiB). Larger problems run in parts; no part is smaller than a tile
+    int64_t digit_bytes = 0;
+    int64_t digit_limit() const { return digit_bytes > 0 ? digit_bytes : int64_t(1) << 31; }
+    void set_digit_bytes(int64_t bytes);
     // FP64 sigma of a small C1 space in one launch (small.cu)
     bool use_small = false;
     DevBuf<uint32_t> small_exc[2];

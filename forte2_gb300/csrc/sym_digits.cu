@@ -41,8 +41,7 @@ constexpr int kYThreads = (kYProd + kYEpi + 1) * 32;
 constexpr int kYA = 8 * kYM * 16 * 2;               // digits of a K step's 16 pairs x 128 strings
 constexpr int kYStagesMax = 6;
 constexpr int kYSmem = 216 * 1024;
-constexpr int64_t kYBytes = int64_t(1) << 31;       // digits at a time
-constexpr int64_t kYBytesE = int64_t(1) << 32;      // E at a time
+constexpr int64_t kYBytes = int64_t(1) << 31;       // digits of 128 strings Kb and of the integrals at most
 constexpr int kYUnit = 88 - 68;                     // exponent of the digits' sums, see below
 constexpr int kYBadRow = 1 << 15;                   // with a row's exponent: it holds an infinity or NaN
 constexpr int kYSlow = 1 << 16;                     // with the first exponent of four: some need the general conversion
@@ -669,15 +668,10 @@ std::shared_ptr<SymDigits> sym_digits_build(const CIStrings* s, const OppositeSy
         nj[h] = (int32_t)jb[h].size();
         std::copy(jb[h].begin(), jb[h].end(), flat.begin() + h * d->njb);
     }
-    // positions at a time: the vector's digits within kYBytes; then hole strings Ka at a time: E within kYBytesE
     d->most = (most + 3) / 4 * 4; // stored four at a time
-    const int64_t most128 = kYBytes / (N0a * n * 16 * 128), all128 = d->lmax / 128;
     if (N1a * nir * (int64_t)d->slots * d->slots * 16 > kYBytes)
         return nullptr;
-    const int64_t parts = (all128 + most128 - 1) / most128;
-    d->chunk = (int)((all128 + parts - 1) / parts * 128);
-    const int64_t mostka = std::max<int64_t>(1, kYBytesE / ((int64_t)d->most * nir * d->chunk * 8)), kparts = (N1a + mostka - 1) / mostka;
-    d->ka = (N1a + kparts - 1) / kparts;
+    sym_digits_plan(*d, s, kYBytes);
     auto put = [](auto& buf, const auto& v) {
         buf.reserve(v.size());
         F2G_CUDA(cudaMemcpy(buf.get(), v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice));
@@ -695,6 +689,17 @@ std::shared_ptr<SymDigits> sym_digits_build(const CIStrings* s, const OppositeSy
     F2G_LAUNCH("k_sy_tab");
     F2G_CUDA(cudaStreamSynchronize(0));
     return d;
+}
+
+// positions at a time: the vector's digits within `bytes`; then hole strings Ka at a time: E within twice that
+void sym_digits_plan(SymDigits& d, const CIStrings* s, int64_t bytes) {
+    const int64_t N0a = s->a.N0, N1a = s->a.N1, n = s->norb;
+    const int64_t most128 = std::max<int64_t>(1, bytes / (N0a * n * 16 * 128)), all128 = d.lmax / 128;
+    const int64_t parts = (all128 + most128 - 1) / most128;
+    d.chunk = (int)((all128 + parts - 1) / parts * 128);
+    const int64_t mostka = std::max<int64_t>(1, 2 * bytes / ((int64_t)d.most * d.os.nirrep * d.chunk * 8));
+    const int64_t kparts = (N1a + mostka - 1) / mostka;
+    d.ka = (N1a + kparts - 1) / kparts;
 }
 
 void sym_digits_reserve(SymDigits& d, const CIStrings* s, int set) {

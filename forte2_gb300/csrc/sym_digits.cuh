@@ -30,6 +30,7 @@ struct SymDigits {
 
 // null if the space is left to the FP64 kernel (opposite_sym.cu)
 std::shared_ptr<SymDigits> sym_digits_build(const CIStrings* s, const OppositeSym& t);
+void sym_digits_plan(SymDigits& d, const CIStrings* s, int64_t bytes); // parts for work buffers of that size
 void sym_digits_reserve(SymDigits& d, const CIStrings* s, int set);
 // sigma += the opposite-spin term for nvec C1-embedded vectors back to back
 void sym_digits_run(SymDigits& d, const CIStrings* s, int set, const double* V, const double* C, double* sig, int nvec,

@@ -116,7 +116,8 @@ int f2g_sigma_set_tensor_cores(void* sigma, int on, int* available);
  * per string pair, no irreps, else error 2; default 1 from 8,193 determinants). 0 turns every digit kernel
  * off, those of blocked spaces and of the RDMs too; 2 is the default of the space. Their errors are those of
  * FP64 sums in the norm; elements far below the largest of their row of the vector are carried in fewer than
- * 53 bits. No reference counterpart. */
+ * 53 bits. which = 8: bytes of a work buffer of these kernels (0: 2 GiB); larger problems run in parts, none
+ * smaller than a tile; error 2 once graphs are captured. No reference counterpart. */
 int f2g_sigma_set_variant(void* sigma, int which, int value);
 /* 1 if a tensor-core build (FP32, or FP64 by digit splitting, sigma or RDM) gave up waiting for its matrix
  * operations (results invalid). */
