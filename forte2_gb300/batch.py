@@ -278,13 +278,15 @@ def footprint_bytes(norb: int, na: int, nb: int, nroot: int, basis_per_root: int
     det_vectors = 8 * ndet * (6 + 2 * m)  # C/sigma staging, transposes, closure buffers
     csf = 4 * ndet + 8 * ndet  # permutation + configuration tables (upper bound)
     davidson = 8 * ndet * (3 * m + 2)  # basis, sigma, residual rows (ncsf <= ndet)
-    # FP64 tensor-core sigma (csrc/oz.cu): integrals' digits and two work buffers of at most 2 GiB
+    # FP64 tensor-core sigma (csrc/oz.cu), where its digit sums are exact (oz_lead) and it is used: the
+    # integrals' digits and two work buffers of at most 2 GiB
     oz = 0
-    if norb <= 16 and min(na, nb) >= 2 and ndet > 8192:
-        rows = [comb(norb, k - 2) * comb(norb - k + 2, 2) for k in (na, nb)]
-        need = max(rows[0] * n0b, rows[1] * n0a,
-                   comb(norb, na - 1) * comb(norb, nb - 1) * (norb - na + 1) * (norb - nb + 1))
-        oz = 2 * min(8 * m * need, 2 << 30) + sum(r * 1024 for r in rows)
+    m1a, m1b = norb - na + 1, norb - nb + 1
+    m2 = [comb(norb - k + 2, 2) for k in (na, nb)]
+    if norb <= 16 and min(na, nb) >= 2 and ndet > 8192 and max(m1a * m1b, *m2) <= 146:
+        n2 = [comb(norb, k - 2) for k in (na, nb)]
+        need = max(n2[0] * m2[0] * n0b, n2[1] * m2[1] * n0a, comb(norb, na - 1) * comb(norb, nb - 1) * m1a * m1b)
+        oz = 2 * min(8 * m * need, 2 << 30) + sum(10752 * k * -(-p // 48) * -(-p // 16) for k, p in zip(n2, m2))
     return int(oz + ss + det_vectors + csf + davidson + (64 << 20))
 
 
