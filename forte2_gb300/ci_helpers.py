@@ -571,7 +571,8 @@ class CISigmaBuilder:
         norm. digit_fp64 also decides how small elements are carried: the digit kernels (FP64 sigma of C1
         and of blocked spaces, density matrices) keep 56 to 62 bits below the largest element of a row of
         the vector. 0 takes the FP64 multiply-add kernels everywhere, 2 returns to the space's default, 1
-        also takes the digits for C1 spaces too small to gain (an error where the sizes rule them out)."""
+        also takes the digits for C1 spaces and density matrices too small to gain (an error where the sizes
+        rule out those of C1 sigma)."""
         check(lib().f2g_sigma_set_variant(self.h, self._VARIANTS[name], int(value)))
         if name == "digit_fp64":
             self._digits = bool(value)

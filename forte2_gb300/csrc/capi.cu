@@ -512,6 +512,7 @@ int f2g_sigma_set_variant(void* sb, int which, int value) {
                 b->use_oz = true;
             else
                 b->set_oz(value != 0);
+            b->digits_always = value == 1;
         } else if (which == 8) {
             b->set_digit_bytes(value);
         } else

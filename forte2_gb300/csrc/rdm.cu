@@ -2,9 +2,9 @@
 // the reference's CISigmaBuilder::compute_{a,b,sf}_1rdm (forte2/ci/ci_sigma_builder_1rdm.cc:9-84),
 // compute_{aa,bb,ab,sf}_2rdm and compute_sf_2cumulant (ci_sigma_builder_2rdm.cc:46-282).
 //
-// The mixed-spin blocks and the larger same-spin blocks are formed on the tensor cores (rdm_gram.cu); the FP64
-// kernels of this file take the small same-spin blocks, and mixed blocks whose strings of one spin outnumber that
-// kernel's operand buffer (a million rows; 20 orbitals with 10 and 3 electrons, say).
+// The larger blocks are formed on the tensor cores (rdm_gram.cu, gram_pays); the FP64 kernels of this file take the small
+// ones, 1-RDMs between two vectors where a hole string has few slots, and mixed blocks whose strings of one spin
+// outnumber that kernel's operand buffer (a million rows; 20 orbitals with 10 and 3 electrons, say).
 //
 // Hole-list Gram kernel (1-RDMs, same-spin 2-RDMs). With K a string with one (two) fewer
 // electrons and its hole-list entries (I = K + p (+ q), sign), every element is a sum over K of

@@ -522,6 +522,32 @@ template <int LIST> void gram_launch(const GramArgs& a, int64_t items, int sms, 
 
 } // namespace
 
+// Is this kernel the faster one? Times of a call from Python on the device's vectors, FP64 kernel and this one.
+static bool gram_pays(const CIStrings& s, int spin, int holes, bool inner, bool sym, int m, int64_t nR) {
+    // Same-spin blocks of two and three holes where a K is worth a tile: from m^2 nR = 1.2e5 (1.1e5: 30 and 37 us; 2.0e5:
+    // 73 and 23 us; 3.9e5: 74 and 24 us). One hole, where a K has few slots: from 2,048 rows R (924 rows: 113 and 181 us)
+    // and for one vector from 8 slots (7: 989 and 1,059 us at (14, 8, 6); 8: 1,327 and 1,073 us at (14, 7, 7); 13: 2,067
+    // and 1,006 us at (16, 4, 8)), for two, whose digits are written twice, from 12 (8: 1,333 and 2,071 us; 11: 1,060 and
+    // 1,082 us at (15, 5, 5); 12: 6,896 and 5,725 us at (16, 5, 8)).
+    if (!inner)
+        return holes == 1 ? nR >= 2048 && m >= (sym ? 8 : 12) : (double)m * m * (double)nR >= 1.2e5;
+    // Mixed blocks: the FP64 kernel takes a launch and, for every pair of alpha hole sets, a pass over the beta spin's
+    // pairs per alpha hole string, this one seven launches (ten for two vectors): FP64 where those passes are few. One
+    // hole each: 6 of them 36 and 37 us (one vector, (5, 3, 3)), 7 40 and 38 us, 10 59 and 37 us (6, 4, 3); two vectors
+    // 8 45 and 46 us (9, 8, 7), 9 50 and 45 us, 20 79 and 46 us (7, 4, 3). Two alpha holes, where there are more pairs:
+    // 4 32 and 36 us (6, 3, 3), 5 60 and 42 us (7, 3, 2); two vectors 6 43 and 49 us (8, 7, 4), 53 and 47 us (6, 4, 2). Two
+    // beta holes, longer passes: 4 32 and 37 us (5, 4, 2), 5 42 and 38 us (6, 5, 4); two vectors 5 38 and 50 us, 6 60 and
+    // 52 us (7, 6, 5). A single pass is the whole FP64 kernel, and a single hole string here few blocks' work: (16, 1, 12)
+    // 51 and 396 us, (13, 13, 6) 43 and 49 us.
+    const bool aab = spin == 0 && holes == 2, abb = spin == 1;
+    const int ha = aab ? 2 : 1, hb = abb ? 2 : 1, n = s.norb;
+    const double passes = (double)host_binom(n - ha, s.na - ha);
+    const double ma = (double)host_binom(n - s.na + ha, ha), alpha = host_binom(n, s.na - ha) * ma * ma;
+    const double mb = (double)host_binom(n - s.nb + hb, hb), beta = host_binom(n, s.nb - hb) * mb * mb;
+    const int few = aab ? (sym || alpha > 520 ? 4 : 6) : abb ? (sym ? 4 : 5) : sym ? 6 : 8;
+    return !(passes <= few && alpha <= 800 && passes * beta <= (passes == 1 ? 131072 : 16384));
+}
+
 bool rdm_gram(SigmaBuilder& sb, GramScratch& g, int spin, int holes, bool inner, const double* CL, const double* CR,
               int64_t d, int64_t ko, int64_t kv, double* out, cudaStream_t st) {
     if (!sb.use_oz)
@@ -537,12 +563,7 @@ bool rdm_gram(SigmaBuilder& sb, GramScratch& g, int spin, int holes, bool inner,
     const int nv = inner ? s.norb : 1;
     if (nK == 0 || m == 0 || nR == 0)
         return true;
-    // The mixed blocks always: their FP64 kernel runs one pass over the other spin's pair list per pair of rows,
-    // 51 us against 22 us at (6 orbitals, 3, 3), 56.3 ms against 6.4 ms at (14, 7, 7). Same-spin blocks where a K is
-    // worth a tile: two and three holes from m^2 nR = 1.2e5 (1.1e5: 30 us FP64, 37 us here; 2.0e5: 73 and 23 us;
-    // 3.9e5: 74 and 24 us), one hole, where a K has few slots, from 2,048 rows R (924 rows: 113 and 181 us; 3,432
-    // rows: 1,320 and 1,060 us)
-    if (!inner && (holes == 1 ? nR < 2048 : (double)m * m * (double)nR < 1.2e5))
+    if (!sb.digits_always && !gram_pays(s, spin, holes, inner, CL == CR, m, nR))
         return false;
     // rows R at a time: digits of a vector within the limit, whole drains of 128
     const int64_t rows = nI * nv, all8 = (nR + 31) / 32 * 4;

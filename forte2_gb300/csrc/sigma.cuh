@@ -90,6 +90,7 @@ struct SigmaBuilder {
     // splitting (oz.cu), where the sizes allow it and the space is large enough to gain. Off: no digit
     // kernel at all, neither this nor those of blocked spaces (sym_digits.cu) and of the RDMs (rdm_gram.cu)
     bool use_oz = true;
+    bool digits_always = false; // also where the FP64 kernels are faster (RDMs of small spaces)
     bool oz_fast = false;
     std::shared_ptr<struct OzSigma> oz;
     bool oz_path() const { return oz && use_oz; }

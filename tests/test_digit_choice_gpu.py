@@ -50,10 +50,12 @@ def test_small_elements_of_sigma(cuda, n, na, nb, irreps):
     assert torch.equal(apply(), default)
 
 
-@pytest.mark.parametrize("n,na,nb", [(4, 2, 2), (6, 4, 3), (8, 3, 2), (9, 4, 4), (8, 1, 8)])
-def test_density_matrices_on_the_fp64_kernels(cuda, n, na, nb):
+@pytest.mark.parametrize("n,na,nb,digits", [(4, 2, 2, 0), (6, 4, 3, 0), (8, 3, 2, 0), (9, 4, 4, 0), (8, 1, 8, 0),
+                                            (4, 2, 2, 1), (5, 4, 2, 1), (8, 7, 2, 1),  # too small to gain
+                                            (6, 5, 2, 2), (7, 6, 3, 2), (8, 8, 3, 2)])  # by block
+def test_density_matrices(cuda, n, na, nb, digits):
     s, sb = builder(n, na, nb)
-    sb.set_variant("digit_fp64", 0)
+    sb.set_variant("digit_fp64", digits)
     x, y = random_ci_vector(s.ndet, 1), random_ci_vector(s.ndet, 2)
     for kind, (spin, h, inner) in kinds(n, na, nb).items():
         k, kin = (na, nb) if spin == 0 else (nb, na)
