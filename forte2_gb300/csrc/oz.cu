@@ -1106,9 +1106,17 @@ bool oz_supported(const CIStrings* s, bool* fast) {
         return false;
     if (oz_lead(std::max({s->a.m1 * s->b.m1, s->a.m2, s->b.m2})) < 0)
         return false;
-    if (fast)
-        *fast = s->nfull > 8192; // below it one launch of small.cu: 4,900 determinants 29 us (89 us here),
-                                 // 15,876 determinants 102 us (90 us), four vectors 324 us (113 us)
+    if (fast) {
+        // Up to 8,192 determinants one launch of small.cu: 4,900 determinants 29 us (89 us here), 15,876 determinants 102
+        // us (90 us), four vectors 324 us (113 us). A beta spin with two or three holes leaves 3 or 4 of the 16 places of a
+        // K step and a column block in use; where the alpha spin too has few electrons or holes, the FP64 kernels are
+        // faster: (14, 2, 12) 113 and 181 us, (16, 14, 14) 292 and 357 us, (13, 10, 11) 270 and 313 us, but 329 and 262
+        // us with the 33,124 determinants of (14, 3, 12); three holes: (11, 2, 8) 110 and 135 us, (12, 2, 9) 138 and 148
+        // us (282 and 218 us for four vectors). With four electrons or holes of alpha: (10, 4, 8) 132 and 119 us.
+        const int few = std::min(na, n - na), holes = n - nb;
+        const bool sparse = few >= 2 && few <= 3 && (holes == 2 || holes == 3);
+        *fast = s->nfull > (!sparse ? 8192 : holes == 2 ? 24000 : 10000);
+    }
     return true;
 }
 

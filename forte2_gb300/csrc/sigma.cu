@@ -683,7 +683,7 @@ SigmaBuilder::SigmaBuilder(CIStrings* s_, double E_, const double* H_, const dou
     use_dense_ss = dense_ss_supported() && std::max(s->a.N0, s->b.N0) >= kDenseSsMinStrings;
     if (!osym)
         oz_supported(s, &oz_fast);
-    if (!oz_fast && !s->blocked() && small_supported(s)) {
+    if (!oz_fast && s->nfull <= 8192 && !s->blocked() && small_supported(s)) {
         use_small = true;
         small_lists(s, small_exc, 0); // ordered before set_hamiltonian's wait on the legacy stream
     }

@@ -113,7 +113,8 @@ int f2g_sigma_set_tensor_cores(void* sigma, int on, int* available);
  * tensor-core GEMMs (split FP16, three products; spaces of at most 4096 strings per spin, else
  * error 2; default 1 from 512 strings per spin). which = 7: FP64 sigma on the tensor cores by exact
  * digit splitting (up to 16 orbitals, two electrons or more of each spin and at most 146 pairs of holes
- * per string pair, no irreps, else error 2; default 1 from 8,193 determinants). 0 turns every digit kernel
+ * per string pair, no irreps, else error 2; default 1 from 8,193 determinants, 10,001 or 24,001 where both
+ * spins have two or three holes or electrons). 0 turns every digit kernel
  * off, those of blocked spaces and of the RDMs too; 2 is the default of the space. Their errors are those of
  * FP64 sums in the norm; elements far below the largest of their row of the vector are carried in fewer than
  * 53 bits. which = 8: bytes of a work buffer of these kernels (0: 2 GiB); larger problems run in parts, none

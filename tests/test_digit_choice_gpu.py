@@ -90,3 +90,18 @@ def test_a_kept_solver_captures_its_iterations_again(cuda):
     solver.run()
     assert len(solver.eigensolver._graphs) == 2
     assert abs(float(solver.evals[0]) - first) < 1e-9
+
+
+@pytest.mark.parametrize("n,na,nb,fast", [(11, 2, 8, False), (12, 2, 9, True), (14, 2, 12, False), (13, 10, 11, False),
+                                          (14, 3, 12, True), (10, 4, 8, True), (12, 11, 7, True)])
+def test_default_kernels_of_spaces_with_few_beta_holes(cuda, n, na, nb, fast):
+    torch = cuda
+    s, sb = builder(n, na, nb)
+    c = torch.as_tensor(random_ci_vector(s.ndet, 3), device="cuda")
+    got = {}
+    for digits in (2, 0, 1):
+        sb.set_variant("digit_fp64", digits)
+        got[digits] = torch.empty_like(c)
+        sb.Hamiltonian(c, got[digits])
+    assert torch.equal(got[2], got[1 if fast else 0])
+    assert torch.linalg.vector_norm(got[1] - got[0]) <= 1e-13 * torch.linalg.vector_norm(got[0])
