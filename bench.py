@@ -34,6 +34,7 @@ import numpy as np
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
+from forte2_gb300.batch import uses_digits  # noqa: E402
 from forte2_gb300.synthetic import cas_dims, hz_flops, make_integrals, random_ci_vector, sparse_flops  # noqa: E402
 
 NORB, NEL = 16, 16
@@ -271,17 +272,21 @@ def count_launches(fn):
 def digit_opposite_roofline(norb, na, nb, seconds, fp64_flops, fp64_peak):
     """Opposite-spin phase of the FP64 sigma on the tensor cores (csrc/oz.cu): per alpha hole string,
     128 beta hole strings and K step of one annihilated orbital (16 beta orbitals), 28 digit products
-    of M = 128, N = 48 per three created orbitals. The phase also forms the row exponents and adds
-    the products' 64-bit integers into sigma (each written and read once: the traffic given)."""
+    of M = 128, N = 48 per three created orbitals. `achieved` counts the products of orbital pairs that
+    exist (the kernel works on 16 beta orbitals, whatever the beta holes, and on whole tiles: `issued_*`
+    count those too). The phase also forms the row exponents and adds the products' 64-bit integers into
+    sigma (each written and read once: the traffic given)."""
     from math import comb
 
     ma, mb = norb - na + 1, norb - nb + 1
     n1a, n1b = comb(norb, na - 1), comb(norb, nb - 1)
-    flop = n1a * ((n1b + 127) // 128) * ma * ((ma + 2) // 3) * 28 * 2 * 128 * 48 * 16
+    flop = n1a * n1b * (ma * mb) ** 2 * 28 * 2
+    issued = n1a * ((n1b + 127) // 128) * ma * ((ma + 2) // 3) * 28 * 2 * 128 * 48 * 16
     peak = _measured_peaks().get("bf16_tflops", 1900.0)
     return {"bound": "tensor", "kernel": "k_oz (opposite-spin sigma in FP16 digits) and its sums",
             "achieved": flop / seconds / 1e12, "peak": peak, "unit": "TFLOP/s", "frac": flop / seconds / 1e12 / peak,
             "peak_source": "MEASURED_PEAKS.json bf16_tflops (dense FP16 runs at the BF16 rate)",
+            "issued_flop": issued, "issued_frac": issued / seconds / 1e12 / peak,
             "flop_per_launch": flop, "launch_ms": 1e3 * seconds, "traffic": 16 * n1a * n1b * ma * mb,
             "traffic_source": "algorithmic: 8 B written and read per hole pair and created orbital pair",
             "fp64_flops": fp64_flops, "fp64_equivalent_tflops": fp64_flops / seconds / 1e12, "fp64_peak": fp64_peak}
@@ -392,13 +397,13 @@ def run_gb300(a):
         v, sample, cores = cpu_baseline(a.norb, a.cpu_seconds, na, nb, ints, c_host)
         cpu = {"value": v, "unit": "sigma-builds/s", "cores": cores, "kind": "port", "sample": sample}
     if rank == 0:
-        digits = a.norb <= 16 and min(na, nb) >= 2 and ndet > 8192
-        if digits:
+        if uses_digits(a.norb, na, nb):
             roofline = digit_opposite_roofline(a.norb, na, nb, t_ab, f_sp["ab"], peak64)
         else:
             roofline = {
                 "bound": "compute", "pipe": "fp64",
-                "kernel": "k_opposite (opposite-spin sigma)" if a.norb > 16 or ndet > 8192 else "k_small_sigma (all terms)",
+                "kernel": "k_small_sigma (all terms)" if ndet <= 8192 and 8 * (ndet + a.norb ** 4) <= 200 * 1024
+                  else "k_opposite (opposite-spin sigma)",
                 "achieved": achieved, "peak": peak64, "unit": "TFLOP/s",
                 "frac": achieved / peak64, "traffic": opposite_traffic(a.norb, na, nb),
                 "traffic_source": "dram read+write per gathered C element of the ncu capture at "
@@ -744,7 +749,7 @@ def run_rdm(a):
     beta_all = comb(n, nb - 1) * (n - nb + 1) ** 2
     ab_flop = 2.0 * alpha_sym * beta_all
     slots = (n - na + 1) * n
-    tiles = (slots + 127) // 128
+    tiles = 1 if slots <= 128 else (slots + 111) // 112
     nt = ((slots + tiles - 1) // tiles + 15) // 16 * 16
     mma_flop = (comb(n, na - 1) * (tiles * (tiles + 1) // 2) * ((comb(n, nb - 1) + 15) // 16)
                 * 36 * 2 * 128 * nt * 16)

@@ -264,6 +264,18 @@ def make_solver(inst, precision="fp64", e_tol=1e-10, maxiter=2000, autotune=True
                        sigma_variants=sigma_variants)
 
 
+def uses_digits(norb: int, na: int, nb: int) -> bool:
+    """Whether the FP64 sigma of a C1 space runs in digits on the tensor cores by default (csrc/oz.cu,
+    oz_supported: the digit sums are exact, and the space is large enough to gain)."""
+    if norb > 16 or min(na, nb) < 2 or max(na, nb) > norb:
+        return False
+    nonzero = max((norb - na + 1) * (norb - nb + 1), comb(norb - na + 2, 2), comb(norb - nb + 2, 2))
+    holes = norb - nb
+    sparse = holes in (2, 3) and min(na, norb - na) in (2, 3)
+    least = 8192 if not sparse else 24000 if holes == 2 else 10000
+    return nonzero <= 146 and comb(norb, na) * comb(norb, nb) > least
+
+
 def footprint_bytes(norb: int, na: int, nb: int, nroot: int, basis_per_root: int = 0) -> int:
     """Estimated device bytes of one CASCI solve (vectors, scratch, string Hamiltonian, CSF maps);
     basis_per_root 0 = the subspace make_solver gives this space."""
@@ -278,12 +290,11 @@ def footprint_bytes(norb: int, na: int, nb: int, nroot: int, basis_per_root: int
     det_vectors = 8 * ndet * (6 + 2 * m)  # C/sigma staging, transposes, closure buffers
     csf = 4 * ndet + 8 * ndet  # permutation + configuration tables (upper bound)
     davidson = 8 * ndet * (3 * m + 2)  # basis, sigma, residual rows (ncsf <= ndet)
-    # FP64 tensor-core sigma (csrc/oz.cu), where its digit sums are exact (oz_lead) and it is used: the
-    # integrals' digits and two work buffers of at most 2 GiB
+    # FP64 tensor-core sigma (csrc/oz.cu): the integrals' digits and two work buffers of at most 2 GiB
     oz = 0
-    m1a, m1b = norb - na + 1, norb - nb + 1
-    m2 = [comb(norb - k + 2, 2) for k in (na, nb)]
-    if norb <= 16 and min(na, nb) >= 2 and ndet > 8192 and max(m1a * m1b, *m2) <= 146:
+    if uses_digits(norb, na, nb):
+        m1a, m1b = norb - na + 1, norb - nb + 1
+        m2 = [comb(norb - k + 2, 2) for k in (na, nb)]
         n2 = [comb(norb, k - 2) for k in (na, nb)]
         need = max(n2[0] * m2[0] * n0b, n2[1] * m2[1] * n0a, comb(norb, na - 1) * comb(norb, nb - 1) * m1a * m1b)
         oz = 2 * min(8 * m * need, 2 << 30) + sum(10752 * k * -(-p // 48) * -(-p // 16) for k, p in zip(n2, m2))

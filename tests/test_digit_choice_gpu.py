@@ -5,6 +5,7 @@ from itertools import combinations
 import numpy as np
 import pytest
 
+from forte2_gb300.batch import uses_digits
 from forte2_gb300.synthetic import make_integrals, random_ci_vector, symmetrize_integrals
 from test_rdm_gram_gpu import gram, kinds, strings
 
@@ -104,4 +105,5 @@ def test_default_kernels_of_spaces_with_few_beta_holes(cuda, n, na, nb, fast):
         got[digits] = torch.empty_like(c)
         sb.Hamiltonian(c, got[digits])
     assert torch.equal(got[2], got[1 if fast else 0])
+    assert uses_digits(n, na, nb) == fast
     assert torch.linalg.vector_norm(got[1] - got[0]) <= 1e-13 * torch.linalg.vector_norm(got[0])
