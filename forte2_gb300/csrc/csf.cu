@@ -804,6 +804,7 @@ SpinAdapter::SpinAdapter(const CIStrings* s_, int twoS_, int twoMs_)
 // 32, 48 or 64, the smallest that gives the fewest tiles. The groups of k_det_to_csf_thin (FP64, a chain of
 // more than 64 determinants and fewer tiles than two per SM) go to `thin`: at CAS(14,14) 2.13 -> 0.76 ms.
 // FP32 sums keep the order of the determinants, and their chain costs little: no thin groups.
+constexpr int kSms = 152;
 static void tiles_of(const SpinAdapter& a, CsfTiles& t, CsfTiles* thin) {
     t.block0[0] = 0;
     if (thin)
@@ -818,7 +819,7 @@ static void tiles_of(const SpinAdapter& a, CsfTiles& t, CsfTiles* thin) {
             if (r * kTileWarps * tiles >= a.ncsfN[N])
                 R = r;
         const int64_t rows = (nc + kTileConf - 1) / kTileConf;
-        const bool is_thin = thin && a.ndetN[N] > 64 && rows * tiles < 304;
+        const bool is_thin = thin && a.ndetN[N] > 64 && rows * tiles < 2 * kSms;
         CsfTiles& o = is_thin ? *thin : t;
         o.N[o.n] = N;
         o.R[o.n] = R;

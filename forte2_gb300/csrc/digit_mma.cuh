@@ -1,5 +1,6 @@
-// What the kernels that multiply digits on the tensor cores share (oz.cu, rdm_gram.cu, sym_digits.cu): tcgen05, mbarrier and
-// copy instructions, and the conversion of exact 64-bit sums of digit products to FP64.
+// What the kernels that multiply digits on the tensor cores share (oz.cu, rdm_gram.cu, sym_digits.cu; opposite_tc.cu uses
+// the instructions): tcgen05, mbarrier and copy instructions, and the conversion of exact 64-bit sums of digit products
+// to FP64.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -13,6 +14,8 @@ namespace f2g {
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
+// tcgen05 shared-memory matrix descriptor: start >> 4 [0,14), leading byte offset >> 4 [16,30), stride byte offset >> 4
+// [32,46), version 1 [46,48), base offset 0, no swizzle [61,64) = 0
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
     return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);

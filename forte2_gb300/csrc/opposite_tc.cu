@@ -56,6 +56,7 @@
 #include <mutex>
 #include <string>
 
+#include "digit_mma.cuh"
 #include "sigma.cuh"
 
 namespace f2g {
@@ -71,22 +72,11 @@ constexpr int kTcN = 256;      // 16 values of s x 16 values of r
 constexpr int kTcMaxK = 80;    // padded alpha-excitation count (na * (n - na + 1) <= 72 for n <= 16)
 constexpr int kTcCols = 512;   // tensor-memory columns allocated: two 256-column accumulators
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
 // byte offset of element (row, k) in a K-major, no-swizzle 16-bit operand of kp columns: core
 // matrices of 8 rows x 8 FP16 (16 B per row, 128 B each); adjacent core matrices along K are 128 B
 // apart (leading byte offset), along rows (kp / 8) * 128 B apart (stride byte offset)
 __device__ __forceinline__ uint32_t kmajor_off(int row, int k, int kp) {
     return (uint32_t)(((row >> 3) * (kp >> 3) + (k >> 3)) * 128 + (row & 7) * 16 + (k & 7) * 2);
-}
-
-// tcgen05 shared-memory matrix descriptor: start >> 4 [0,14), leading byte offset >> 4 [16,30),
-// stride byte offset >> 4 [32,46), version 1 [46,48), base offset 0, no swizzle [61,64) = 0
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
 // instruction descriptor, kind::f16: D F32 [4,6) = 1, A F16 [7,10) = 0, B F16 [10,13) = 0, both
@@ -103,14 +93,6 @@ __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t da, uint64_t d
 __device__ __forceinline__ void mma_commit(uint32_t mbar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
                  : "memory");
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
 }
 
 // bounded wait for the phase `parity` of an mbarrier; returns false if it gave up after `limit` polls.
@@ -150,8 +132,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
                    "=r"(r[15])
                  : "r"(taddr));
 }
-
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // 2^e as a float for -126 <= e <= 127
 __device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }

@@ -42,7 +42,7 @@
 //
 // Bound and figures (one GB300, 2.0 GHz): sigma at CAS(16,16) 1974 ms with the FP64 kernels, 240 ms here
 // (opposite spin 1510 -> 169 ms, same spin 230 -> 34 and 37 ms); CAS(14,14) 87.3 -> 14.3 ms; errors against
-// 64-bit torch 6.4e-16 -> 4.7e-16 there. k_oz is bound by instruction issue (integer ALU 50-60 %: digits,
+// 64-bit torch 6.5e-16 -> 3.5e-16 of the norm in its CSF closure. k_oz is bound by instruction issue (integer ALU 50-60 %: digits,
 // read-out), the tensor pipe is 50 % busy in the opposite-spin term, 25 % in the same-spin terms. Kept: A
 // from tensor memory (an MMA of N = 48 then takes N / 2 clocks; from shared memory 44); a chunk of 48
 // columns (7 accumulators and 3 stages fill the 512 columns).
@@ -65,7 +65,8 @@ constexpr int kOzM = 128;             // rows per tile
 constexpr int kOzStages = 3;          // A stages in tensor memory
 constexpr int kOzStageCols = kOzS * 8; // 16 halves = 8 columns per digit
 constexpr int kOzProd = 8, kOzEpi = 8;
-constexpr int kOzThreads = 20 * 32;    // 8 producer and 8 epilogue warps, MMA issue, B loads (registers come in units of 4 warps)
+// 8 producer and 8 epilogue warps, MMA issue, B loads (registers come in units of 4 warps)
+constexpr int kOzThreads = 20 * 32;
 constexpr int kOzSub = 16 * 16 * 2;                      // one digit of 16 columns x 16 K
 constexpr int kOzBlockBytes = kOzSub * kOzS;             // 16 columns x 16 K x 7 digits
 constexpr int kOzDigitBytes = 3 * kOzSub;                // one digit of a K step of a 48-column chunk
@@ -990,7 +991,9 @@ template <int DIGIT> __device__ __forceinline__ void oz_store8(const double (&x)
         const unsigned long long u = (unsigned long long)__double_as_longlong(x[j]);
         y[j] = oz_digits((uint32_t)(u >> 32), (uint32_t)u, e);
     }
-#define F2G_OZ_ROW(I)                                                                                                     *reinterpret_cast<uint4*>(dst + I * DIGIT) = make_uint4(oz_half2<I>(y[0], y[1]), oz_half2<I>(y[2], y[3]),                                                                     oz_half2<I>(y[4], y[5]), oz_half2<I>(y[6], y[7]));
+#define F2G_OZ_ROW(I)                                                                                                 \
+    *reinterpret_cast<uint4*>(dst + I * DIGIT) = make_uint4(oz_half2<I>(y[0], y[1]), oz_half2<I>(y[2], y[3]),         \
+                                                            oz_half2<I>(y[4], y[5]), oz_half2<I>(y[6], y[7]));
     F2G_OZ_ROW(0)
     F2G_OZ_ROW(1)
     F2G_OZ_ROW(2)
@@ -1250,7 +1253,7 @@ static void oz_launch(OzArgs& a, int64_t nk, int64_t tiles, int max_ctas, cudaSt
     const int sms = oz_sms();
     const int64_t room = 227 * 1024 - 1024;
     a.nt = (int)tiles;
-    // the integers of a tile's D are kept for all its chunks while they and four K steps of B fit
+    // the integers of a tile's D are kept for all its chunks while they and three K steps of B fit
     a.reuse = !SS && (int64_t)a.ksteps * kOzYBytes + 3 * kOzStepBytes <= room;
     const int64_t ybytes = SS ? 0 : (int64_t)(a.reuse ? a.ksteps : 2) * kOzYBytes;
     a.nbuf = (int)std::min<int64_t>(SS ? 6 : kOzMaxRing, (room - ybytes) / kOzStepBytes);
@@ -1316,12 +1319,14 @@ static void oz_sum_ab(const OzSigma& o, const OzScratch& w, const uint32_t* rows
                       int64_t x1, double* S, const WaitCtl& wait, cudaStream_t st) {
     const CIStrings* s = o.s;
     k_oz_sum_ab<NB><<<dim3((unsigned)nrows, (unsigned)ceil_div(s->b.N0, 256)), 256, 0, st>>>(
-        w.E.get(), w.rexp.get(), o.ldE, s->a.m1, s->b.m1, s->na, s->nb, s->norb, o.vexp.get(), rows, v0, s->a.N0, s->b.N0, s->a.N1, x0, x1,
+        w.E.get(), w.rexp.get(), o.ldE, s->a.m1, s->b.m1, s->na, s->nb, s->norb, o.vexp.get(), rows, v0, s->a.N0,
+        s->b.N0, s->a.N1, x0, x1,
         s->a.down1.get(), s->b.down1.get(), s->a.str.get(), S, wait);
     F2G_LAUNCH("k_oz_sum_ab");
 }
 
-void oz_opposite(OzSigma& o, int set, const double* C, double* S, int nvec, int max_ctas, const WaitCtl& wait, cudaStream_t st) {
+void oz_opposite(OzSigma& o, int set, const double* C, double* S, int nvec, int max_ctas, const WaitCtl& wait,
+                 cudaStream_t st) {
     const CIStrings* s = o.s;
     OzScratch& w = o.scr[set];
     const int64_t N1a = s->a.N1, N1b = s->b.N1, N0b = s->b.N0;

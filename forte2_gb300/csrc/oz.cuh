@@ -67,6 +67,7 @@ void oz_reserve(OzSigma& oz, int set, int nvec);
 void oz_diag(const OzSigma& oz, const double* C, double* S, int nvec, cudaStream_t st);
 void oz_same_spin(OzSigma& oz, int set, int spin, const double* C, double* S, int nvec, int max_ctas, const WaitCtl& wait,
                   cudaStream_t st);
-void oz_opposite(OzSigma& oz, int set, const double* C, double* S, int nvec, int max_ctas, const WaitCtl& wait, cudaStream_t st);
+void oz_opposite(OzSigma& oz, int set, const double* C, double* S, int nvec, int max_ctas, const WaitCtl& wait,
+                 cudaStream_t st);
 
 } // namespace f2g

@@ -9,8 +9,7 @@
 //
 // Arithmetic. A source row is scaled by its largest exponent to integers of 62 bits and cut into eight signed digits
 // of base 256, which are exact FP16 numbers. Products of digits i and j belong to group i + j; the groups 0..7 are
-// kept (the next one is 2^-64 of the row maxima, so that rows with one large and many small elements lose nothing
-// that FP64 sums would keep). A group's sum over 128 rows (256 for groups 0..3, which have half the products) is an
+// kept. A group's sum over 128 rows (256 for groups 0..3, which have half the products) is an
 // integer below 2^24: exact in the FP32 accumulators. Then it is added into a 64-bit integer in a register, so a
 // K's whole sum is exact; it is rounded once per K and added in FP64.
 //
@@ -26,8 +25,11 @@
 // refilled in turn, so that the MMAs of one overlap with the drain of the other (as one piece 6.64 ms, so 5.75 ms).
 // Rows of a digit lie 64 bytes together in shared memory (64-byte swizzle): with unswizzled core matrices, 16 bytes
 // together, every 16-byte copy was a wavefront of its own and the copies bound the kernel (7.75 ms, then 6.64). One
-// vector, FP64 kernels -> this file: mixed block 56.3 -> 6.4 ms, same spin 8.5 -> 1.7 ms and 1-RDM 1.32 -> 1.06 ms per
-// spin; CAS(10,10) mixed 3-RDM block 1,394 -> 129 us, same-spin 3-RDM 139 -> 30 us.
+// vector, FP64 kernels -> this file: mixed block 56.4 -> 6.5 ms, same spin 8.5 -> 1.7 ms and 1-RDM 1.33 -> 1.08 ms per
+// spin; CAS(10,10) mixed 3-RDM block 1,406 -> 142 us, same-spin 3-RDM 146 -> 47 us (whole calls).
+//
+// Accuracy: a product loses less than 2^-58 of the product of its two source rows' largest elements (2^-63 of each from
+// the digits' cut, at most 2^-59 from the groups left out).
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -640,7 +642,8 @@ bool rdm_gram(SigmaBuilder& sb, GramScratch& g, int spin, int holes, bool inner,
                      (sym && a.ntile == 1 ? 8192 : 0); // a tile's last digits are read as 128 rows of 64 bytes; behind the
                                                        // first of two operands lies the second
     static_assert(kGSmem - (sizeof(GramShared) + 1023) / 1024 * 1024 >= 2 * 2 * 112 * 512);
-    // stages as large as leave two (seven of one K step: same spin 1.99 against 1.73 ms without drains); spt double K steps of 8 digits (twice that of 4), a divisor of per_lo
+    // stages as large as leave two (seven of one K step: same spin 1.99 against 1.73 ms without drains); spt double
+    // K steps of 8 digits (twice that of 4), a divisor of per_lo
     a.spt = a.per_lo;
     while (a.spt > 1 && 2 * a.spt * a.stage_bytes > ring)
         a.spt /= 2;

@@ -61,6 +61,7 @@ __device__ inline int s2neg(uint64_t X, int hi, int lo) {
 // q > s), all indices ascending, the last fastest. (A thread per string took 285 us for the 70 strings of
 // (8e,8o), a chain of 53 entries each, whatever the number of strings.)
 constexpr int kBuildSsThreads = 128;
+unsigned build_ss_grid(int64_t N0) { return (unsigned)std::min<int64_t>(N0, 1 << 20); }
 template <typename T>
 __global__ void __launch_bounds__(kBuildSsThreads)
     k_build_ss(int n, int k, int64_t N0, int nnz, const uint64_t* str, const uint64_t* binom, const double* h,
@@ -787,9 +788,9 @@ void SigmaBuilder::build_string_hamiltonian(int spin, StringHamiltonian& sh, boo
     if (!s->blocked()) {
         sh.col.reserve(total);
         sh.val.reserve(total);
-        k_build_ss<double><<<(unsigned)std::min<int64_t>(ss.N0, 1 << 20), kBuildSsThreads, 0, st>>>(n, ss.k, ss.N0, nnz_full, ss.str.get(),
-                                                                s->binom.get(), dH.get(), dV.get(), with_e0 ? E : 0.0,
-                                                                3, sh.col.get(), sh.val.get());
+        k_build_ss<double><<<build_ss_grid(ss.N0), kBuildSsThreads, 0, st>>>(
+            n, ss.k, ss.N0, nnz_full, ss.str.get(), s->binom.get(), dH.get(), dV.get(), with_e0 ? E : 0.0, 3,
+            sh.col.get(), sh.val.get());
         F2G_LAUNCH("k_build_ss");
         return;
     }
@@ -797,9 +798,9 @@ void SigmaBuilder::build_string_hamiltonian(int spin, StringHamiltonian& sh, boo
     // (a symmetric space keeps about 1/nirrep of them); the layout depends on the strings alone
     TmpBuf<int32_t> fc(total, st);
     TmpBuf<double> fv(total, st);
-    k_build_ss<double><<<(unsigned)std::min<int64_t>(ss.N0, 1 << 20), kBuildSsThreads, 0, st>>>(n, ss.k, ss.N0, nnz_full, ss.str.get(), s->binom.get(),
-                                                            dH.get(), dV.get(), with_e0 ? E : 0.0, 3, fc.get(),
-                                                            fv.get());
+    k_build_ss<double><<<build_ss_grid(ss.N0), kBuildSsThreads, 0, st>>>(
+        n, ss.k, ss.N0, nnz_full, ss.str.get(), s->binom.get(), dH.get(), dV.get(), with_e0 ? E : 0.0, 3, fc.get(),
+        fv.get());
     F2G_LAUNCH("k_build_ss");
     const DetBlocks& B = s->blocks;
     if (ss_nnz_filtered[spin] < 0) {
@@ -849,7 +850,8 @@ void build_ss_values(int n, int k, int64_t N0, int nnz, const uint64_t* str, con
                      const double* V, double e0, int32_t* col, double* val, cudaStream_t st) {
     if (N0 == 0 || nnz == 0)
         return;
-    k_build_ss<double><<<(unsigned)std::min<int64_t>(N0, 1 << 20), kBuildSsThreads, 0, st>>>(n, k, N0, nnz, str, binom, h, V, e0, 3, col, val);
+    k_build_ss<double><<<build_ss_grid(N0), kBuildSsThreads, 0, st>>>(n, k, N0, nnz, str, binom, h, V, e0, 3, col,
+                                                                      val);
     F2G_LAUNCH("k_build_ss");
 }
 
@@ -1679,9 +1681,9 @@ void SigmaBuilder::term_c1(int which, const double* C, double* sigma, cudaStream
     const size_t total = (size_t)ss.N0 * tmp.nnz;
     tmp.col.reserve(total);
     tmp.val.reserve(total);
-    k_build_ss<double><<<(unsigned)std::min<int64_t>(ss.N0, 1 << 20), kBuildSsThreads, 0, st>>>(n, ss.k, ss.N0, tmp.nnz, ss.str.get(), s->binom.get(),
-                                                            dH.get(), dV.get(), 0.0, parts, tmp.col.get(),
-                                                            tmp.val.get());
+    k_build_ss<double><<<build_ss_grid(ss.N0), kBuildSsThreads, 0, st>>>(
+        n, ss.k, ss.N0, tmp.nnz, ss.str.get(), s->binom.get(), dH.get(), dV.get(), 0.0, parts, tmp.col.get(),
+        tmp.val.get());
     F2G_LAUNCH("k_build_ss term");
     const int64_t NA = s->a.N0, NB = s->b.N0;
     if (spin == 0) {

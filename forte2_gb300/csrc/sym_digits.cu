@@ -43,9 +43,9 @@ constexpr int kYStagesMax = 6;
 constexpr int kYSmem = 216 * 1024;
 constexpr int64_t kYBytes = int64_t(1) << 31;       // digits of 128 strings Kb and of the integrals at most
 constexpr int kYUnit = 88 - 68;                     // exponent of the digits' sums, see below
-constexpr int kYBadRow = 1 << 15;                   // with a row's exponent: it holds an infinity or NaN
-constexpr int kYSlow = 1 << 16;                     // with the first exponent of four: some need the general conversion
-constexpr int kYBad = 1 << 14;                       // exponent of an output pair with an integral that is not finite
+constexpr int kYBadRow = 1 << 15; // with a row's exponent: it holds an infinity or NaN
+constexpr int kYSlow = 1 << 16; // with the first exponent of four: some need the general conversion
+constexpr int kYBad = 1 << 14;    // exponent of an output pair with an integral that is not finite
 
 struct SymShared {
     alignas(8) uint64_t full[kYStagesMax], empty[kYStagesMax], acc_full[4], acc_empty[4], drain;
@@ -644,9 +644,8 @@ std::shared_ptr<SymDigits> sym_digits_build(const CIStrings* s, const OppositeSy
             most = std::max(most, c);
         }
     }
-    // Below some 2e7 products the FP64 kernel's one launch is the faster one: (10 orbitals, 5, 5) in 8, 4 and 2 irreps
-    // (5e6, 1.4e7 and 4e7) sigma 292, 246, 295 us, here 327, 259, 212 us, (12, 6, 6) in 8 (1.2e8) 829 and 546 us, all
-    // with one launch per block of the same-spin terms (now 113, 148, 167 and 331 us by this line)
+    // Below some 2e7 products the FP64 kernel's one launch is the faster one: sigma of (10 orbitals, 5, 5) in 8 and 4 irreps
+    // (5e6 and 1.4e7 products) 35 and 13 us faster, in 2 (4e7) 246 and 162 us, of (12, 6, 6) in 8 (1.2e8) 637 and 341 us
     if (most > kSymSlots || (double)N1a * (double)N1b * most * most < 2e7)
         return nullptr;
     d->slots = (most + 15) / 16 * 16;
