@@ -1212,6 +1212,12 @@ void OzSigma::plan(cudaStream_t st) {
     F2G_CUDA(cudaStreamSynchronize(st));
 }
 
+// Same spin: column tiles at a time, of `per` elements of E each; k_oz_sum_b takes four blocks of a grid's second
+// dimension (65,535 at most) for one
+static int64_t oz_tiles(const OzSigma& o, int64_t tiles, int64_t per) {
+    return std::min({tiles, std::max<int64_t>(1, o.max_elems / per), int64_t(16383)});
+}
+
 void oz_limit(OzSigma& o, int64_t bytes, cudaStream_t st) {
     o.max_elems = bytes / (int64_t)sizeof(long long);
     for (OzScratch& w : o.scr)
@@ -1229,7 +1235,7 @@ void oz_reserve(OzSigma& o, int set, int nvec) {
         const SpinStrings& ss = o.s->spin(sp);
         const int64_t ncol = o.s->spin(1 - sp).N0, tiles = (ncol + kOzM - 1) / kOzM * nvec;
         const int64_t per = ss.N2 * ss.m2 * kOzM;
-        const int64_t nt = std::min(tiles, std::max<int64_t>(1, o.max_elems / per));
+        const int64_t nt = oz_tiles(o, tiles, per);
         e = std::max<size_t>(e, (size_t)(nt * per));
         r = std::max<size_t>(r, (size_t)(nt * kOzM * ss.N2));
     }
@@ -1275,7 +1281,7 @@ void oz_same_spin(OzSigma& o, int set, int spin, const double* C, double* S, int
     OzSpin& t = o.spin[spin];
     OzScratch& w = o.scr[set];
     const int64_t ncol = s->spin(1 - spin).N0, nd = s->nfull, tpv = (ncol + kOzM - 1) / kOzM, tiles = tpv * nvec;
-    const int64_t per = ss.N2 * ss.m2 * kOzM, step = std::min(tiles, std::max<int64_t>(1, o.max_elems / per));
+    const int64_t per = ss.N2 * ss.m2 * kOzM, step = oz_tiles(o, tiles, per);
     const int np = ss.k * (ss.k - 1) / 2;
     for (int64_t t0 = 0; t0 < tiles; t0 += step) {
         const int64_t nt = std::min(step, tiles - t0), nx = nt * kOzM;
