@@ -120,6 +120,15 @@ void DetBlocks::enumerate(int na, int nb, int sym, const std::vector<std::vector
         throw Error(2, "CIStrings: the number of active orbitals must be between 0 and 62");
     if (sym < 0 || sym >= nirrep)
         throw Error(2, "CIStrings: the state symmetry " + std::to_string(sym) + " is not an irrep of the orbitals");
+    // irreps of strings: products of those of the orbitals ({1, 2} gives 3 too)
+    uint32_t closed = 1; // one bit per irrep
+    for (int h : orbsym)
+        for (int g = 0; g < 8; ++g)
+            if (closed >> g & 1)
+                closed |= 1u << (g ^ h);
+    for (int h = nirrep; h < 8; ++h)
+        if (closed >> h & 1)
+            nirrep = h + 1;
 
     // bounds of the non-empty spaces, indexed like the spaces (ci_occupation.cc:107-141)
     Occ lo{}, hi{}, size{};
