@@ -23,8 +23,9 @@
 // most 2^24, so the FP32 sums are exact (see oz_lead for the bound). Digits and accumulators of neighbouring
 // groups lie next to each other along N, so 11 MMAs do the 28 products of a K step. The epilogue combines
 // the seven sums in a 64-bit integer T (unit: 2^-56 of the largest |a| times the largest |b|). What is
-// dropped (i + j > 6) is at most six products of 2^14 in the next group: with the digits' cut, below 2^-53 of the largest
-// |a| times the largest |b| per product (2^-51 with slack in both, see oz_lead). In the norm of a row that is less than
+// dropped (i + j > 6) is at most six products of 2^14 in the next group: with the digits' cut, below 2^-52 of the largest
+// |a| times the largest |b| per product (2^-50 with slack in both, see oz_lead), and 2^-50 (2^-48) once per output of a
+// hole string for its last group's rounding and its alignment with seven others. In the norm of a row that is less than
 // the roundings of an FP64 chain (figures below). It is more for an output whose own products are all far below that
 // largest one: a tail of 1e-8 beside a 1 whose integral is zero is left with about half its digits.
 //

@@ -28,8 +28,8 @@
 // vector, FP64 kernels -> this file: mixed block 56.4 -> 6.5 ms, same spin 8.5 -> 1.7 ms and 1-RDM 1.33 -> 1.08 ms per
 // spin; CAS(10,10) mixed 3-RDM block 1,406 -> 142 us, same-spin 3-RDM 146 -> 47 us (whole calls).
 //
-// Accuracy: a product loses less than 2^-58 of the product of its two source rows' largest elements (2^-63 of each from
-// the digits' cut, at most 2^-59 from the groups left out).
+// Accuracy: a product loses less than 2^-56 of the product of its two source rows' largest elements (2^-62 of each from
+// the digits' cut, at most 2^-57.2 from the groups left out).
 #include <cuda_fp16.h>
 
 #include <algorithm>

@@ -16,8 +16,8 @@
 // kept, sums of at most 64 rows of eight products are exact in FP32, and an element of E is their 96-bit sum rounded
 // once. k_sy_sum adds sgn E into sigma, a thread per determinant in a fixed order.
 //
-// Accuracy. A product of E[Kb][(p, r)] loses less than 2^-58 of the largest |V[p, r, q, s]| max_Ib |C(Ka + q, Ib)| in its
-// sum: 2^-62 each from the element and the integral, at most 2^-59 from the digit products left out. Compared with a
+// Accuracy. A product of E[Kb][(p, r)] loses less than 2^-56 of the largest |V[p, r, q, s]| max_Ib |C(Ka + q, Ib)| in its
+// sum: 2^-61 each from the element and the integral, at most 2^-57.2 from the digit products left out. Compared with a
 // sum in FP64 that is less in the norm of the rows that meet in a Ka, and more for an element whose own products are
 // all 2^-6 and less of that largest one. (With one scale for the whole vector that held for its norm alone: rows at 1e-12
 // of the largest were left with 22 bits.)
